@@ -386,6 +386,22 @@ int mpet_residual_noalloc(mpet_ctx* ctx, const double* b, const double* x, doubl
  * or the FP32 copy (x, y float).  Used by tests and the bandwidth bench. */
 int mpet_spmv(mpet_ctx* ctx, int32_t precision, const void* x, void* y);
 
+/* How the inner FP32 iterations of a mixed-precision solve form A x: cell by
+ * cell from the geometry and the coefficients of the last mpet_assemble (1),
+ * from the stored FP32 copy (0), or by the size of the matrix (-1, default).
+ * The stored copy serves wherever the element product cannot: triangles, a
+ * Robin term in the matrix, or a variant forced by mpet_set_spmv_variant.
+ * Takes effect at the next mpet_assemble, which must follow.  No reference
+ * counterpart (engine option and test hook). */
+int mpet_set_element_product(mpet_ctx* ctx, int32_t mode);
+
+/* y = A x as those iterations form it (float device arrays of length N);
+ * *elements (may be NULL) says whether cell by cell.  Columns of
+ * Dirichlet DOFs that mpet_apply_symmetric zeroed are still there in the
+ * element product: the inner vectors are zero at those DOFs.  No reference
+ * counterpart (test hook). */
+int mpet_krylov_product(mpet_ctx* ctx, const float* x, float* y, int32_t* elements);
+
 /* apply_symmetric / MatZeroRowsColumns (src/mpet/mpet/bc_symmetric.py:11-22):
  * zero the Dirichlet columns of the assembled matrix in place (rows were
  * replaced by mpet_assemble).  b, if not NULL, is lifted with x_bc. */

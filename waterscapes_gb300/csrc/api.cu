@@ -284,6 +284,8 @@ int mpet_assemble(mpet_ctx* c, double dt, int32_t apply_bc) {
     launch_assemble_matrix(c, dt, apply_bc != 0, c->A.v32 != nullptr);
     launch_robin_matrix(c, dt);
     refresh_system_copies(c);
+    build_patches(c);
+    set_patch_coefficients(c, dt, apply_bc != 0);
     MPET_CUDA(cudaStreamSynchronize(c->stream));
     c->assembled = true;
     c->bc_cols_zeroed = false;
@@ -491,6 +493,7 @@ int mpet_set_batch(mpet_ctx* c, int32_t ninst, const int32_t* vertex_instance) {
     require(ninst >= 1 && vertex_instance, MPET_ERR_INVALID, "need ninst >= 1 and an instance per vertex");
     setup_batch(c, ninst, vertex_instance);
     set_instances(c, ninst, vertex_instance);
+    release_patches(c);  // patches of one instance each
     c->precond_ready = false;
     c->u_hier_valid = false;
     API_END(c)
@@ -861,6 +864,24 @@ int mpet_spmv(mpet_ctx* c, int32_t precision, const void* x, void* y) {
     API_END(c)
 }
 
+int mpet_set_element_product(mpet_ctx* c, int32_t mode) {
+    API_BEGIN(c)
+    require(mode >= -1 && mode <= 1, MPET_ERR_INVALID, "mode: -1 (by size), 0 (stored matrix) or 1 (elements)");
+    c->sys_patch_mode = mode;
+    c->assembled = false;
+    API_END(c)
+}
+
+int mpet_krylov_product(mpet_ctx* c, const float* x, float* y, int32_t* elements) {
+    API_BEGIN(c)
+    require(c->assembled, MPET_ERR_STATE, "mpet_assemble must come first");
+    require(c->prm.precision == MPET_PRECISION_MIXED, MPET_ERR_STATE, "no FP32 products (setup precision is FP64)");
+    require(x && y && x != y, MPET_ERR_INVALID, "x and y must be distinct device arrays");
+    if (elements) *elements = c->sys_patch ? 1 : 0;
+    krylov_product_f32(c, x, y);
+    API_END(c)
+}
+
 int mpet_apply_symmetric(mpet_ctx* c, double* b, const double* xbc) {
     API_BEGIN(c)
     require(c->assembled, MPET_ERR_STATE, "mpet_assemble must come first");
@@ -924,6 +945,8 @@ int mpet_set_spmv_variant(mpet_ctx* c, int32_t variant) {
     destroy_minres_graph(c);
     c->A.variant = variant;
     c->A.variant64 = -1;  // the forced variant serves both precisions
+    c->sys_patch = false;  // ... and the inner iterations
+    c->sys_patch_mode = 0;
     API_END(c)
 }
 

@@ -882,6 +882,97 @@ void launch_mf_cells(mpet_ctx* c, double dt) {
     MPET_CHECK_LAUNCH();
 }
 
+// ---- data of the patch products -----------------------------------------------------
+
+// (padding slots: zeros)
+__global__ void k_patch_geometry(int64_t nslots, int P, const int32_t* __restrict__ cell,
+                                 const double* __restrict__ geo, float* out) {
+    const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (s >= nslots) return;
+    const int64_t p = s / P;
+    const int l = (int)(s % P);
+    const int32_t c = cell[s];
+    Geo G{};
+    if (c >= 0) load_geo(geo, c, G);
+#pragma unroll
+    for (int q = 0; q < 9; ++q) out[(p * 10 + q) * P + l] = (float)G.b[1 + q / 3][q % 3];
+    out[(p * 10 + 9) * P + l] = (float)(G.vol * kappa<3>());
+}
+
+void launch_patch_geometry(mpet_ctx* c) {
+    const PatchSet& s = c->patch;
+    k_patch_geometry<<<grid_for(s.np * s.P, 256), 256, 0, c->stream>>>(s.np * s.P, s.P, s.cell, c->geo, s.sys);
+    MPET_CHECK_LAUNCH();
+}
+
+__global__ void k_patch_coef(int64_t nslots, int P, const int32_t* __restrict__ cell, int ncell, MatCoef C,
+                             float* out) {
+    const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (s >= nslots) return;
+    const int64_t p = s / P;
+    const int l = (int)(s % P);
+    const int32_t c = cell[s];
+    const int J = C.J;
+    for (int q = 0; q < ncell; ++q) {
+        double v = 0.0;
+        if (c >= 0 && q < J) {
+            v = -C.dt_theta * C.Kof(q, c);
+        } else if (c >= 0) {
+            const int a = (q - J) / J, b = (q - J) % J;
+            v = -(C.dt_theta * ((a == b ? C.Ssumof(a, c) : 0.0) - C.Sof(a, b, c)) +
+                  C.rank_inv * C.rank_b[a] * C.rank_b[b]) -
+                (a == b ? C.cof(a, c) : 0.0);
+        }
+        out[(p * ncell + q) * P + l] = (float)v;
+    }
+}
+
+void set_patch_coefficients(mpet_ctx* c, double dt, bool apply_bc) {
+    PatchSet& s = c->patch;
+    const MatCoef C = make_coef(c, dt);
+    const int J = c->J;
+    PatchCoef q{};
+    // From 3e6 entries on: the two kernels of an element product take about 13 us however
+    // small the mesh, the stored product 4.5 us at 0.2e6 entries (4^3 cube, A=2), 7.4 at 1.6e6
+    // (8^3; a whole iteration 72 us stored, 77 by elements), 14.7 at 5.3e6 (12^3; 121 and 112)
+    // and 769 against 195 at 1.03e9 (64^3, A=4).  Boundary-facet terms of the matrix are not
+    // element products.
+    bool use = s.ready() && !(c->nf > 0 && c->f_beta_matrix) &&
+               (c->sys_patch_mode == 1 || (c->sys_patch_mode < 0 && c->nnz >= 3000000));
+    float* const coef0 = s.coef;
+    if (use) {
+        q.mu = (float)C.mu;
+        q.lam = (float)C.lmbda;
+        for (int a = 0; a < J; ++a) {
+            q.cpl[a] = (float)C.cpl[a];
+            q.Kd[a] = (float)C.Kd[a];
+            for (int b = 0; b < J; ++b)
+                q.Cm[a * MPET_MAX_NETWORKS + b] = (float)C.Cm[a * MPET_MAX_NETWORKS + b];
+        }
+        q.bc = apply_bc ? 1 : 0;
+        q.ncell = C.coef_const ? 0 : (C.cc || C.Sc ? J + J * J : J);
+        const int64_t need = s.np * s.P * q.ncell;
+        if (need > s.ncoef) {
+            if (device_fits(c, (size_t)need * sizeof(float))) {
+                c->pool.release(s.coef);
+                s.coef = c->pool.alloc<float>(need);
+                s.ncoef = need;
+            } else {
+                use = false;
+            }
+        }
+        if (use && q.ncell > 0) {
+            k_patch_coef<<<grid_for(s.np * s.P, 256), 256, 0, c->stream>>>(s.np * s.P, s.P, s.cell, q.ncell, C, s.coef);
+            MPET_CHECK_LAUNCH();
+        }
+    }
+    // captured iterations hold the coefficients and the choice
+    if (use != c->sys_patch || (use && (s.coef != coef0 || memcmp(&q, &c->patch_coef, sizeof(q)) != 0)))
+        destroy_minres_graph(c);
+    c->sys_patch = use;
+    c->patch_coef = q;
+}
+
 void launch_rhs(mpet_ctx* c, double dt, const double* up_prev, double* b) {
     RhsArgs A{};
     A.nnodes = c->nnodes;

@@ -172,6 +172,42 @@ struct Csr {
     int32_t* skl = nullptr;
 };
 
+// Patches of tetrahedra for the FP32 element products (patch.cuh).  Slot p * P + l is lane l
+// of patch p; each patch lists its nodes, vertices first.
+struct PatchSet {
+    int P = 0;                     // cells per patch, one thread each
+    int max_pn = 0, max_pv = 0;    // most nodes / vertices of a patch
+    int64_t np = 0, npn = 0, nsh = 0, nslot = 0;  // patches, patch nodes, shared nodes, their partial sums
+    int64_t nshv = 0, nslotv = 0;  // vertices among the shared nodes (the first ones), their partial sums
+    int32_t* cell = nullptr;       // np * P: mesh cell of each slot, -1 for padding
+    uint32_t* lid = nullptr;       // (p * 5 + w) * P + l: local node ids 2 w and 2 w + 1 of the slot's cell
+    int32_t* pn_ptr = nullptr;     // np + 1: first patch node
+    int32_t* pn_nv = nullptr;      // np: vertices of the patch
+    int32_t* pn_node = nullptr;    // npn: node, sign bit set where the displacement is Dirichlet
+    int32_t* pn_sh = nullptr;      // npn: -1, or the slot of this patch's partial sum of a shared node
+    int32_t* sh_ptr = nullptr;     // nsh + 1: first slot of each shared node (one per patch, ascending)
+    int32_t* sh_node = nullptr;    // nsh: node, sign bit as in pn_node
+    uint16_t* gl_ptr = nullptr;    // npn + np: first contribution of each patch node, relative to its patch
+    uint32_t* pos = nullptr;       // as lid: places of the cell's ten values among the contributions
+    int32_t* inst = nullptr;       // np: instance of the patch (batches; a patch holds one instance)
+    float* part = nullptr;         // partial sums of the shared nodes
+    float* part_p = nullptr;       // J planes of nslotv: partial sums of the pressure rows
+    float* sys = nullptr;          // (p * 10 + q) * P + l: b_1, b_2, b_3 (9 values) and |T| / 20
+    float* coef = nullptr;         // (p * ncell + q) * P + l: per-cell coefficients (PatchCoef::ncell)
+    int64_t ncoef = 0;             // floats allocated for them
+    bool tried = false;
+    bool ready() const { return np > 0; }
+};
+
+// Coefficients of the patch products: (p_a, div v) and (div u, q_a) with cpl_a, the
+// pressure-pressure block Cm_ab (p_b, q_a) + [a == b] Kd_a (grad p_a, grad q_a).
+struct PatchCoef {
+    float mu, lam;
+    float cpl[MPET_MAX_NETWORKS], Cm[MPET_MAX_NETWORKS * MPET_MAX_NETWORKS], Kd[MPET_MAX_NETWORKS];
+    int ncell;  // values per cell in PatchSet::coef: 0 none, J the Kd_a, J + J J the Kd_a and Cm_ab
+    int bc;     // Dirichlet rows are unit rows
+};
+
 struct AmgLevel {
     Csr A, P, R;       // P: n x nc (prolongation), R = P^T
     bool mf = false;   // products with A formed matrix-free from per-cell data (first displacement level)
@@ -361,6 +397,12 @@ struct mpet_ctx {
     float* mf_tab = nullptr;
     int mf_mode = -1;             // -1 autotuned, 0 CSR, 1 matrix-free (test hook)
     float mf_ms[2] = {0.f, 0.f};  // autotuner: Chebyshev product with the CSR level / matrix-free
+    // element products on patches of cells (FP32, tetrahedra), their coefficients as of the last
+    // assembly, whether the inner products use them, and the choice (-1: by the matrix's size)
+    mpet::PatchSet patch;
+    mpet::PatchCoef patch_coef{};
+    bool sys_patch = false;
+    int sys_patch_mode = -1;
     bool gmres = false;           // solves by restarted GMRES (non-symmetric system)
     // constant-pressure constraints (int p_k = 0, multiplier p_null_k): networks, the P1
     // load vector (int phi_v), W_k = A^-1 B_k^T (nq x N), the inverse of B W, multipliers
@@ -527,6 +569,11 @@ void build_topology(mpet_ctx* c);
 void build_pattern(mpet_ctx* c);
 void build_bc(mpet_ctx* c);
 
+// patches of cells for the FP32 element products, once per mesh and batch partition; leaves
+// c->patch without patches where they cannot serve (2D, FP64 only, HBM short)
+void build_patches(mpet_ctx* c);
+void release_patches(mpet_ctx* c);
+
 // facets.cu
 void build_facets(mpet_ctx* c);
 void launch_facet_rhs(mpet_ctx* c, double dt, const double* up_prev, double* b);
@@ -538,6 +585,10 @@ void launch_assemble_prec_blocks(mpet_ctx* c, double dt);
 // per-cell data of the matrix-free first displacement level (c->mf_cell, c->mf_tab);
 // leaves c->mf_cell null when HBM is short
 void launch_mf_cells(mpet_ctx* c, double dt);
+// per-cell geometry of the patch products (once per patch set), and their coefficients for
+// this assembly (sets c->patch_coef and c->sys_patch)
+void launch_patch_geometry(mpet_ctx* c);
+void set_patch_coefficients(mpet_ctx* c, double dt, bool apply_bc);
 void setup_network_modes(mpet_ctx* c, double dt);
 void set_instances(mpet_ctx* c, int ninst, const int32_t* vertex_inst_host);
 void launch_rhs(mpet_ctx* c, double dt, const double* up_prev, double* b);
@@ -610,6 +661,8 @@ void fill_sell(mpet_ctx* c, Csr& A);
 void build_node_blocks(mpet_ctx* c);
 bool device_fits(mpet_ctx* c, size_t bytes);
 void refresh_system_copies(mpet_ctx* c);
+// y = A x (FP32) as the inner Krylov iterations form it
+void krylov_product_f32(mpet_ctx* c, const float* x, float* y);
 bool spmv_variant_available(const Csr& A, int variant);
 constexpr int SPMV_TILE = 2048;  // entries per staged tile
 void destroy_minres_graph(mpet_ctx* c);

@@ -14,6 +14,8 @@
 #include <cub/cub.cuh>
 #include <thrust/iterator/counting_iterator.h>
 
+#include <algorithm>
+
 #include "mpet_internal.cuh"
 
 namespace mpet {
@@ -545,6 +547,398 @@ void build_bc(mpet_ctx* c) {
                 c->dof_bc);
     MPET_CHECK_LAUNCH();
     MPET_CUDA(cudaStreamSynchronize(s));
+}
+
+
+// ---- patches of cells --------------------------------------------------------------
+//
+// Cells in Morton order of their centroids (instance by instance in a batch), cut into
+// patches of at most P cells; per patch its node list, the cells' local ids, the places of
+// their contributions and, for nodes of several patches, the slots of their partial sums.  All
+// from sorted 64-bit keys, as above: the numbering is the same in every run.
+
+__device__ __forceinline__ u64 spread3(u64 v) {
+    u64 r = 0;
+    for (int b = 0; b < 14; ++b) r |= ((v >> b) & 1ULL) << (3 * b);
+    return r;
+}
+
+__global__ void k_cell_morton(const double* __restrict__ x, const int32_t* __restrict__ cells, int64_t nc,
+                              const int32_t* __restrict__ inst, double lo0, double lo1, double lo2, double scale,
+                              u64* key, int32_t* idx) {
+    const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (c >= nc) return;
+    const double lo[3] = {lo0, lo1, lo2};
+    u64 m = 0;
+    for (int k = 0; k < 3; ++k) {
+        double s = 0.0;
+        for (int v = 0; v < 4; ++v) s += x[3 * (int64_t)cells[4 * c + v] + k];
+        double q = (0.25 * s - lo[k]) * scale;
+        q = q < 0.0 ? 0.0 : (q > 16383.0 ? 16383.0 : q);
+        m |= spread3((u64)q) << k;
+    }
+    key[c] = ((u64)(inst ? inst[c] : 0) << 42) | m;
+    idx[c] = (int32_t)c;
+}
+
+__global__ void k_patch_slots(int64_t np, int P, const int32_t* __restrict__ pstart,
+                              const int32_t* __restrict__ order, int32_t* cell) {
+    const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (s >= np * P) return;
+    const int64_t p = s / P;
+    const int l = (int)(s % P);
+    cell[s] = l < pstart[p + 1] - pstart[p] ? order[pstart[p] + l] : -1;
+}
+
+__global__ void k_patch_node_keys(int64_t np, int P, const int32_t* __restrict__ cell,
+                                  const int32_t* __restrict__ cn, u64* key) {
+    const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (r >= np * P * 10) return;
+    const int64_t s = r / 10;
+    const int32_t c = cell[s];
+    // (padding repeats the patch's first node)
+    const int64_t cc = c >= 0 ? c : cell[s / P * P];
+    key[r] = ((u64)(s / P) << 32) | (u64)cn[10 * cc + (c >= 0 ? r % 10 : 0)];
+}
+
+__global__ void k_patch_ptr(const u64* __restrict__ key, int64_t n, int64_t np, int64_t nv, int32_t* ptr,
+                            int32_t* pnv) {
+    const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (p > np) return;
+    const int64_t b = lower_bound_u64(key, n, (u64)p << 32);
+    ptr[p] = (int32_t)b;
+    if (p < np) pnv[p] = (int32_t)(lower_bound_u64(key, n, ((u64)p << 32) | (u64)nv) - b);
+}
+
+// cells of the patch at each of its nodes
+__global__ void k_patch_valence(int64_t np, int P, const int32_t* __restrict__ cell, const int32_t* __restrict__ cn,
+                                const u64* __restrict__ key, const int32_t* __restrict__ ptr, int32_t* val) {
+    const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (r >= np * P * 10) return;
+    const int64_t s = r / 10, p = s / P;
+    const int32_t c = cell[s];
+    if (c < 0) return;
+    const int32_t b = ptr[p];
+    const u64 k = ((u64)p << 32) | (u64)cn[10 * (int64_t)c + r % 10];
+    atomicAdd(val + b + lower_bound_u64(key + b, ptr[p + 1] - b, k), 1);
+}
+
+// order of a patch's nodes: vertices, then edges, each by decreasing valence (a warp's
+// threads then add about equally many contributions), then by node
+__global__ void k_patch_order_keys(int64_t npn, const u64* __restrict__ key, const int32_t* __restrict__ val,
+                                   int64_t nv, u64* okey, int32_t* idx) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= npn) return;
+    const u64 node = key[i] & 0xffffffffu;
+    const int v = val[i] < 255 ? val[i] : 255;
+    okey[i] = ((key[i] >> 32) << 40) | ((node < (u64)nv ? 0ULL : 1ULL) << 39) | ((u64)(255 - v) << 31) | node;
+    idx[i] = (int32_t)i;
+}
+
+__global__ void k_patch_reorder(int64_t npn, const int32_t* __restrict__ idx, const u64* __restrict__ key,
+                                u64* okey, int32_t* inv) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= npn) return;
+    okey[i] = key[idx[i]];
+    inv[idx[i]] = (int32_t)i;
+}
+
+// local ids of every slot's cell, and the contribution keys (patch node << 16) | (j P + lane)
+__global__ void k_patch_lids(int64_t np, int P, const int32_t* __restrict__ cell, const int32_t* __restrict__ cn,
+                             const u64* __restrict__ key, const int32_t* __restrict__ inv,
+                             const int32_t* __restrict__ ptr, uint32_t* lid, u64* gkey) {
+    const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (s >= np * P) return;
+    const int64_t p = s / P;
+    const int l = (int)(s % P);
+    const int32_t c = cell[s];
+    const int32_t b = ptr[p];
+    const int64_t n = ptr[p + 1] - b;
+    for (int w = 0; w < 5; ++w) {
+        uint32_t v = 0;
+        for (int h = 0; h < 2; ++h) {
+            const int j = 2 * w + h;
+            uint32_t i = 0;
+            if (c >= 0)
+                i = (uint32_t)(inv[b + lower_bound_u64(key + b, n, ((u64)p << 32) | (u64)cn[10 * (int64_t)c + j])] - b);
+            v |= i << (16 * h);
+            gkey[s * 10 + j] = c >= 0 ? (((u64)b + i) << 16) | (u64)(j * P + l) : ~0ULL;
+        }
+        lid[(p * 5 + w) * P + l] = v;
+    }
+}
+
+// place of each slot's values among its patch's contributions (sorted by node, then lane)
+__global__ void k_patch_pos(int64_t np, int P, const int32_t* __restrict__ cell, const u64* __restrict__ gkey,
+                            int64_t n, const int32_t* __restrict__ ptr, const uint32_t* __restrict__ lid,
+                            const int32_t* __restrict__ pstart, uint32_t* pos) {
+    const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (s >= np * P) return;
+    const int64_t p = s / P;
+    const int l = (int)(s % P);
+    const int32_t c = cell[s];
+    const int64_t g0 = 10 * (int64_t)pstart[p];
+    const int64_t gn = 10 * (int64_t)(pstart[p + 1] - pstart[p]);
+    for (int w = 0; w < 5; ++w) {
+        const uint32_t ids = lid[(p * 5 + w) * P + l];
+        uint32_t v = 0;
+        for (int h = 0; h < 2; ++h) {
+            const int j = 2 * w + h;
+            uint32_t q = 0xffffu;  // (padding)
+            if (c >= 0)
+                q = (uint32_t)lower_bound_u64(gkey + g0, gn,
+                                              (((u64)ptr[p] + ((ids >> (16 * h)) & 0xffffu)) << 16) | (u64)(j * P + l));
+            v |= q << (16 * h);
+        }
+        pos[(p * 5 + w) * P + l] = v;
+    }
+}
+
+__global__ void k_patch_gl_ptr(const u64* __restrict__ gkey, int64_t n, const u64* __restrict__ key, int64_t npn,
+                               const int32_t* __restrict__ ptr, const int32_t* __restrict__ pstart,
+                               uint16_t* gl_ptr) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= npn) return;
+    const int64_t p = (int64_t)(key[i] >> 32);
+    gl_ptr[i + p] = (uint16_t)(lower_bound_u64(gkey, n, (u64)i << 16) - 10 * (int64_t)pstart[p]);
+    if (i + 1 == ptr[p + 1]) gl_ptr[i + p + 1] = (uint16_t)(10 * (pstart[p + 1] - pstart[p]));
+}
+
+__global__ void k_patch_node_major(int64_t npn, const u64* __restrict__ key, u64* nkey) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i < npn) nkey[i] = (key[i] << 32) | (u64)i;
+}
+
+// per node: whether several patches hold it, and its number of partial sums
+__global__ void k_patch_shared(int64_t nnodes, const u64* __restrict__ nkey, int64_t npn, int32_t* shared,
+                               int32_t* slots) {
+    const int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (v >= nnodes) return;
+    const int n = (int)(lower_bound_u64(nkey, npn, (u64)(v + 1) << 32) - lower_bound_u64(nkey, npn, (u64)v << 32));
+    shared[v] = n > 1;
+    slots[v] = n > 1 ? n : 0;
+}
+
+__global__ void k_patch_fill_shared(int64_t npn, const u64* __restrict__ nkey,
+                                    const int32_t* __restrict__ shared, const int32_t* __restrict__ sid,
+                                    const int32_t* __restrict__ sbase, const int32_t* __restrict__ slots,
+                                    const uint8_t* __restrict__ node_bc, int32_t* pn_node, int32_t* pn_sh,
+                                    int32_t* sh_ptr, int32_t* sh_node) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= npn) return;
+    const int64_t v = (int64_t)(nkey[i] >> 32), pn = (int64_t)(nkey[i] & 0xffffffffu);
+    pn_node[pn] = (int32_t)v | (node_bc[v] ? (int32_t)0x80000000 : 0);
+    if (!shared[v]) {
+        pn_sh[pn] = -1;
+        return;
+    }
+    const int rank = (int)(i - lower_bound_u64(nkey, npn, (u64)v << 32));
+    pn_sh[pn] = sbase[v] + rank;
+    if (rank == 0) {
+        sh_node[sid[v]] = pn_node[pn];
+        sh_ptr[sid[v]] = sbase[v];
+        sh_ptr[sid[v] + 1] = sbase[v] + slots[v];  // (the next shared node writes the same value)
+    }
+}
+
+void release_patches(mpet_ctx* c) {
+    PatchSet& s = c->patch;
+    for (void* p : {(void*)s.cell, (void*)s.lid, (void*)s.pn_ptr, (void*)s.pn_nv, (void*)s.pn_node, (void*)s.pn_sh,
+                    (void*)s.sh_ptr, (void*)s.sh_node, (void*)s.gl_ptr, (void*)s.pos, (void*)s.inst, (void*)s.part,
+                    (void*)s.part_p, (void*)s.sys, (void*)s.coef})
+        c->pool.release(p);
+    s = PatchSet();
+    c->sys_patch = false;
+}
+
+void build_patches(mpet_ctx* c) {
+    PatchSet& s = c->patch;
+    if (s.tried) return;
+    s.tried = true;
+    const int64_t nc = c->nc;
+    if (c->dim != 3 || nc < 1 || c->prm.precision != MPET_PRECISION_MIXED) return;
+    // cells per patch: 256 once every SM gets two patches of them, else smaller patches so that
+    // a small mesh still spreads over the chip
+    const int P = nc >= 256 * 304 ? 256 : (nc >= 128 * 152 ? 128 : 64);
+    const int J = c->J;
+    if (!device_fits(c, (size_t)nc * (200 + 4 * (10 + J * J + J)) + (size_t)c->nnodes * (16 + 4 * J) * 2)) return;
+    cudaStream_t st = c->stream;
+    const int T = 256;
+    // patch boundaries (host): instance by instance, patches of equal size
+    std::vector<int64_t> ncell(c->ninst > 0 ? c->ninst : 1, 0);
+    if (c->ninst > 0) {
+        std::vector<int32_t> ci(nc);
+        MPET_CUDA(cudaMemcpyAsync(ci.data(), c->cell_inst, sizeof(int32_t) * nc, cudaMemcpyDeviceToHost, st));
+        MPET_CUDA(cudaStreamSynchronize(st));
+        for (int32_t i : ci) ncell[i]++;
+    } else {
+        ncell[0] = nc;
+    }
+    std::vector<int32_t> pstart, pinst;
+    int64_t base = 0;
+    for (size_t i = 0; i < ncell.size(); ++i) {
+        const int64_t k = (ncell[i] + P - 1) / P;
+        for (int64_t q = 0; q < k; ++q) {
+            pstart.push_back((int32_t)(base + ncell[i] * q / k));
+            pinst.push_back((int32_t)i);
+        }
+        base += ncell[i];
+    }
+    const int64_t np = (int64_t)pstart.size();
+    pstart.push_back((int32_t)nc);
+    if (np * P * 10 >= 2147483647LL || c->nnodes >= (1LL << 30)) return;  // (32-bit keys, flag bits)
+    TmpBuf d_pstart(sizeof(int32_t) * (np + 1));
+    MPET_CUDA(cudaMemcpyAsync(d_pstart.p, pstart.data(), sizeof(int32_t) * (np + 1), cudaMemcpyHostToDevice, st));
+    // bounding box of the vertices
+    std::vector<double> xyz((size_t)c->nv * 3);
+    MPET_CUDA(cudaMemcpyAsync(xyz.data(), c->x, sizeof(double) * xyz.size(), cudaMemcpyDeviceToHost, st));
+    MPET_CUDA(cudaStreamSynchronize(st));
+    double lo[3] = {1e300, 1e300, 1e300}, ext = 0.0;
+    for (int k = 0; k < 3; ++k) {
+        double hi = -1e300;
+        for (int64_t v = 0; v < c->nv; ++v) {
+            lo[k] = xyz[3 * v + k] < lo[k] ? xyz[3 * v + k] : lo[k];
+            hi = xyz[3 * v + k] > hi ? xyz[3 * v + k] : hi;
+        }
+        ext = hi - lo[k] > ext ? hi - lo[k] : ext;
+    }
+    const double scale = ext > 0.0 ? 16384.0 / ext : 0.0;
+    s.cell = c->pool.alloc<int32_t>(np * P);
+    {
+        TmpBuf k0(sizeof(u64) * nc), k1(sizeof(u64) * nc), i0(sizeof(int32_t) * nc), i1(sizeof(int32_t) * nc);
+        k_cell_morton<<<grid_for(nc, T), T, 0, st>>>(c->x, c->cells, nc, c->ninst > 0 ? c->cell_inst : nullptr, lo[0],
+                                                     lo[1], lo[2], scale, k0.as<u64>(), i0.as<int32_t>());
+        MPET_CHECK_LAUNCH();
+        size_t tb = 0;
+        const int eb = 42 + bits_for((u64)ncell.size());
+        MPET_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, k0.as<u64>(), k1.as<u64>(), i0.as<int32_t>(),
+                                                  i1.as<int32_t>(), (int)nc, 0, eb, st));
+        TmpBuf tmp(tb);
+        MPET_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, tb, k0.as<u64>(), k1.as<u64>(), i0.as<int32_t>(),
+                                                  i1.as<int32_t>(), (int)nc, 0, eb, st));
+        k_patch_slots<<<grid_for(np * P, T), T, 0, st>>>(np, P, d_pstart.as<int32_t>(), i1.as<int32_t>(), s.cell);
+        MPET_CHECK_LAUNCH();
+        MPET_CUDA(cudaStreamSynchronize(st));
+    }
+    // patch nodes
+    const int64_t nref = np * P * 10;
+    u64* key = nullptr;
+    {
+        TmpBuf keys(sizeof(u64) * nref);
+        k_patch_node_keys<<<grid_for(nref, T), T, 0, st>>>(np, P, s.cell, c->cell_nodes, keys.as<u64>());
+        MPET_CHECK_LAUNCH();
+        s.npn = sort_unique(c, keys.as<u64>(), nref, 32 + bits_for((u64)np), &key);
+    }
+    s.pn_ptr = c->pool.alloc<int32_t>(np + 1);
+    s.pn_nv = c->pool.alloc<int32_t>(np);
+    k_patch_ptr<<<grid_for(np + 1, T), T, 0, st>>>(key, s.npn, np, c->nv, s.pn_ptr, s.pn_nv);
+    MPET_CHECK_LAUNCH();
+    std::vector<int32_t> ptr(np + 1), pnv(np);
+    MPET_CUDA(cudaMemcpyAsync(ptr.data(), s.pn_ptr, sizeof(int32_t) * (np + 1), cudaMemcpyDeviceToHost, st));
+    MPET_CUDA(cudaMemcpyAsync(pnv.data(), s.pn_nv, sizeof(int32_t) * np, cudaMemcpyDeviceToHost, st));
+    // the patch nodes in their order within the patch
+    TmpBuf inv(sizeof(int32_t) * s.npn), okey(sizeof(u64) * s.npn);
+    {
+        TmpBuf val(sizeof(int32_t) * s.npn), k0(sizeof(u64) * s.npn), i0(sizeof(int32_t) * s.npn),
+            i1(sizeof(int32_t) * s.npn);
+        MPET_CUDA(cudaMemsetAsync(val.p, 0, sizeof(int32_t) * s.npn, st));
+        k_patch_valence<<<grid_for(nref, T), T, 0, st>>>(np, P, s.cell, c->cell_nodes, key, s.pn_ptr,
+                                                         val.as<int32_t>());
+        k_patch_order_keys<<<grid_for(s.npn, T), T, 0, st>>>(s.npn, key, val.as<int32_t>(), c->nv, k0.as<u64>(),
+                                                             i0.as<int32_t>());
+        MPET_CHECK_LAUNCH();
+        size_t tb = 0;
+        const int eb = 40 + bits_for((u64)np);
+        MPET_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, k0.as<u64>(), okey.as<u64>(), i0.as<int32_t>(),
+                                                  i1.as<int32_t>(), (int)s.npn, 0, eb, st));
+        TmpBuf tmp(tb);
+        MPET_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, tb, k0.as<u64>(), okey.as<u64>(), i0.as<int32_t>(),
+                                                  i1.as<int32_t>(), (int)s.npn, 0, eb, st));
+        k_patch_reorder<<<grid_for(s.npn, T), T, 0, st>>>(s.npn, i1.as<int32_t>(), key, okey.as<u64>(),
+                                                          inv.as<int32_t>());
+        MPET_CHECK_LAUNCH();
+        MPET_CUDA(cudaStreamSynchronize(st));
+    }
+    // local ids and places of the contributions
+    s.lid = c->pool.alloc<uint32_t>(np * P * 5);
+    s.pos = c->pool.alloc<uint32_t>(np * P * 5);
+    s.gl_ptr = c->pool.alloc<uint16_t>(s.npn + np);
+    {
+        TmpBuf keys(sizeof(u64) * nref);
+        k_patch_lids<<<grid_for(np * P, T), T, 0, st>>>(np, P, s.cell, c->cell_nodes, key, inv.as<int32_t>(),
+                                                        s.pn_ptr, s.lid, keys.as<u64>());
+        MPET_CHECK_LAUNCH();
+        u64* gk = nullptr;
+        sort_unique(c, keys.as<u64>(), nref, 64, &gk);
+        k_patch_pos<<<grid_for(np * P, T), T, 0, st>>>(np, P, s.cell, gk, nc * 10, s.pn_ptr, s.lid,
+                                                       d_pstart.as<int32_t>(), s.pos);
+        k_patch_gl_ptr<<<grid_for(s.npn, T), T, 0, st>>>(gk, nc * 10, okey.as<u64>(), s.npn, s.pn_ptr,
+                                                         d_pstart.as<int32_t>(), s.gl_ptr);
+        MPET_CHECK_LAUNCH();
+        MPET_CUDA(cudaStreamSynchronize(st));
+        c->pool.release(gk);
+    }
+    for (int64_t p = 0; p < np; ++p) {
+        s.max_pn = std::max(s.max_pn, ptr[p + 1] - ptr[p]);
+        s.max_pv = std::max(s.max_pv, pnv[p]);
+    }
+    // nodes of several patches
+    s.pn_node = c->pool.alloc<int32_t>(s.npn);
+    s.pn_sh = c->pool.alloc<int32_t>(s.npn);
+    {
+        const int64_t nn = c->nnodes;
+        TmpBuf keys(sizeof(u64) * s.npn), shared(sizeof(int32_t) * (nn + 1)), slots(sizeof(int32_t) * (nn + 1)),
+            sid(sizeof(int32_t) * (nn + 1)), sbase(sizeof(int32_t) * (nn + 1));
+        k_patch_node_major<<<grid_for(s.npn, T), T, 0, st>>>(s.npn, okey.as<u64>(), keys.as<u64>());
+        MPET_CHECK_LAUNCH();
+        u64* nk = nullptr;
+        sort_unique(c, keys.as<u64>(), s.npn, 32 + bits_for((u64)nn), &nk);
+        for (TmpBuf* b : {&shared, &slots}) MPET_CUDA(cudaMemsetAsync(b->p, 0, sizeof(int32_t) * (nn + 1), st));
+        k_patch_shared<<<grid_for(nn, T), T, 0, st>>>(nn, nk, s.npn, shared.as<int32_t>(), slots.as<int32_t>());
+        MPET_CHECK_LAUNCH();
+        size_t tb = 0;
+        MPET_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, shared.as<int32_t>(), sid.as<int32_t>(), (int)(nn + 1), st));
+        TmpBuf tmp(tb);
+        MPET_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, tb, shared.as<int32_t>(), sid.as<int32_t>(), (int)(nn + 1), st));
+        MPET_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, tb, slots.as<int32_t>(), sbase.as<int32_t>(), (int)(nn + 1), st));
+        int32_t tot[4];
+        MPET_CUDA(cudaMemcpyAsync(&tot[0], sid.as<int32_t>() + nn, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+        MPET_CUDA(cudaMemcpyAsync(&tot[1], sbase.as<int32_t>() + nn, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+        MPET_CUDA(cudaMemcpyAsync(&tot[2], sid.as<int32_t>() + c->nv, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+        MPET_CUDA(cudaMemcpyAsync(&tot[3], sbase.as<int32_t>() + c->nv, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+        MPET_CUDA(cudaStreamSynchronize(st));
+        s.nsh = tot[0];
+        s.nslot = tot[1];
+        s.nshv = tot[2];
+        s.nslotv = tot[3];
+        s.sh_ptr = c->pool.alloc<int32_t>(s.nsh + 1);
+        s.sh_node = c->pool.alloc<int32_t>(s.nsh);
+        MPET_CUDA(cudaMemsetAsync(s.sh_ptr, 0, sizeof(int32_t) * (s.nsh + 1), st));
+        k_patch_fill_shared<<<grid_for(s.npn, T), T, 0, st>>>(s.npn, nk, shared.as<int32_t>(), sid.as<int32_t>(),
+                                                              sbase.as<int32_t>(), slots.as<int32_t>(), c->node_bc,
+                                                              s.pn_node, s.pn_sh, s.sh_ptr, s.sh_node);
+        MPET_CHECK_LAUNCH();
+        MPET_CUDA(cudaStreamSynchronize(st));
+        c->pool.release(nk);
+    }
+    c->pool.release(key);
+    // shared memory of a block (patch.cuh): x at the nodes and the contributions
+    if (4 * (5 * s.max_pn + J * s.max_pv + (30 + 4 * J) * P) > 200 * 1024) {
+        release_patches(c);
+        c->patch.tried = true;
+        return;
+    }
+    if (c->ninst > 0) {
+        s.inst = c->pool.alloc<int32_t>(np);
+        MPET_CUDA(cudaMemcpyAsync(s.inst, pinst.data(), sizeof(int32_t) * np, cudaMemcpyHostToDevice, st));
+    }
+    s.part = c->pool.alloc<float>(s.nslot * 4);
+    s.part_p = c->pool.alloc<float>(s.nslotv * J);
+    s.sys = c->pool.alloc<float>(np * P * 10);
+    MPET_CUDA(cudaStreamSynchronize(st));
+    s.P = P;
+    s.np = np;
+    launch_patch_geometry(c);
 }
 
 }  // namespace mpet

@@ -1381,6 +1381,10 @@ static void launch_p2lap_mf(mpet_ctx* c, const T* x, const Epi& epi) {
     c->n_launch++;
 }
 
+#include "patch.cuh"
+
+void krylov_product_f32(mpet_ctx* c, const float* x, float* y) { krylov_product<float>(c, x, y); }
+
 // operator of an AMG level: its CSR copy, the matrix-free first displacement
 // level, or the displacement block of the system
 template <typename T, int NV, class Epi>
@@ -1967,7 +1971,7 @@ static void minres_three(mpet_ctx* c) {
         T* r2 = (T*)c->kr[ir2];
         T* y = (T*)c->kr[iy];
         k_mr_v<T><<<G, 256, 0, c->stream>>>(n, y, v, c->sc);
-        launch_spmv<T, 1>(c, c->A, vals<T>(c->A), v, EpiMinres<T>{y, r1, v, c->sc});
+        minres_product<T>(c, EpiMinres<T>{y, r1, v, c->sc});
         c->n_spmv++;
         k_mr_alfa<<<1, 256, 0, c->stream>>>(c->sc, c->partials);
         k_mr_axpy<T><<<G, 256, 0, c->stream>>>(n, y, r2, c->sc);
@@ -2688,7 +2692,7 @@ static void bminres_three(mpet_ctx* c) {
         k_bmr_freeze<<<gi, 128, 0, c->stream>>>(ni, c->bsc, c->bdone);
         k_bmr_v<T><<<(unsigned)nch, 256, 0, c->stream>>>(c->ch_lo, c->ch_len, c->ch_inst, y, v, c->bsc, c->bdone);
         MPET_CHECK_LAUNCH();
-        launch_spmv<T, 1>(c, c->A, vals<T>(c->A), v, EpiStore<T, 1>{y});
+        krylov_product<T>(c, v, y);
         c->n_spmv++;
         k_bmr_axpy_dot<T><<<(unsigned)nch, 256, 0, c->stream>>>(c->ch_lo, c->ch_len, c->ch_inst, y, r1, v, c->bsc,
                                                                  c->ch_part, c->bdone);
@@ -3180,7 +3184,7 @@ static int gmres_run(mpet_ctx* c, const T* rhs, T* d, double target, int maxit, 
         bool conv = false;
         for (int j = 0; j < m && total < maxit; ++j) {
             T* vj = V + (int64_t)j * n;
-            launch_spmv<T, 1>(c, c->A, vals<T>(c->A), vj, EpiStore<T, 1>{z});
+            krylov_product<T>(c, vj, z);
             c->n_spmv++;
             precond<T>(c, z, w);
             double* h = &H[(size_t)j * (m + 1)];  // column j, rows 0..j+1
@@ -3237,7 +3241,7 @@ static int gmres_run(mpet_ctx* c, const T* rhs, T* d, double target, int maxit, 
             return conv ? MPET_OK : MPET_ERR_MAXIT;
         }
         // restart from r = M^-1 (rhs - A d)
-        launch_spmv<T, 1>(c, c->A, vals<T>(c->A), d, EpiStore<T, 1>{w});
+        krylov_product<T>(c, d, w);
         c->n_spmv++;
         k_gm_sub<T><<<G, 256, 0, c->stream>>>(n, rhs, w, z);
         MPET_CHECK_LAUNCH();
