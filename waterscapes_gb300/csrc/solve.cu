@@ -93,6 +93,13 @@ struct VecIO<double, 4> {
     }
 };
 
+// Components computed of an NV-wide row: the padded layout holds at most three (the fourth is
+// zero in every vector of the displacement hierarchy and stays zero).  In FP64 the products of
+// the hierarchy are bound by the FP64 pipe, so a fourth multiply-add per entry was a quarter of
+// their time.
+template <int NV>
+__host__ __device__ constexpr int ncomp() { return NV == 4 ? 3 : NV; }
+
 // ---- SpMV with fused epilogues -------------------------------------------------------
 //
 // An epilogue has pre(row), which loads the row's other operands and is
@@ -131,9 +138,9 @@ struct EpiAxpby {
         return p;
     }
     __device__ __forceinline__ void apply(int64_t row, const T* acc, const Pre& p, double&, double&) const {
-        T out[NV];
+        T out[NV] = {};
 #pragma unroll
-        for (int k = 0; k < NV; ++k) out[k] = alpha * acc[k] + beta * p.zz[k];
+        for (int k = 0; k < ncomp<NV>(); ++k) out[k] = alpha * acc[k] + beta * p.zz[k];
         VecIO<T, NV>::store(y, row, out);
     }
 };
@@ -161,9 +168,9 @@ struct EpiCheb {
         return p;
     }
     __device__ __forceinline__ void apply(int64_t row, const T* acc, const Pre& p, double&, double&) const {
-        T dd[NV], xx[NV];
+        T dd[NV] = {}, xx[NV] = {};
 #pragma unroll
-        for (int k = 0; k < NV; ++k) {
+        for (int k = 0; k < ncomp<NV>(); ++k) {
             dd[k] = c1 * p.dd[k] + c2 * p.di * (p.bb[k] - acc[k]);
             xx[k] = p.xx[k] + dd[k];
         }
@@ -283,7 +290,7 @@ __global__ void __launch_bounds__(256) k_spmv(int64_t n, const int64_t* __restri
                         T xv[NV];
                         VecIO<T, NV>::load(x, cc[u], xv);
 #pragma unroll
-                        for (int k = 0; k < NV; ++k) acc[k] += aa[u] * xv[k];
+                        for (int k = 0; k < ncomp<NV>(); ++k) acc[k] += aa[u] * xv[k];
                     }
                 }
             }
@@ -291,7 +298,7 @@ __global__ void __launch_bounds__(256) k_spmv(int64_t n, const int64_t* __restri
 #pragma unroll
         for (int o = LPR / 2; o > 0; o >>= 1)
 #pragma unroll
-            for (int k = 0; k < NV; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
+            for (int k = 0; k < ncomp<NV>(); ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
         if (row < n && sub == 0) epi.apply(row, acc, pre, r0, r1);
     }
     if constexpr (Epi::kRed > 0) {
@@ -364,7 +371,7 @@ __device__ __forceinline__ void spmv_sell_body(int64_t n, int64_t nslices, const
                     T xv[NV];
                     VecIO<T, NV>::load(x, cc[u], xv);
 #pragma unroll
-                    for (int k = 0; k < NV; ++k) acc[k] += aa[u] * xv[k];
+                    for (int k = 0; k < ncomp<NV>(); ++k) acc[k] += aa[u] * xv[k];
                 }
             }
         }
@@ -445,7 +452,7 @@ __global__ void __launch_bounds__(256) k_spmv_sell_h(int64_t n, int64_t nslices,
                     float xv[NV];
                     VecIO<float, NV>::load(x, cc[u], xv);
 #pragma unroll
-                    for (int k = 0; k < NV; ++k) acc[k] += aa[u] * xv[k];
+                    for (int k = 0; k < ncomp<NV>(); ++k) acc[k] += aa[u] * xv[k];
                 }
             }
         }
@@ -454,7 +461,7 @@ __global__ void __launch_bounds__(256) k_spmv_sell_h(int64_t n, int64_t nslices,
             VecIO<float, NV>::load(x, row, xr);
             const float d = dg[row];
 #pragma unroll
-            for (int k = 0; k < NV; ++k) acc[k] = acc[k] * hs + d * xr[k];
+            for (int k = 0; k < ncomp<NV>(); ++k) acc[k] = acc[k] * hs + d * xr[k];
             epi.apply(row, acc, pre, r0, r1);
         }
     }
@@ -873,7 +880,7 @@ __global__ void __launch_bounds__(256) k_spmv_staged(const int64_t* __restrict__
                             T xv[NV];
                             VecIO<T, NV>::load(x, cc[u], xv);
 #pragma unroll
-                            for (int k = 0; k < NV; ++k) acc[k] += aa[u] * xv[k];
+                            for (int k = 0; k < ncomp<NV>(); ++k) acc[k] += aa[u] * xv[k];
                         }
                     }
                 }
@@ -881,7 +888,7 @@ __global__ void __launch_bounds__(256) k_spmv_staged(const int64_t* __restrict__
 #pragma unroll
             for (int o = LPR / 2; o > 0; o >>= 1)
 #pragma unroll
-                for (int k = 0; k < NV; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
+                for (int k = 0; k < ncomp<NV>(); ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
             if (row < re && sub == 0) epi.apply(row, acc, pre, r0, r1);
         }
         __syncthreads();  // buffer b consumed before it is refilled
@@ -1555,17 +1562,29 @@ __global__ void k_cheb_first(int64_t n, int nvec, const T* __restrict__ b, const
     x[i] = v;
 }
 
-template <typename T>
-__global__ void k_dense_coarse(int64_t n, int nvec, const double* __restrict__ cinv, const T* __restrict__ b, T* x) {
+// Coarsest level: a warp per row of the dense FP64 inverse, every component of the row from one
+// pass over it.
+template <typename T, int NV>
+__global__ void k_dense_coarse(int64_t n, const double* __restrict__ cinv, const T* __restrict__ b, T* x) {
+    constexpr int NC = ncomp<NV>();
     const int lane = threadIdx.x & 31;
-    const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    if (warp >= n * nvec) return;
-    const int64_t row = warp / nvec;
-    const int k = (int)(warp % nvec);
-    double s = 0.0;
-    for (int64_t j = lane; j < n; j += 32) s += cinv[row * n + j] * (double)b[nvec * j + k];
-    s = warp_sum(s);
-    if (lane == 0) x[nvec * row + k] = (T)s;
+    const int64_t row = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    if (row >= n) return;
+    double s[NC];
+#pragma unroll
+    for (int k = 0; k < NC; ++k) s[k] = 0.0;
+#pragma unroll 4
+    for (int64_t j = lane; j < n; j += 32) {
+        T v[NV];
+        VecIO<T, NV>::load(b, j, v);
+        const double a = cinv[row * n + j];
+#pragma unroll
+        for (int k = 0; k < NC; ++k) s[k] += a * (double)v[k];
+    }
+    T out[NV] = {};
+#pragma unroll
+    for (int k = 0; k < NC; ++k) out[k] = (T)warp_sum(s[k]);
+    if (lane == 0) VecIO<T, NV>::store(x, row, out);
 }
 
 template <typename T>
@@ -1780,8 +1799,7 @@ static void cheb(mpet_ctx* c, AmgHier& h, AmgLevel& L, const T* b, const T* xin,
 template <typename T, int NV>
 static void vcycle(mpet_ctx* c, AmgHier& h, size_t k, const T* b, T* x) {
     if (k + 1 == h.lev.size()) {
-        const int64_t rows = h.ncoarse * NV;
-        k_dense_coarse<T><<<grid_for(rows * 32, 256), 256, 0, c->stream>>>(h.ncoarse, NV, h.cinv, b, x);
+        k_dense_coarse<T, NV><<<grid_for(h.ncoarse * 32, 64), 64, 0, c->stream>>>(h.ncoarse, h.cinv, b, x);
         MPET_CHECK_LAUNCH();
         c->n_launch++;
         return;
