@@ -304,7 +304,7 @@ int mpet_set_amg_setup(mpet_ctx* ctx, int32_t where);
 
 /* The SpMV variant the set-up autotuner chose for each level of hierarchy
  * `block` (bits as for the system matrix; 8: the system's displacement block,
- * 16: matrix-free first level): its operator, prolongation and restriction
+ * 16: matrix-free first level, 64: row tiles): its operator, prolongation and restriction
  * (-1 on the coarsest level).  Arrays of mpet_get_amg_info's level count; any
  * may be NULL.  No reference counterpart (tuning report). */
 int mpet_get_amg_variants(mpet_ctx* ctx, int32_t block, int32_t* a_variant, int32_t* p_variant, int32_t* r_variant);
@@ -385,6 +385,15 @@ int mpet_residual_noalloc(mpet_ctx* ctx, const double* b, const double* x, doubl
 /* y = A x with the assembled values; precision selects FP64 (x, y double)
  * or the FP32 copy (x, y float).  Used by tests and the bandwidth bench. */
 int mpet_spmv(mpet_ctx* ctx, int32_t precision, const void* x, void* y);
+
+/* Products of the preconditioner's level operators by row tiles (variant 64
+ * in mpet_get_amg_variants: a block gathers the x entries of its rows'
+ * distinct columns into shared memory once): offered to the set-up autotuner
+ * for the two finest levels from 20,000 rows on (-1, default), never (0), or
+ * used on every level where they can be built (1).  Takes effect at the next
+ * mpet_setup_preconditioner, which must follow.  No reference counterpart
+ * (engine option and test hook). */
+int mpet_set_row_tiles(mpet_ctx* ctx, int32_t mode);
 
 /* How the inner FP32 iterations of a mixed-precision solve form A x: cell by
  * cell from the geometry and the coefficients of the last mpet_assemble (1),

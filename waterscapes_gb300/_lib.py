@@ -133,6 +133,7 @@ SIGNATURES = {
     "mpet_residual_noalloc": [_P, _P, _P, _P, _P],
     "mpet_spmv": [_P, _I32, _P, _P],
     "mpet_apply_symmetric": [_P, _P, _P],
+    "mpet_set_row_tiles": [_P, _I32],
     "mpet_set_element_product": [_P, _I32],
     "mpet_krylov_product": [_P, _P, _P, ctypes.POINTER(_I32)],
     "mpet_get_spmv_tuning": [_P, _P, ctypes.POINTER(_I32)],

@@ -494,6 +494,8 @@ int mpet_set_batch(mpet_ctx* c, int32_t ninst, const int32_t* vertex_instance) {
     setup_batch(c, ninst, vertex_instance);
     set_instances(c, ninst, vertex_instance);
     release_patches(c);  // patches of one instance each
+    c->pool.release(c->node_order);
+    c->node_order = nullptr;
     c->precond_ready = false;
     c->u_hier_valid = false;
     API_END(c)
@@ -757,8 +759,8 @@ int mpet_get_amg_variants(mpet_ctx* c, int32_t block, int32_t* a_variant, int32_
     for (size_t k = 0; k < h.lev.size(); ++k) {
         const AmgLevel& L = h.lev[k];
         if (a_variant) a_variant[k] = L.mf ? 16 : (L.nb_uu ? 8 : L.A.variant);
-        if (p_variant) p_variant[k] = k + 1 < h.lev.size() ? L.P.variant : -1;
-        if (r_variant) r_variant[k] = k + 1 < h.lev.size() ? L.R.variant : -1;
+        if (p_variant) p_variant[k] = k + 1 < h.lev.size() ? (L.tiled() ? L.Pt : L.P).variant : -1;
+        if (r_variant) r_variant[k] = k + 1 < h.lev.size() ? (L.tiled() ? L.Rt : L.R).variant : -1;
     }
     API_END(c)
 }
@@ -861,6 +863,15 @@ int mpet_spmv(mpet_ctx* c, int32_t precision, const void* x, void* y) {
     } else {
         spmv<double>(c, c->A, 1, (const double*)x, (double*)y);
     }
+    API_END(c)
+}
+
+int mpet_set_row_tiles(mpet_ctx* c, int32_t mode) {
+    API_BEGIN(c)
+    require(mode >= -1 && mode <= 1, MPET_ERR_INVALID, "mode: -1 (autotuned), 0 (never) or 1 (wherever they can be)");
+    c->tile_mode = mode;
+    c->u_hier_valid = false;
+    c->precond_ready = false;
     API_END(c)
 }
 

@@ -124,6 +124,24 @@ struct NodeBlocks {
     int32_t* skl = nullptr;        // batches: lowest and highest instance of each slice's lanes
 };
 
+// Row tiles of a level operator (tile.cuh, variant 64)
+struct RowTiles {
+    int64_t nt = 0;            // tiles (0: none)
+    int R = 0;                 // rows per tile, 256 / R lanes per row
+    int mc = 0;                // columns stored per tile (the most distinct ones, rounded up)
+    bool fp32 = false;         // values in FP32 (else FP64)
+    int32_t* row = nullptr;    // nt * R: rows by decreasing length within a tile, -1 past the end
+    int32_t* col = nullptr;    // nt * mc: distinct columns ascending, then the first one again
+    int64_t* eoff = nullptr;   // nt + 1: first stored entry
+    uint16_t* steps = nullptr; // nt * 8: steps of each warp (a pair of entries per lane and step)
+    void* v = nullptr;         // values, local column ids: pair (step, lane) at eoff + 2 (32 step + lane)
+    uint16_t* lc = nullptr;
+    int32_t* skl = nullptr;    // batches: lowest and highest instance of each tile's rows
+    // first displacement level: the vectors of the level are in tile order (perm[node] = place,
+    // null: node order); columns are places then
+    int32_t* perm = nullptr;
+};
+
 struct Csr {
     int64_t n = 0, m = 0, nnz = 0;
     int64_t* rp = nullptr;
@@ -141,7 +159,7 @@ struct Csr {
     // (needs tiles; with bit 2: the SELL kernel with its epilogue loads after
     // the accumulation, 6 and 7), bit 2 = SELL-32 copy (needs s_off);
     // 8 = node-block copy (9: its FP32 kernel held to 64 registers, 4 blocks per
-    // SM); 32 = SELL-32 with FP16 off-diagonals (needs s_v16)
+    // SM); 32 = SELL-32 with FP16 off-diagonals (needs s_v16); 64 = row tiles (needs rt)
     int variant = 0;
     // mixed precision: variant and lanes per row of the FP64 products when they
     // were tuned apart from the FP32 copy's (-1: none, use variant / lpr)
@@ -170,6 +188,7 @@ struct Csr {
     // (lo > hi for a slice without rows); the products of the batched
     // iterations skip a slice whose instances have all converged
     int32_t* skl = nullptr;
+    RowTiles rt;  // row tiles (level operators only; variant 64)
 };
 
 // Patches of tetrahedra for the FP32 element products (patch.cuh).  Slot p * P + l is lane l
@@ -211,6 +230,11 @@ struct PatchCoef {
 struct AmgLevel {
     Csr A, P, R;       // P: n x nc (prolongation), R = P^T
     bool mf = false;   // products with A formed matrix-free from per-cell data (first displacement level)
+    // the level's transfers and diagonal in the order of its tiles (A.rt.perm), used with A's variant 64
+    Csr Pt, Rt;
+    double* dinv64t = nullptr;
+    float* dinv32t = nullptr;
+    bool tiled() const { return A.rt.perm && A.variant == 64 && !mf; }
     double* dinv64 = nullptr;
     float* dinv32 = nullptr;
     double rho = 1.0;  // spectral radius estimate of D^-1 A
@@ -431,6 +455,8 @@ struct mpet_ctx {
     bool rhs_div_matrix = true;   // pressure rows' divergence term from the node-block product (test hook: false)
     int32_t* u_perm = nullptr;    // P2 node -> row of the spatially ordered first displacement level
     int32_t* u_iperm = nullptr;   // and back (built once per mesh)
+    int tile_mode = -1;           // row tiles of the level operators: -1 autotuned, 0 never, 1 wherever they can be built
+    int32_t* node_order = nullptr;  // P2 nodes along a space-filling curve (instance by instance), for row tiles
     // last device set-up, summed over its hierarchies (ms): block copy, diagonal +
     // spectral radius, strength + aggregation, tentative + smoothed prolongator,
     // transposes, Galerkin products, coarsest inverse, layouts + autotuning
@@ -573,6 +599,16 @@ void build_bc(mpet_ctx* c);
 // c->patch without patches where they cannot serve (2D, FP64 only, HBM short)
 void build_patches(mpet_ctx* c);
 void release_patches(mpet_ctx* c);
+// row tiles of A in the given order of its rows (null: as numbered), vectors nvec wide; A.rt
+// stays empty where they cannot serve (long rows, HBM short)
+// (with an order the level's vectors are to be in tile order: A.rt.perm)
+void build_row_tiles(mpet_ctx* c, Csr& A, const int32_t* order, int nvec, bool fp32);
+// P with its rows, R with its columns, dinv with its entries in the order perm (FP64 CSR only)
+void permute_transfers(mpet_ctx* c, const int32_t* perm, const int32_t* row, const Csr& P, const Csr& R,
+                       const double* dinv, Csr& Pt, Csr& Rt, double** dinvt);
+void release_row_tiles(mpet_ctx* c, RowTiles& r);
+// c->node_order, built when first needed
+const int32_t* node_order(mpet_ctx* c);
 
 // facets.cu
 void build_facets(mpet_ctx* c);
@@ -665,6 +701,7 @@ void refresh_system_copies(mpet_ctx* c);
 void krylov_product_f32(mpet_ctx* c, const float* x, float* y);
 bool spmv_variant_available(const Csr& A, int variant);
 constexpr int SPMV_TILE = 2048;  // entries per staged tile
+constexpr int TILE_MAX_COLS = 2048;  // distinct columns of a row tile
 void destroy_minres_graph(mpet_ctx* c);
 void convert_values_to_f32(mpet_ctx* c);
 

@@ -741,6 +741,23 @@ __global__ void k_patch_fill_shared(int64_t npn, const u64* __restrict__ nkey,
     }
 }
 
+// lower corner and longest side of the vertices' bounding box
+static void bounding_box(mpet_ctx* c, double lo[3], double& ext) {
+    std::vector<double> xyz((size_t)c->nv * 3);
+    MPET_CUDA(cudaMemcpyAsync(xyz.data(), c->x, sizeof(double) * xyz.size(), cudaMemcpyDeviceToHost, c->stream));
+    MPET_CUDA(cudaStreamSynchronize(c->stream));
+    ext = 0.0;
+    for (int k = 0; k < 3; ++k) {
+        double hi = -1e300;
+        lo[k] = 1e300;
+        for (int64_t v = 0; v < c->nv; ++v) {
+            lo[k] = xyz[3 * v + k] < lo[k] ? xyz[3 * v + k] : lo[k];
+            hi = xyz[3 * v + k] > hi ? xyz[3 * v + k] : hi;
+        }
+        ext = hi - lo[k] > ext ? hi - lo[k] : ext;
+    }
+}
+
 void release_patches(mpet_ctx* c) {
     PatchSet& s = c->patch;
     for (void* p : {(void*)s.cell, (void*)s.lid, (void*)s.pn_ptr, (void*)s.pn_nv, (void*)s.pn_node, (void*)s.pn_sh,
@@ -789,19 +806,8 @@ void build_patches(mpet_ctx* c) {
     if (np * P * 10 >= 2147483647LL || c->nnodes >= (1LL << 30)) return;  // (32-bit keys, flag bits)
     TmpBuf d_pstart(sizeof(int32_t) * (np + 1));
     MPET_CUDA(cudaMemcpyAsync(d_pstart.p, pstart.data(), sizeof(int32_t) * (np + 1), cudaMemcpyHostToDevice, st));
-    // bounding box of the vertices
-    std::vector<double> xyz((size_t)c->nv * 3);
-    MPET_CUDA(cudaMemcpyAsync(xyz.data(), c->x, sizeof(double) * xyz.size(), cudaMemcpyDeviceToHost, st));
-    MPET_CUDA(cudaStreamSynchronize(st));
-    double lo[3] = {1e300, 1e300, 1e300}, ext = 0.0;
-    for (int k = 0; k < 3; ++k) {
-        double hi = -1e300;
-        for (int64_t v = 0; v < c->nv; ++v) {
-            lo[k] = xyz[3 * v + k] < lo[k] ? xyz[3 * v + k] : lo[k];
-            hi = xyz[3 * v + k] > hi ? xyz[3 * v + k] : hi;
-        }
-        ext = hi - lo[k] > ext ? hi - lo[k] : ext;
-    }
+    double lo[3], ext;
+    bounding_box(c, lo, ext);
     const double scale = ext > 0.0 ? 16384.0 / ext : 0.0;
     s.cell = c->pool.alloc<int32_t>(np * P);
     {
@@ -939,6 +945,316 @@ void build_patches(mpet_ctx* c) {
     s.P = P;
     s.np = np;
     launch_patch_geometry(c);
+}
+
+
+// ---- row tiles --------------------------------------------------------------------
+
+__global__ void k_node_morton(const double* __restrict__ x, const int64_t* __restrict__ ekey, int64_t nn, int64_t nv,
+                              const int32_t* __restrict__ inst, double lo0, double lo1, double lo2, double scale,
+                              u64* key, int32_t* idx) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= nn) return;
+    const double lo[3] = {lo0, lo1, lo2};
+    u64 m = 0;
+    for (int k = 0; k < 3; ++k) {
+        const double p = i < nv ? x[3 * i + k]
+                                : 0.5 * (x[3 * (ekey[i - nv] / nv) + k] + x[3 * (ekey[i - nv] % nv) + k]);
+        double q = (p - lo[k]) * scale;
+        q = q < 0.0 ? 0.0 : (q > 16383.0 ? 16383.0 : q);
+        m |= spread3((u64)q) << k;
+    }
+    key[i] = ((u64)(inst ? inst[i] : 0) << 42) | m;
+    idx[i] = (int32_t)i;
+}
+
+const int32_t* node_order(mpet_ctx* c) {
+    if (c->node_order) return c->node_order;
+    const int64_t nn = c->nnodes;
+    double lo[3], ext;
+    bounding_box(c, lo, ext);
+    int32_t* o = c->pool.alloc<int32_t>(nn);
+    TmpBuf k0(sizeof(u64) * nn), k1(sizeof(u64) * nn), i0(sizeof(int32_t) * nn);
+    k_node_morton<<<grid_for(nn, 256), 256, 0, c->stream>>>(c->x, c->edge_key, nn, c->nv,
+                                                            c->ninst > 0 ? c->node_inst : nullptr, lo[0], lo[1], lo[2],
+                                                            ext > 0.0 ? 16384.0 / ext : 0.0, k0.as<u64>(),
+                                                            i0.as<int32_t>());
+    MPET_CHECK_LAUNCH();
+    size_t tb = 0;
+    const int eb = 42 + bits_for((u64)(c->ninst > 0 ? c->ninst : 1));
+    MPET_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, k0.as<u64>(), k1.as<u64>(), i0.as<int32_t>(), o, (int)nn, 0,
+                                              eb, c->stream));
+    TmpBuf tmp(tb);
+    MPET_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, tb, k0.as<u64>(), k1.as<u64>(), i0.as<int32_t>(), o, (int)nn, 0,
+                                              eb, c->stream));
+    MPET_CUDA(cudaStreamSynchronize(c->stream));
+    c->node_order = o;
+    return o;
+}
+
+__global__ void k_tile_row_keys(int64_t n, int R, const int32_t* __restrict__ order, const int64_t* __restrict__ rp,
+                                u64* key, int32_t* row) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int32_t r = order ? order[i] : (int32_t)i;
+    key[i] = ((u64)(i / R) << 32) | (u64)(0xffffffffu - (unsigned)(rp[r + 1] - rp[r]));
+    row[i] = r;
+}
+
+__global__ void k_tile_perm(int64_t n, const int32_t* __restrict__ row, int32_t* perm) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i < n) perm[row[i]] = (int32_t)i;
+}
+
+// steps of every warp (its first row is its longest) and the entries of every tile
+__global__ void k_tile_steps(int64_t nt, int R, int lpr, const int32_t* __restrict__ row,
+                             const int64_t* __restrict__ rp, uint16_t* steps, int64_t* ent) {
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (t >= nt) return;
+    const int rw = 32 / lpr;
+    int64_t sum = 0;
+    for (int w = 0; w < 8; ++w) {
+        const int32_t r = row[t * R + w * rw];
+        const int64_t len = r >= 0 ? rp[r + 1] - rp[r] : 0;
+        const int64_t s = (len + 2 * lpr - 1) / (2 * lpr);
+        steps[t * 8 + w] = (uint16_t)(s < 65535 ? s : 65535);
+        sum += s;
+    }
+    ent[t] = sum * 64;
+}
+
+__global__ void k_tile_col_keys(int64_t nrows, int R, const int32_t* __restrict__ row, const int64_t* __restrict__ rp,
+                                const int32_t* __restrict__ ci, const int32_t* __restrict__ perm, u64* key) {
+    const int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 3;  // eight lanes per row
+    const int l = threadIdx.x & 7;
+    if (i >= nrows || row[i] < 0) return;
+    const int32_t r = row[i];
+    for (int64_t e = rp[r] + l; e < rp[r + 1]; e += 8) key[e] = ((u64)(i / R) << 32) | (u64)(unsigned)(perm ? perm[ci[e]] : ci[e]);
+}
+
+__global__ void k_tile_cptr(const u64* __restrict__ key, int64_t n, int64_t nt, int32_t* cptr) {
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (t <= nt) cptr[t] = (int32_t)lower_bound_u64(key, n, (u64)t << 32);
+}
+
+// the tiles' column lists, mc apart, padded with the first column
+__global__ void k_tile_cols(int64_t nt, int mc, const u64* __restrict__ key, const int32_t* __restrict__ cptr,
+                            int32_t* col) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= nt * mc) return;
+    const int64_t t = i / mc;
+    const int q = (int)(i % mc), n = cptr[t + 1] - cptr[t];
+    col[i] = n > 0 ? (int32_t)(key[cptr[t] + (q < n ? q : 0)] & 0xffffffffu) : 0;
+}
+
+template <typename T>
+__global__ void k_tile_fill(int64_t nt, int R, int lpr, const int32_t* __restrict__ row,
+                            const int64_t* __restrict__ rp, const int32_t* __restrict__ ci,
+                            const int32_t* __restrict__ perm, const double* __restrict__ v,
+                            const int32_t* __restrict__ cptr, int mc, const int32_t* __restrict__ col,
+                            const int64_t* __restrict__ eoff, const uint16_t* __restrict__ steps, T* tv,
+                            uint16_t* tl) {
+    const int64_t th = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (th >= nt * 256) return;
+    const int64_t t = th >> 8;
+    const int w = (int)(th >> 5) & 7, lane = (int)th & 31;
+    const int rw = 32 / lpr, sub = lane % lpr;
+    int base = 0;
+    for (int q = 0; q < w; ++q) base += steps[t * 8 + q];
+    const int n = steps[t * 8 + w];
+    const int32_t r = row[t * R + w * rw + lane / lpr];
+    const int64_t b = r >= 0 ? rp[r] : 0, len = r >= 0 ? rp[r + 1] - b : 0;
+    const int32_t* cs = col + t * mc;
+    const int nc = cptr[t + 1] - cptr[t];
+    // padding: value 0 at the row's last column (a valid place, as in the SELL copy)
+    auto place = [&](int64_t e) { return (uint16_t)lower_bound_i32(cs, nc, perm ? perm[ci[e]] : ci[e]); };
+    const uint16_t pad = len > 0 ? place(b + len - 1) : 0;
+    for (int q = 0; q < n; ++q)
+        for (int h = 0; h < 2; ++h) {
+            const int64_t e = 2 * ((int64_t)q * lpr + sub) + h;
+            const int64_t o = eoff[t] + 2 * ((int64_t)(base + q) * 32 + lane) + h;
+            tv[o] = e < len ? (T)v[b + e] : T(0);
+            tl[o] = e < len ? place(b + e) : pad;
+        }
+}
+
+void release_row_tiles(mpet_ctx* c, RowTiles& r) {
+    for (void* p : {(void*)r.row, (void*)r.perm, (void*)r.col, (void*)r.eoff, (void*)r.steps, r.v, (void*)r.lc,
+                    (void*)r.skl})
+        c->pool.release(p);
+    r = RowTiles();
+}
+
+// false: a tile of R rows does not fit in shared memory
+static bool build_tiles_of(mpet_ctx* c, Csr& A, const int32_t* order, int nvec, bool fp32, int R) {
+    const int lpr = 256 / R;
+    RowTiles& r = A.rt;
+    const int64_t n = A.n, nnz = A.nnz;
+    cudaStream_t st = c->stream;
+    const int64_t nt = (n + R - 1) / R;
+    const int T = 256;
+    r.row = c->pool.alloc<int32_t>(nt * R);
+    MPET_CUDA(cudaMemsetAsync(r.row, 0xff, sizeof(int32_t) * nt * R, st));
+    {
+        TmpBuf k0(sizeof(u64) * n), k1(sizeof(u64) * n), i0(sizeof(int32_t) * n);
+        k_tile_row_keys<<<grid_for(n, T), T, 0, st>>>(n, R, order, A.rp, k0.as<u64>(), i0.as<int32_t>());
+        MPET_CHECK_LAUNCH();
+        size_t tb = 0;
+        const int eb = 32 + bits_for((u64)nt);
+        MPET_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, k0.as<u64>(), k1.as<u64>(), i0.as<int32_t>(), r.row,
+                                                  (int)n, 0, eb, st));
+        TmpBuf tmp(tb);
+        MPET_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, tb, k0.as<u64>(), k1.as<u64>(), i0.as<int32_t>(), r.row,
+                                                  (int)n, 0, eb, st));
+        MPET_CUDA(cudaStreamSynchronize(st));
+    }
+    if (order) {
+        r.perm = c->pool.alloc<int32_t>(n);
+        k_tile_perm<<<grid_for(n, T), T, 0, st>>>(n, r.row, r.perm);
+        MPET_CHECK_LAUNCH();
+    }
+    r.steps = c->pool.alloc<uint16_t>(nt * 8);
+    r.eoff = c->pool.alloc<int64_t>(nt + 1);
+    k_tile_steps<<<grid_for(nt, T), T, 0, st>>>(nt, R, lpr, r.row, A.rp, r.steps, r.eoff);
+    MPET_CHECK_LAUNCH();
+    std::vector<int64_t> eo(nt + 1);
+    MPET_CUDA(cudaMemcpyAsync(eo.data(), r.eoff, sizeof(int64_t) * nt, cudaMemcpyDeviceToHost, st));
+    MPET_CUDA(cudaStreamSynchronize(st));
+    int64_t total = 0, max_ent = 0;
+    for (int64_t t = 0; t < nt; ++t) {
+        const int64_t e = eo[t];
+        max_ent = std::max(max_ent, e);
+        eo[t] = total;
+        total += e;
+    }
+    eo[nt] = total;
+    MPET_CUDA(cudaMemcpyAsync(r.eoff, eo.data(), sizeof(int64_t) * (nt + 1), cudaMemcpyHostToDevice, st));
+    if (max_ent > 65536) {  // (bounds the steps of a warp)
+        release_row_tiles(c, r);
+        return false;
+    }
+    // distinct columns
+    u64* key = nullptr;
+    int64_t ncol = 0;
+    {
+        TmpBuf keys(sizeof(u64) * nnz);
+        k_tile_col_keys<<<grid_for(nt * R * 8, T), T, 0, st>>>(nt * R, R, r.row, A.rp, A.ci, r.perm, keys.as<u64>());
+        MPET_CHECK_LAUNCH();
+        ncol = sort_unique(c, keys.as<u64>(), nnz, 32 + bits_for((u64)nt), &key);
+    }
+    TmpBuf cptr(sizeof(int32_t) * (nt + 1));
+    k_tile_cptr<<<grid_for(nt + 1, T), T, 0, st>>>(key, ncol, nt, cptr.as<int32_t>());
+    MPET_CHECK_LAUNCH();
+    std::vector<int32_t> cp(nt + 1);
+    MPET_CUDA(cudaMemcpyAsync(cp.data(), cptr.p, sizeof(int32_t) * (nt + 1), cudaMemcpyDeviceToHost, st));
+    MPET_CUDA(cudaStreamSynchronize(st));
+    for (int64_t t = 0; t < nt; ++t) r.mc = std::max(r.mc, cp[t + 1] - cp[t]);
+    r.mc = (r.mc + 31) / 32 * 32;
+    // (x in shared memory: three blocks per SM at least)
+    if ((size_t)r.mc * nvec * (fp32 ? 4 : 8) > 72 * 1024 || r.mc > TILE_MAX_COLS) {
+        c->pool.release(key);
+        release_row_tiles(c, r);
+        return false;
+    }
+    r.col = c->pool.alloc<int32_t>(nt * r.mc);
+    k_tile_cols<<<grid_for(nt * r.mc, T), T, 0, st>>>(nt, r.mc, key, cptr.as<int32_t>(), r.col);
+    MPET_CHECK_LAUNCH();
+    MPET_CUDA(cudaStreamSynchronize(st));
+    c->pool.release(key);
+    r.lc = c->pool.alloc<uint16_t>(total);
+    if (fp32) {
+        r.v = c->pool.alloc<float>(total);
+        k_tile_fill<float><<<grid_for(nt * 256, T), T, 0, st>>>(nt, R, lpr, r.row, A.rp, A.ci, r.perm, A.v64,
+                                                                     cptr.as<int32_t>(), r.mc,
+                                                                r.col, r.eoff, r.steps, (float*)r.v, r.lc);
+    } else {
+        r.v = c->pool.alloc<double>(total);
+        k_tile_fill<double><<<grid_for(nt * 256, T), T, 0, st>>>(nt, R, lpr, r.row, A.rp, A.ci, r.perm, A.v64,
+                                                                     cptr.as<int32_t>(), r.mc,
+                                                                 r.col, r.eoff, r.steps, (double*)r.v, r.lc);
+    }
+    MPET_CHECK_LAUNCH();
+    MPET_CUDA(cudaStreamSynchronize(st));
+    r.fp32 = fp32;
+    r.R = R;
+    r.nt = nt;
+    return true;
+}
+
+void build_row_tiles(mpet_ctx* c, Csr& A, const int32_t* order, int nvec, bool fp32) {
+    const int64_t n = A.n, nnz = A.nnz;
+    if (n == 0 || nnz == 0 || nnz >= 2147483647LL || !A.v64) return;
+    const size_t ev = (fp32 ? 4 : 8) + 2;
+    if (!device_fits(c, (size_t)nnz * (24 + ev + ev / 4) + (size_t)n * 24)) return;
+    // Rows per tile: 256 (the more rows, the fewer x entries per row: the displacement level at
+    // 64^3 takes 1650, 1237 and 1071 us with 64, 128 and 256, 1157 with 512), less on a small level
+    // so that every SM has two tiles.
+    int R = 256;
+    while (R > 32 && n < (int64_t)R * 304) R >>= 1;
+    for (; R >= 32; R >>= 1)
+        if (build_tiles_of(c, A, order, nvec, fp32, R)) return;
+}
+
+// ---- a level's transfers in tile order -----------------------------------------------
+
+__global__ void k_perm_len(int64_t n, const int32_t* __restrict__ row, const int64_t* __restrict__ rp, int64_t* len) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i <= n) len[i] = i < n ? rp[row[i] + 1] - rp[row[i]] : 0;
+}
+
+__global__ void k_perm_rows(int64_t n, const int32_t* __restrict__ row, const int64_t* __restrict__ rp,
+                            const int32_t* __restrict__ ci, const double* __restrict__ v,
+                            const int64_t* __restrict__ rpt, int32_t* cit, double* vt,
+                            const double* __restrict__ dinv, double* dinvt) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int64_t b = rp[row[i]], len = rp[row[i] + 1] - b;
+    for (int64_t e = 0; e < len; ++e) {
+        cit[rpt[i] + e] = ci[b + e];
+        vt[rpt[i] + e] = v[b + e];
+    }
+    dinvt[i] = dinv[row[i]];
+}
+
+__global__ void k_perm_cols(int64_t nnz, const int32_t* __restrict__ ci, const int32_t* __restrict__ perm,
+                            int32_t* cit) {
+    const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (e < nnz) cit[e] = perm[ci[e]];
+}
+
+void permute_transfers(mpet_ctx* c, const int32_t* perm, const int32_t* row, const Csr& P, const Csr& R,
+                       const double* dinv, Csr& Pt, Csr& Rt, double** dinvt) {
+    cudaStream_t st = c->stream;
+    Pt.n = P.n;
+    Pt.m = P.m;
+    Pt.nnz = P.nnz;
+    Pt.rp = c->pool.alloc<int64_t>(P.n + 1);
+    Pt.ci = c->pool.alloc<int32_t>(P.nnz);
+    Pt.v64 = c->pool.alloc<double>(P.nnz);
+    *dinvt = c->pool.alloc<double>(P.n);
+    {
+        TmpBuf len(sizeof(int64_t) * (P.n + 1));
+        k_perm_len<<<grid_for(P.n + 1, 256), 256, 0, st>>>(P.n, row, P.rp, len.as<int64_t>());
+        MPET_CHECK_LAUNCH();
+        size_t tb = 0;
+        MPET_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, len.as<int64_t>(), Pt.rp, (int)(P.n + 1), st));
+        TmpBuf tmp(tb);
+        MPET_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, tb, len.as<int64_t>(), Pt.rp, (int)(P.n + 1), st));
+        k_perm_rows<<<grid_for(P.n, 256), 256, 0, st>>>(P.n, row, P.rp, P.ci, P.v64, Pt.rp, Pt.ci, Pt.v64, dinv,
+                                                        *dinvt);
+        MPET_CHECK_LAUNCH();
+        MPET_CUDA(cudaStreamSynchronize(st));
+    }
+    Rt.n = R.n;
+    Rt.m = R.m;
+    Rt.nnz = R.nnz;
+    Rt.rp = c->pool.alloc<int64_t>(R.n + 1);
+    Rt.ci = c->pool.alloc<int32_t>(R.nnz);
+    Rt.v64 = c->pool.alloc<double>(R.nnz);
+    MPET_CUDA(cudaMemcpyAsync(Rt.rp, R.rp, sizeof(int64_t) * (R.n + 1), cudaMemcpyDeviceToDevice, st));
+    MPET_CUDA(cudaMemcpyAsync(Rt.v64, R.v64, sizeof(double) * R.nnz, cudaMemcpyDeviceToDevice, st));
+    k_perm_cols<<<grid_for(R.nnz, 256), 256, 0, st>>>(R.nnz, R.ci, perm, Rt.ci);
+    MPET_CHECK_LAUNCH();
 }
 
 }  // namespace mpet

@@ -109,6 +109,7 @@ __host__ __device__ constexpr int ncomp() { return NV == 4 ? 3 : NV; }
 template <typename T, int NV>
 struct EpiStore {
     T* y;
+    static constexpr bool kTile = false;  // runs with the row-tile kernel
     static constexpr int kRed = 0;
     static constexpr bool kSystem = NV == 1;  // runs with the node-block system kernel
     struct Pre {};
@@ -124,6 +125,7 @@ struct EpiAxpby {
     T* y;
     const T* z;
     T alpha, beta;
+    static constexpr bool kTile = true;  // runs with the row-tile kernel
     static constexpr int kRed = 0;
     static constexpr bool kSystem = false;
     struct Pre {
@@ -154,6 +156,7 @@ struct EpiCheb {
     T* xout;
     const T* dinv;
     T c1, c2;
+    static constexpr bool kTile = true;  // runs with the row-tile kernel
     static constexpr int kRed = 0;
     static constexpr bool kSystem = false;
     struct Pre {
@@ -194,6 +197,7 @@ struct EpiMinres {
     const T* r1;
     const T* v;
     const MinresScalars* sc;
+    static constexpr bool kTile = false;  // runs with the row-tile kernel
     static constexpr int kRed = 1;
     static constexpr bool kSystem = true;
     struct Pre {
@@ -213,6 +217,7 @@ struct EpiResid64 {
     double* r;
     const double* b;
     const double* dinv;
+    static constexpr bool kTile = false;  // runs with the row-tile kernel
     static constexpr int kRed = 2;
     static constexpr bool kSystem = true;
     struct Pre {
@@ -1169,6 +1174,7 @@ static void launch_nb(mpet_ctx* c, const NodeBlocks& nb, const T* x, const Epi& 
 // b += the pressure rows' displacement-column products (FP64 right-hand side term)
 struct EpiAddRhs {
     double* b;
+    static constexpr bool kTile = false;  // runs with the row-tile kernel
     static constexpr int kRed = 0;
     static constexpr bool kSystem = true;
     struct Pre {};
@@ -1220,6 +1226,8 @@ const double* sell_vals<double>(const Csr& A) { return A.s_v64; }
 template <>
 const float* sell_vals<float>(const Csr& A) { return A.s_v32; }
 
+#include "tile.cuh"
+
 template <typename T, int NV, class Epi>
 static void launch_spmv(mpet_ctx* c, const Csr& A, const T* va, const T* x, const Epi& epi) {
     // FP64 products of a matrix tuned on its FP32 copy use their own tuning when they have one
@@ -1229,6 +1237,12 @@ static void launch_spmv(mpet_ctx* c, const Csr& A, const T* va, const T* x, cons
     if constexpr (NV == 1 && Epi::kSystem) {
         if ((variant == 8 || variant == 9) && A.nb && nb_vals<T>(*A.nb) && va == vals<T>(A)) {
             launch_nb<T>(c, *A.nb, x, epi, variant == 9);
+            return;
+        }
+    }
+    if constexpr (Epi::kTile) {
+        if (variant == 64 && A.rt.nt > 0 && A.rt.fp32 == (sizeof(T) == 4) && va == vals<T>(A)) {
+            launch_tile<T, NV>(c, A.rt, A.n, x, epi);
             return;
         }
     }
@@ -1414,15 +1428,16 @@ static void level_spmv(mpet_ctx* c, const AmgLevel& L, const T* x, const Epi& ep
 template <typename T>
 static const T* dinv_of(const AmgLevel& L);
 template <>
-const double* dinv_of<double>(const AmgLevel& L) { return L.dinv64; }
+const double* dinv_of<double>(const AmgLevel& L) { return L.tiled() ? L.dinv64t : L.dinv64; }
 template <>
-const float* dinv_of<float>(const AmgLevel& L) { return L.dinv32; }
+const float* dinv_of<float>(const AmgLevel& L) { return L.tiled() ? L.dinv32t : L.dinv32; }
 
 // Variant v (bits as in Csr::variant) can run on A with its current lanes
 // per row: staged needs row tiles, SELL its copy, 8 entries per lane (CSR)
 // 32 lanes per row.
 bool spmv_variant_available(const Csr& A, int v) {
     if (v == 32) return A.s_v16 != nullptr;
+    if (v == 64) return A.rt.nt > 0;
     if (v == 8) return A.nb != nullptr;
     if (v == 9) return A.nb != nullptr && A.v32 != nullptr;  // FP32 node blocks at 4 blocks per SM
     if (v < 0 || v > 5) return false;
@@ -1454,7 +1469,8 @@ static void autotune_matrix(mpet_ctx* c, Csr& A, const T* x, const Epi& epi, dou
     for (int lpr : {lpr0, lpr0 / 2, lpr0 * 2}) {
         if ((lpr < 4 || lpr > 32) && lpr != lpr0) continue;
         A.lpr = lpr;
-        for (int v : {0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 32}) {
+        for (int v : {0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 32, 64}) {
+            if (v == 64 && (!Epi::kTile || lpr != lpr0)) continue;
             if (v == 32 && (sizeof(T) != 4 || !A.s_v16 || lpr != lpr0)) continue;
             if (v == 9 && sizeof(T) != 4) continue;
             if (!spmv_variant_available(A, v) || (v >= 4 && v < 8 && (!sell_vals<T>(A) || lpr != lpr0))) continue;
@@ -1491,6 +1507,7 @@ static void autotune_matrix(mpet_ctx* c, Csr& A, const T* x, const Epi& epi, dou
     }
     A.variant = best_v;
     A.lpr = best_lpr;
+    if (Epi::kTile && c->tile_mode == 1 && A.rt.nt > 0) A.variant = 64;
     c->n_launch = l0;
 }
 
@@ -1536,8 +1553,10 @@ static void autotune_hier(mpet_ctx* c, AmgHier& h) {
         if (k + 1 < h.lev.size()) {
             AmgLevel& C = h.lev[k + 1];
             MPET_CUDA(cudaMemsetAsync(C.x, 0, sizeof(double) * C.A.n * NV, c->stream));
-            autotune_matrix<T, NV>(c, L.P, (const T*)C.x, EpiAxpby<T, NV>{(T*)L.t0, (const T*)L.t0, T(1), T(1)});
-            autotune_matrix<T, NV>(c, L.R, (const T*)L.r, EpiStore<T, NV>{(T*)C.b});
+            Csr& P = L.tiled() ? L.Pt : L.P;
+            Csr& R = L.tiled() ? L.Rt : L.R;
+            autotune_matrix<T, NV>(c, P, (const T*)C.x, EpiAxpby<T, NV>{(T*)L.t0, (const T*)L.t0, T(1), T(1)});
+            autotune_matrix<T, NV>(c, R, (const T*)L.r, EpiStore<T, NV>{(T*)C.b});
         }
     }
 }
@@ -1810,9 +1829,11 @@ static void vcycle(mpet_ctx* c, AmgHier& h, size_t k, const T* b, T* x) {
     T* r = (T*)L.r;
     cheb<T, NV>(c, h, L, b, nullptr, xs);
     level_spmv<T, NV>(c, L, xs, EpiAxpby<T, NV>{r, b, T(-1), T(1)});
-    launch_spmv<T, NV>(c, L.R, vals<T>(L.R), r, EpiStore<T, NV>{(T*)C.b});
+    const Csr& R = L.tiled() ? L.Rt : L.R;
+    const Csr& P = L.tiled() ? L.Pt : L.P;
+    launch_spmv<T, NV>(c, R, vals<T>(R), r, EpiStore<T, NV>{(T*)C.b});
     vcycle<T, NV>(c, h, k + 1, (const T*)C.b, (T*)C.x);
-    launch_spmv<T, NV>(c, L.P, vals<T>(L.P), (const T*)C.x, EpiAxpby<T, NV>{xs, xs, T(1), T(1)});
+    launch_spmv<T, NV>(c, P, vals<T>(P), (const T*)C.x, EpiAxpby<T, NV>{xs, xs, T(1), T(1)});
     cheb<T, NV>(c, h, L, b, xs, x);
 }
 
@@ -1955,9 +1976,10 @@ static void precond(mpet_ctx* c, const T* r, T* z) {
         const int64_t nodes = c->nnodes;
         T* bin = (T*)hu.pack_in;
         T* xout = (T*)hu.pack_out;
-        k_pack34<T><<<grid_for(nodes, 256), 256, 0, main>>>(nodes, c->dim, r, bin, hu.perm);
+        const int32_t* perm = hu.lev[0].tiled() ? hu.lev[0].A.rt.perm : hu.perm;
+        k_pack34<T><<<grid_for(nodes, 256), 256, 0, main>>>(nodes, c->dim, r, bin, perm);
         vcycle<T, 4>(c, hu, 0, bin, xout);
-        k_unpack43<T><<<grid_for(nodes, 256), 256, 0, main>>>(nodes, c->dim, xout, z, hu.perm);
+        k_unpack43<T><<<grid_for(nodes, 256), 256, 0, main>>>(nodes, c->dim, xout, z, perm);
         MPET_CHECK_LAUNCH();
         c->n_launch += 2;
     }
@@ -3016,6 +3038,22 @@ __global__ void k_skl_nb(int64_t ns, const int32_t* __restrict__ perm, const int
     skl[2 * s + 1] = hi;
 }
 
+// row tiles: the rows of each tile
+__global__ void k_skl_tiles(int64_t nt, int R, const int32_t* __restrict__ row, const int32_t* __restrict__ inst,
+                            int32_t* skl) {
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (t >= nt) return;
+    int lo = INT_MAX, hi = -1;
+    for (int q = 0; q < R; ++q) {
+        const int32_t r = row[t * R + q];
+        if (r < 0) continue;
+        lo = inst[r] < lo ? inst[r] : lo;
+        hi = inst[r] > hi ? inst[r] : hi;
+    }
+    skl[2 * t] = hi >= 0 ? lo : 0;
+    skl[2 * t + 1] = hi;
+}
+
 // coarse rows take the instance of the fine rows that prolongate from them
 // (all of one instance: instance meshes share no entry)
 __global__ void k_coarse_inst(int64_t nf, const int64_t* __restrict__ rp, const int32_t* __restrict__ ci,
@@ -3060,11 +3098,25 @@ static void hier_skip_maps(mpet_ctx* c, AmgHier& h, const int32_t* inst0, int64_
             MPET_CHECK_LAUNCH();
         }
         L.A.skl = skl_of_rows(c, n, L.inst);
+        if (L.A.rt.nt > 0) {
+            RowTiles& r = L.A.rt;
+            r.skl = c->pool.alloc<int32_t>(2 * r.nt);
+            k_skl_tiles<<<grid_for(r.nt, 256), 256, 0, c->stream>>>(r.nt, r.R, r.row, L.inst, r.skl);
+            MPET_CHECK_LAUNCH();
+        }
     }
     for (size_t k = 0; k + 1 < h.lev.size(); ++k) {
         AmgLevel& L = h.lev[k];
         L.P.skl = skl_of_rows(c, L.P.n, L.inst);
         L.R.skl = skl_of_rows(c, L.R.n, h.lev[k + 1].inst);
+        if (L.A.rt.perm) {
+            TmpBuf it(sizeof(int32_t) * L.A.n);
+            k_gather_i32<<<grid_for(L.A.n, 256), 256, 0, c->stream>>>(L.A.n, L.A.rt.row, L.inst, it.as<int32_t>());
+            MPET_CHECK_LAUNCH();
+            L.Pt.skl = skl_of_rows(c, L.A.n, it.as<int32_t>());
+            L.Rt.skl = skl_of_rows(c, L.Rt.n, h.lev[k + 1].inst);
+            MPET_CUDA(cudaStreamSynchronize(c->stream));
+        }
     }
 }
 
@@ -3615,6 +3667,7 @@ static void release_csr(mpet_ctx* c, Csr& A) {
                     (void*)A.s_ci, (void*)A.s_v32, (void*)A.s_v64, (void*)A.skl, (void*)A.s_v16,
                     (void*)A.s_d32})
         c->pool.release(p);
+    release_row_tiles(c, A.rt);
     A = Csr();
 }
 
@@ -3623,7 +3676,9 @@ void release_hier(mpet_ctx* c, AmgHier& h) {
         release_csr(c, L.A);
         release_csr(c, L.P);
         release_csr(c, L.R);
-        for (void* p : {(void*)L.dinv64, (void*)L.dinv32, L.x, L.b, L.r, L.d, L.t0, L.t1, (void*)L.inst})
+        release_csr(c, L.Pt);
+        release_csr(c, L.Rt);
+        for (void* p : {(void*)L.dinv64, (void*)L.dinv32, (void*)L.dinv64t, (void*)L.dinv32t, L.x, L.b, L.r, L.d, L.t0, L.t1, (void*)L.inst})
             c->pool.release(p);
     }
     h.lev.clear();
@@ -3632,6 +3687,30 @@ void release_hier(mpet_ctx* c, AmgHier& h) {
     h.pack_in = h.pack_out = nullptr;
     h.ncoarse = 0;
     h.perm = h.iperm = nullptr;  // the context owns the permutation
+}
+
+static void finish_device_csr(mpet_ctx* c, Csr& d, bool fp32);
+
+// P, R and the inverse diagonal of a level whose tiles have their own order
+static void tiled_transfers(mpet_ctx* c, AmgLevel& L, bool fp32) {
+    if (!L.A.rt.perm) return;
+    permute_transfers(c, L.A.rt.perm, L.A.rt.row, L.P, L.R, L.dinv64, L.Pt, L.Rt, &L.dinv64t);
+    finish_device_csr(c, L.Pt, fp32);
+    finish_device_csr(c, L.Rt, fp32);
+    if (fp32) {
+        L.dinv32t = c->pool.alloc<float>(L.A.n);
+        k_f64_to_f32<<<grid_for(L.A.n, 256), 256, 0, c->stream>>>(L.A.n, L.dinv64t, L.dinv32t);
+        MPET_CHECK_LAUNCH();
+    }
+}
+
+// Row tiles of the large level operators: below 20,000 rows their set-up (a millisecond or
+// two of sorts) is not repaid.  The P2 nodes go along a space-filling curve (vertices and edges
+// are numbered apart), other levels as they are numbered.
+static void level_tiles(mpet_ctx* c, AmgHier& h, size_t k, int nvec, bool fp32) {
+    Csr& A = h.lev[k].A;
+    if (c->tile_mode == 0 || (c->tile_mode < 0 && (A.n < 20000 || k > 1))) return;
+    build_row_tiles(c, A, nvec == 4 && k == 0 && !h.perm && A.n == c->nnodes ? node_order(c) : nullptr, nvec, fp32);
 }
 
 void upload_amg(mpet_ctx* c, AmgHier& h, const HostAmg& ha, int nvec, bool fp32) {
@@ -3647,6 +3726,7 @@ void upload_amg(mpet_ctx* c, AmgHier& h, const HostAmg& ha, int nvec, bool fp32)
         AmgLevel& L = h.lev[k];
         upload_csr(c, hl.A, L.A, fp32);
         if (fp32 && k == 0) build_sell_half(c, L.A);
+        level_tiles(c, h, k, nvec, fp32);
         L.rho = hl.rho;
         const int64_t n = hl.A.n;
         L.dinv64 = c->pool.alloc<double>(n);
@@ -3659,6 +3739,7 @@ void upload_amg(mpet_ctx* c, AmgHier& h, const HostAmg& ha, int nvec, bool fp32)
         if (k + 1 < ha.lev.size()) {
             upload_csr(c, hl.P, L.P, fp32);
             upload_csr(c, hl.R, L.R, fp32);
+            tiled_transfers(c, L, fp32);
         }
         const int64_t nn = n * nvec;
         L.x = c->pool.alloc<double>(nn);
@@ -3711,6 +3792,7 @@ void finish_device_hier(mpet_ctx* c, AmgHier& h, int nvec, bool fp32) {
         AmgLevel& L = h.lev[k];
         finish_device_csr(c, L.A, fp32);
         if (fp32 && k == 0) build_sell_half(c, L.A);
+        level_tiles(c, h, k, nvec, fp32);
         const int64_t n = L.A.n;
         if (fp32) {
             L.dinv32 = c->pool.alloc<float>(n);
@@ -3720,6 +3802,7 @@ void finish_device_hier(mpet_ctx* c, AmgHier& h, int nvec, bool fp32) {
         if (k + 1 < h.lev.size()) {
             finish_device_csr(c, L.P, fp32);
             finish_device_csr(c, L.R, fp32);
+            tiled_transfers(c, L, fp32);
         }
         const int64_t nn = n * nvec;
         L.x = c->pool.alloc<double>(nn);
