@@ -468,6 +468,7 @@ struct mpet_ctx {
     double* est_sum = nullptr;
     int32_t* est_bad = nullptr;
     double* partials = nullptr;   // reduction partials
+    unsigned* red_cnt = nullptr;  // arrivals of a reduction's blocks (zero between launches)
     mpet::MinresScalars* sc = nullptr;
     mpet::MinresScalars* sc_host = nullptr;  // pinned
 

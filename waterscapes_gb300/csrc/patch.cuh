@@ -92,7 +92,7 @@ struct DotAcc {
 struct PatchOut {
     float* y;
     const float* r1;
-    const MinresScalars* sc;
+    MinresScalars* sc;
 };
 
 template <bool DOT>
@@ -105,17 +105,18 @@ __device__ __forceinline__ void patch_row(const PatchOut& O, int64_t row, float 
     O.y[row] = acc;
 }
 
+// this block's partial of x . y; the block of the second kernel (first > 0) that arrives last
+// adds the partials of both and takes the scalar step (alfa)
 template <bool DOT>
-__device__ __forceinline__ void patch_dot_finish(const DotAcc& dot, double* partials, int first, int total) {
+__device__ __forceinline__ void patch_dot_finish(const DotAcc& dot, double* partials, int first, unsigned* cnt,
+                                                 MinresScalars* sc) {
     if (DOT) {
         __shared__ double sh[8];
         const double s = block_sum256(dot.value(), sh);
-        if (threadIdx.x == 0) {
-            partials[first + blockIdx.x] = s;
-            // the second kernel's first block clears the partials that neither kernel has
-            if (first > 0 && blockIdx.x == 0)
-                for (int p = total; p < NB_RED; ++p) partials[p] = 0.0;
-        }
+        if (threadIdx.x == 0) partials[first + blockIdx.x] = s;
+        if (first == 0 || !last_block(cnt)) return;
+        const double t = sum_partials_n(partials, first + gridDim.x, sh);
+        if (threadIdx.x == 0) mr_alfa_one(sc, t);
     }
 }
 
@@ -326,7 +327,7 @@ __global__ void __launch_bounds__(256, J <= 4 ? 3 : 2) k_patch_sys(PatchArgs A, 
         }
         __syncthreads();  // the next patch reuses the shared arrays
     }
-    patch_dot_finish<DOT>(dot, partials, 0, 0);
+    patch_dot_finish<DOT>(dot, partials, 0, nullptr, nullptr);
 }
 
 // rows of the nodes of several patches: items 0..nsh-1 the u rows of a shared node, then the
@@ -336,7 +337,7 @@ __global__ void __launch_bounds__(256) k_patch_sys_shared(int64_t nsh, const int
                                                           const int32_t* __restrict__ sh_ptr,
                                                           const float4* __restrict__ part, PatchDims D, int bc,
                                                           const float* __restrict__ x, PatchOut O, double* partials,
-                                                          int first, int total,
+                                                          int first, unsigned* cnt,
                                                           const int32_t* __restrict__ node_inst,
                                                           const double* __restrict__ skip) {
     const float cr = DOT ? O.sc->f_c_r1 : 0.f;
@@ -386,7 +387,7 @@ __global__ void __launch_bounds__(256) k_patch_sys_shared(int64_t nsh, const int
             patch_row<DOT>(O, row, bc && D.dof_bc[row] ? xv : a, r1, xv, cr, dot);
         }
     }
-    patch_dot_finish<DOT>(dot, partials, first, total);
+    patch_dot_finish<DOT>(dot, partials, first, cnt, O.sc);
 }
 
 template <int J, bool DOT>
@@ -402,7 +403,7 @@ static void launch_patch_sys_j(mpet_ctx* c, const float* x, const PatchOut& O) {
     MPET_CUDA(cudaFuncSetAttribute(k_patch_sys<J, DOT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     k_patch_sys<J, DOT><<<g1, s.P, sm, c->stream>>>(patch_args(c), D, c->patch_coef, x, O, c->partials, skip);
     k_patch_sys_shared<J, DOT><<<g2, 256, 0, c->stream>>>(s.nsh, s.sh_node, s.sh_ptr, (const float4*)s.part, D,
-                                                          c->patch_coef.bc, x, O, c->partials, g1, g1 + g2,
+                                                          c->patch_coef.bc, x, O, c->partials, g1, c->red_cnt,
                                                           c->node_inst, skip);
     MPET_CHECK_LAUNCH();
     c->n_launch += 2;
@@ -436,13 +437,17 @@ static void krylov_product(mpet_ctx* c, const T* x, T* y) {
     launch_spmv<T, 1>(c, c->A, vals<T>(c->A), x, EpiStore<T, 1>{y});
 }
 
+// the Lanczos step of MINRES: y = A v - (beta / oldb) r1 and alfa = v . y
 template <typename T>
 static void minres_product(mpet_ctx* c, const EpiMinres<T>& e) {
     if constexpr (sizeof(T) == 4) {
         if (c->sys_patch) {
-            launch_patch_sys<true>(c, e.v, PatchOut{e.y, e.r1, e.sc});
+            launch_patch_sys<true>(c, e.v, PatchOut{e.y, e.r1, c->sc});
             return;
         }
     }
     launch_spmv<T, 1>(c, c->A, vals<T>(c->A), e.v, e);
+    k_mr_alfa<<<1, 256, 0, c->stream>>>(c->sc, c->partials);
+    MPET_CHECK_LAUNCH();
+    c->n_launch++;
 }

@@ -1402,6 +1402,12 @@ static void launch_p2lap_mf(mpet_ctx* c, const T* x, const Epi& epi) {
     c->n_launch++;
 }
 
+// (defined with the MINRES kernels)
+__device__ void mr_alfa_one(MinresScalars* s, double t);
+__global__ void k_mr_alfa(MinresScalars* s, const double* partials);
+__device__ __forceinline__ bool last_block(unsigned* cnt);
+__device__ __forceinline__ double sum_partials_n(const double* p, int n, double* sh);
+
 #include "patch.cuh"
 
 void krylov_product_f32(mpet_ctx* c, const float* x, float* y) { krylov_product<float>(c, x, y); }
@@ -1634,26 +1640,6 @@ __global__ void k_mr_v(int64_t n, const T* __restrict__ y, T* v, const MinresSca
     v[i] = y[i] * msc<T>(sc->inv_beta, sc->f_inv_beta);
 }
 
-template <typename T>
-__global__ void k_mr_axpy(int64_t n, T* y, const T* __restrict__ r2, const MinresScalars* sc) {
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    y[i] -= msc<T>(sc->c_r2, sc->f_c_r2) * r2[i];
-}
-
-// w = (v - oldeps w1 - delta w2) / gamma ; d += phi w  (w1, w2 already rotated)
-template <typename T>
-__global__ void k_mr_update(int64_t n, const T* __restrict__ v, const T* __restrict__ w1, const T* __restrict__ w2,
-                            T* w, T* d, const MinresScalars* sc) {
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const T oe = msc<T>(sc->oldeps, sc->f_oldeps), de = msc<T>(sc->delta, sc->f_delta);
-    const T ig = msc<T>(sc->inv_gamma, sc->f_inv_gamma), ph = msc<T>(sc->phi, sc->f_phi);
-    const T wn = (v[i] - oe * w1[i] - de * w2[i]) * ig;
-    w[i] = wn;
-    d[i] += ph * wn;
-}
-
 // the FP32 copies of the scalars (after every update of the FP64 ones)
 __device__ __forceinline__ void mr_mirror(MinresScalars* s) {
     s->f_inv_beta = (float)s->inv_beta;
@@ -1739,13 +1725,102 @@ __global__ void k_mr_alfa(MinresScalars* s, const double* partials) {
     double t = sum_partials(partials, sh);
     if (threadIdx.x == 0) mr_alfa_one(s, t);
 }
-__global__ void k_mr_beta(MinresScalars* s, const double* partials) {
-    __shared__ double sh[8];
-    double t = sum_partials(partials, sh);
-    if (threadIdx.x == 0) mr_beta_one(s, t);
+// True in the block of this launch that arrives last (every block calls it once, after thread 0
+// has written the block's partial); that block may read the others' partials.  The counter wraps
+// to zero for the next launch.
+__device__ __forceinline__ bool last_block(unsigned* cnt) {
+    __shared__ bool last;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicInc(cnt, gridDim.x - 1) == gridDim.x - 1;
+        __threadfence();
+    }
+    __syncthreads();
+    return last;
 }
 
+// Sum of n partials by one 256-thread block (fixed order); for the last block of a launch.
+__device__ __forceinline__ double sum_partials_n(const double* p, int n, double* sh) {
+    double v = 0.0;
+    for (int i = threadIdx.x; i < n; i += 256) v += __ldcg(p + i);
+    return block_sum256(v, sh);
+}
 
+// The vector work of a MINRES iteration in three kernels.  One thread handles a P2 node's
+// displacement rows or a pressure row; items 0..nodes-1 are the nodes (nodes = 0: every row by
+// itself, without packing).
+//
+// k_mr_lanczos: y -= c_r2 r2, and the displacement rows of y in the padded layout that the
+// preconditioner's first level takes.  k_mr_dot: the preconditioned vector z from that layout,
+// the partial sums of r . z, and in the block that arrives last the scalar step of the iteration.
+// k_mr_direction: w = (v - oldeps w1 - delta w2) / gamma, d += phi w, v = z / beta (the next
+// Lanczos vector).  Against one kernel per operation (nine a iteration with two single-block ones)
+// the vectors are read once less and four launches and their drains are saved: 58 -> 50 us per
+// iteration on the 4^3 cube (A=2, FP32), 256 -> 230 at 24^3 (total pressure).
+template <typename T>
+__global__ void __launch_bounds__(256) k_mr_lanczos(int64_t nodes, int dim, int64_t n, T* y,
+                                                    const T* __restrict__ r2, T* packed,
+                                                    const int32_t* __restrict__ perm, const MinresScalars* sc) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const T c = msc<T>(sc->c_r2, sc->f_c_r2);
+    if (i < nodes) {
+        T v[4] = {T(0), T(0), T(0), T(0)};
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            if (k < dim) v[k] = y[dim * i + k] - c * r2[dim * i + k];
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            if (k < dim) y[dim * i + k] = v[k];
+        VecIO<T, 4>::store(packed, perm ? perm[i] : i, v);
+    } else {
+        const int64_t row = dim * nodes + (i - nodes);
+        if (row < n) y[row] -= c * r2[row];
+    }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) k_mr_dot(int64_t nodes, int dim, int64_t n, const T* __restrict__ r, T* z,
+                                                const T* __restrict__ packed, const int32_t* __restrict__ perm,
+                                                double* partials, unsigned* cnt, MinresScalars* sc) {
+    __shared__ double sh[8];
+    // a thread's products are summed in the working precision (a few dozen terms), then in FP64
+    T acc = T(0);
+    const int64_t items = nodes + (n - dim * nodes);
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < items; i += (int64_t)gridDim.x * blockDim.x) {
+        if (i < nodes) {
+            T v[4];
+            VecIO<T, 4>::load(packed, perm ? perm[i] : i, v);
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+                if (k < dim) {
+                    z[dim * i + k] = v[k];
+                    acc += r[dim * i + k] * v[k];
+                }
+        } else {
+            const int64_t row = dim * nodes + (i - nodes);
+            acc += r[row] * z[row];
+        }
+    }
+    const double s = block_sum256((double)acc, sh);
+    if (threadIdx.x == 0) partials[blockIdx.x] = s;
+    if (!last_block(cnt)) return;
+    const double t = sum_partials_n(partials, gridDim.x, sh);
+    if (threadIdx.x == 0) mr_beta_one(sc, t);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) k_mr_direction(int64_t n, const T* __restrict__ z, T* v,
+                                                      const T* __restrict__ w1, const T* __restrict__ w2, T* w, T* d,
+                                                      const MinresScalars* sc) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const T oe = msc<T>(sc->oldeps, sc->f_oldeps), de = msc<T>(sc->delta, sc->f_delta);
+    const T ig = msc<T>(sc->inv_gamma, sc->f_inv_gamma), ph = msc<T>(sc->phi, sc->f_phi);
+    const T wn = (v[i] - oe * w1[i] - de * w2[i]) * ig;
+    w[i] = wn;
+    d[i] += ph * wn;
+    v[i] = z[i] * msc<T>(sc->inv_beta, sc->f_inv_beta);
+}
 
 __global__ void k_outer_norms(MinresScalars* s, const double* partials) {
     __shared__ double sh[8];
@@ -1941,13 +2016,21 @@ __global__ void k_modes(int64_t nv, int J, const int32_t* __restrict__ vinst, co
     }
 }
 
+// row of each P2 node in the vectors of the first displacement level (null: the node itself)
+static const int32_t* first_level_perm(const mpet_ctx* c) {
+    const AmgHier& h = c->amg_u;
+    return h.lev[0].tiled() ? h.lev[0].A.rt.perm : h.perm;
+}
+
 // Block-diagonal preconditioner z = M^-1 r.  The J pressure V-cycles (on the
 // networks, or on the network eigenmodes between two vertex-wise
 // transforms) are forked onto side streams and run concurrently with the
 // displacement V-cycle on the main stream (inside a CUDA graph capture they
 // become parallel branches); the main stream joins them at the end.
+// packed: the displacement rows of r are already in the first level's input, and those of z are
+// left in its output (k_mr_lanczos, k_mr_dot).
 template <typename T>
-static void precond(mpet_ctx* c, const T* r, T* z) {
+static void precond(mpet_ctx* c, const T* r, T* z, bool packed = false) {
     cudaStream_t main = c->stream;
     const T* rp = r + c->Nu;
     T* zp = z + c->Nu;
@@ -1976,12 +2059,17 @@ static void precond(mpet_ctx* c, const T* r, T* z) {
         const int64_t nodes = c->nnodes;
         T* bin = (T*)hu.pack_in;
         T* xout = (T*)hu.pack_out;
-        const int32_t* perm = hu.lev[0].tiled() ? hu.lev[0].A.rt.perm : hu.perm;
-        k_pack34<T><<<grid_for(nodes, 256), 256, 0, main>>>(nodes, c->dim, r, bin, perm);
+        const int32_t* perm = first_level_perm(c);
+        if (!packed) {
+            k_pack34<T><<<grid_for(nodes, 256), 256, 0, main>>>(nodes, c->dim, r, bin, perm);
+            c->n_launch++;
+        }
         vcycle<T, 4>(c, hu, 0, bin, xout);
-        k_unpack43<T><<<grid_for(nodes, 256), 256, 0, main>>>(nodes, c->dim, xout, z, perm);
+        if (!packed) {
+            k_unpack43<T><<<grid_for(nodes, 256), 256, 0, main>>>(nodes, c->dim, xout, z, perm);
+            c->n_launch++;
+        }
         MPET_CHECK_LAUNCH();
-        c->n_launch += 2;
     }
     for (int a = 0; a < c->J; ++a) MPET_CUDA(cudaStreamWaitEvent(main, c->ev_join[a], 0));
     if (c->net_modes) {
@@ -1994,14 +2082,23 @@ static void precond(mpet_ctx* c, const T* r, T* z) {
 
 // ---- MINRES ----------------------------------------------------------------------------
 
-// Three MINRES iterations.  The Lanczos vectors rotate through kr[0..2]
+// Three MINRES iterations, from the Lanczos vector v = kr[2] / beta.  The Lanczos vectors rotate through kr[0..2]
 // (r1, r2, y) and the direction vectors through kw[0..2] (w, w1, w2); both
 // rotations have period 3, so three iterations start and end in the same
 // buffer assignment and can be captured once and replayed as a CUDA graph.
 template <typename T>
 static void minres_three(mpet_ctx* c) {
     const int64_t n = c->N;
-    const int G = grid_for(n, 256);
+    // (elasticity form: the hierarchy works on the rows as they are)
+    const bool pack = !c->u_elast;
+    const AmgHier& hu = c->amg_u;
+    const int64_t nodes = pack ? c->nnodes : 0, items = nodes + (n - c->dim * nodes);
+    const int32_t* perm = pack ? first_level_perm(c) : nullptr;
+    const int G = grid_for(items, 256);
+    // two blocks per SM (each block's FP64 sum takes half a microsecond of its SM's FP64 pipe), more
+    // where that leaves a thread more than 16 rows
+    const int Gd = (int)std::min<int64_t>(NB_RED, std::max<int64_t>(std::min<int64_t>(grid_for(items, 256), 304),
+                                                                    grid_for(items, 4096)));
     T* v = (T*)c->kv;
     T* d = (T*)c->kd;
     int ir1 = 0, ir2 = 1, iy = 2;
@@ -2010,26 +2107,23 @@ static void minres_three(mpet_ctx* c) {
         T* r1 = (T*)c->kr[ir1];
         T* r2 = (T*)c->kr[ir2];
         T* y = (T*)c->kr[iy];
-        k_mr_v<T><<<G, 256, 0, c->stream>>>(n, y, v, c->sc);
         minres_product<T>(c, EpiMinres<T>{y, r1, v, c->sc});
         c->n_spmv++;
-        k_mr_alfa<<<1, 256, 0, c->stream>>>(c->sc, c->partials);
-        k_mr_axpy<T><<<G, 256, 0, c->stream>>>(n, y, r2, c->sc);
+        k_mr_lanczos<T><<<G, 256, 0, c->stream>>>(nodes, c->dim, n, y, r2, (T*)hu.pack_in, perm, c->sc);
         MPET_CHECK_LAUNCH();
-        c->n_launch += 3;
         const int old1 = ir1;
         ir1 = ir2;
         ir2 = iy;
         iy = old1;
-        precond<T>(c, (const T*)c->kr[ir2], (T*)c->kr[iy]);
-        k_dot<T><<<NB_RED, 256, 0, c->stream>>>(n, (const T*)c->kr[ir2], (const T*)c->kr[iy], c->partials);
-        k_mr_beta<<<1, 256, 0, c->stream>>>(c->sc, c->partials);
+        precond<T>(c, (const T*)c->kr[ir2], (T*)c->kr[iy], pack);
+        k_mr_dot<T><<<Gd, 256, 0, c->stream>>>(nodes, c->dim, n, (const T*)c->kr[ir2], (T*)c->kr[iy],
+                                               (const T*)hu.pack_out, perm, c->partials, c->red_cnt, c->sc);
         const int oldw1 = iw1;
         iw1 = iw2;
         iw2 = iw;
         iw = oldw1;
-        k_mr_update<T><<<G, 256, 0, c->stream>>>(n, v, (const T*)c->kw[iw1], (const T*)c->kw[iw2],
-                                                 (T*)c->kw[iw], d, c->sc);
+        k_mr_direction<T><<<grid_for(n, 256), 256, 0, c->stream>>>(n, (const T*)c->kr[iy], v, (const T*)c->kw[iw1],
+                                                                  (const T*)c->kw[iw2], (T*)c->kw[iw], d, c->sc);
         MPET_CHECK_LAUNCH();
         c->n_launch += 3;
     }
@@ -2385,6 +2479,8 @@ static int solve_impl(mpet_ctx* c, const double* b, double* x, mpet_stats* st, b
         }
         MPET_CUDA(cudaMemsetAsync(c->kd, 0, sizeof(T) * n, c->stream));
         for (int q = 0; q < 3; ++q) MPET_CUDA(cudaMemsetAsync(c->kw[q], 0, sizeof(T) * n, c->stream));
+        k_mr_v<T><<<G, 256, 0, c->stream>>>(n, (const T*)c->kr[2], (T*)c->kv, c->sc);
+        MPET_CHECK_LAUNCH();
         int done = 0;
         MPET_CUDA(cudaEventRecord(c->ev_in0, c->stream));
         int s2 = minres_run<T>(c, target, maxit - iters, &done);
@@ -3583,6 +3679,8 @@ void alloc_krylov(mpet_ctx* c) {
     }
     c->orr = c->pool.alloc<double>(n);
     c->partials = c->pool.alloc<double>(2 * NB_RED);
+    c->red_cnt = c->pool.alloc<unsigned>(1);
+    MPET_CUDA(cudaMemsetAsync(c->red_cnt, 0, sizeof(unsigned), c->stream));
     c->dev_err = c->pool.alloc<int>(1);
     MPET_CUDA(cudaMemsetAsync(c->dev_err, 0, sizeof(int), c->stream));
     if (!c->ev_fork) MPET_CUDA(cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
