@@ -480,6 +480,7 @@ struct mpet_ctx {
 
     // MINRES iterations replayed from a CUDA graph (3 iterations per launch)
     cudaStream_t cap_stream = nullptr;
+    bool pdl = false, pdl_chain = false;  // programmatic dependent launches (launch_k)
     cudaGraphExec_t mr_graph = nullptr;  // whole inner solve: WHILE node over 3 iterations
     void* loop_ctl = nullptr;            // device loop control (target, budget, iterations)
     void* loop_ctl_host = nullptr;       // pinned copy

@@ -144,6 +144,7 @@ __global__ void __launch_bounds__(256, J <= 4 ? 3 : 2) k_patch_sys(PatchArgs A, 
     unsigned* snd = reinterpret_cast<unsigned*>(scp + 4 * J * P);
     unsigned* sgp = snd + M;  // first and past-the-last contribution
     float4* part = reinterpret_cast<float4*>(A.part);
+    pdl_wait();
     const float cr = DOT ? O.sc->f_c_r1 : 0.f;
     DotAcc dot;
     for (int64_t p = blockIdx.x; p < A.np; p += gridDim.x) {
@@ -327,6 +328,7 @@ __global__ void __launch_bounds__(256, J <= 4 ? 3 : 2) k_patch_sys(PatchArgs A, 
         }
         __syncthreads();  // the next patch reuses the shared arrays
     }
+    pdl_trigger();
     patch_dot_finish<DOT>(dot, partials, 0, nullptr, nullptr);
 }
 
@@ -340,6 +342,7 @@ __global__ void __launch_bounds__(256) k_patch_sys_shared(int64_t nsh, const int
                                                           int first, unsigned* cnt,
                                                           const int32_t* __restrict__ node_inst,
                                                           const double* __restrict__ skip) {
+    pdl_wait();
     const float cr = DOT ? O.sc->f_c_r1 : 0.f;
     DotAcc dot;
     const int64_t items = nsh + (int64_t)J * D.nshv;
@@ -387,6 +390,7 @@ __global__ void __launch_bounds__(256) k_patch_sys_shared(int64_t nsh, const int
             patch_row<DOT>(O, row, bc && D.dof_bc[row] ? xv : a, r1, xv, cr, dot);
         }
     }
+    pdl_trigger();
     patch_dot_finish<DOT>(dot, partials, first, cnt, O.sc);
 }
 
@@ -401,8 +405,8 @@ static void launch_patch_sys_j(mpet_ctx* c, const float* x, const PatchOut& O) {
     const int g1 = (int)std::min<int64_t>(s.np, 456);
     const int g2 = (int)std::min<int64_t>(std::max<int64_t>((items + 255) / 256, 1), NB_RED - 456);
     MPET_CUDA(cudaFuncSetAttribute(k_patch_sys<J, DOT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    k_patch_sys<J, DOT><<<g1, s.P, sm, c->stream>>>(patch_args(c), D, c->patch_coef, x, O, c->partials, skip);
-    k_patch_sys_shared<J, DOT><<<g2, 256, 0, c->stream>>>(s.nsh, s.sh_node, s.sh_ptr, (const float4*)s.part, D,
+    launch_k(c, k_patch_sys<J, DOT>, g1, s.P, sm, patch_args(c), D, c->patch_coef, x, O, c->partials, skip);
+    launch_k(c, k_patch_sys_shared<J, DOT>, g2, 256, 0, s.nsh, s.sh_node, s.sh_ptr, (const float4*)s.part, D,
                                                           c->patch_coef.bc, x, O, c->partials, g1, c->red_cnt,
                                                           c->node_inst, skip);
     MPET_CHECK_LAUNCH();
@@ -447,7 +451,7 @@ static void minres_product(mpet_ctx* c, const EpiMinres<T>& e) {
         }
     }
     launch_spmv<T, 1>(c, c->A, vals<T>(c->A), e.v, e);
-    k_mr_alfa<<<1, 256, 0, c->stream>>>(c->sc, c->partials);
+    launch_k(c, k_mr_alfa, 1, 256, 0, c->sc, c->partials);
     MPET_CHECK_LAUNCH();
     c->n_launch++;
 }

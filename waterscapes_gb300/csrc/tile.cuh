@@ -92,7 +92,6 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 4 : 5) k_spmv_tile(TileA
     typedef typename Pair<T>::type P2;
     T* sx = reinterpret_cast<T*>(smem);
     const int64_t t = blockIdx.x;
-    if (skip && slice_frozen(A.skl, t, skip)) return;  // (the whole block)
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, sub = lane % LPR;
     int cid[CQ];
 #pragma unroll
@@ -113,15 +112,6 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 4 : 5) k_spmv_tile(TileA
             steps = q == w ? s : steps;
         }
     }
-#pragma unroll
-    for (int q = 0; q < CQ; ++q) {
-        const int i = tid + q * 256;
-        if (i < A.mc) TileX<T, NV>::copy(sx + NV * i, x + NV * (int64_t)cid[q]);
-    }
-    cp_async_commit();
-    const bool own = row >= 0 && sub == 0;
-    typename Epi::Pre pre{};
-    if (own) pre = epi.pre(row);
     const P2* pv = reinterpret_cast<const P2*>(va + e0) + base * 32 + lane;
     const uint32_t* pc = reinterpret_cast<const uint32_t*>(A.lc + e0) + base * 32 + lane;
     P2 a[PF];
@@ -132,6 +122,18 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 4 : 5) k_spmv_tile(TileA
             a[u] = __ldcs(pv + u * 32);
             cc[u] = __ldcs(pc + u * 32);
         }
+    // (so far nothing that an earlier kernel writes)
+    pdl_wait();
+    if (skip && slice_frozen(A.skl, t, skip)) return;  // (the whole block)
+#pragma unroll
+    for (int q = 0; q < CQ; ++q) {
+        const int i = tid + q * 256;
+        if (i < A.mc) TileX<T, NV>::copy(sx + NV * i, x + NV * (int64_t)cid[q]);
+    }
+    cp_async_commit();
+    const bool own = row >= 0 && sub == 0;
+    typename Epi::Pre pre{};
+    if (own) pre = epi.pre(row);
     cp_async_wait<0>();
     __syncthreads();
     T acc[NV];
@@ -167,6 +169,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 4 : 5) k_spmv_tile(TileA
     for (int o = LPR / 2; o > 0; o >>= 1)
 #pragma unroll
         for (int k = 0; k < NC; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
+    pdl_trigger();
     double r0 = 0.0, r1 = 0.0;
     if (own) epi.apply(row, acc, pre, r0, r1);
 }
@@ -177,7 +180,7 @@ static void launch_tile_l(mpet_ctx* c, const RowTiles& r, int64_t n, const T* x,
     auto kern = k_spmv_tile<T, NV, LPR, Epi>;
     if (sm > 48 * 1024) MPET_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     const TileArgs A{n, r.perm ? nullptr : r.row, r.col, r.eoff, r.steps, r.lc, r.skl, r.mc};
-    kern<<<(unsigned)r.nt, 256, sm, c->stream>>>(A, (const T*)r.v, x, epi, r.skl ? c->skip_done : nullptr);
+    launch_k(c, kern, r.nt, 256, sm, A, (const T*)r.v, x, epi, r.skl ? c->skip_done : (const double*)nullptr);
     MPET_CHECK_LAUNCH();
     c->n_launch++;
 }
