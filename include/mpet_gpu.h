@@ -398,8 +398,8 @@ int mpet_set_row_tiles(mpet_ctx* ctx, int32_t mode);
 /* How the inner FP32 iterations of a mixed-precision solve form A x: cell by
  * cell from the geometry and the coefficients of the last mpet_assemble (1),
  * from the stored FP32 copy (0), or by the size of the matrix (-1, default).
- * The stored copy serves wherever the element product cannot: triangles, a
- * Robin term in the matrix, or a variant forced by mpet_set_spmv_variant.
+ * The stored copy serves wherever the element product cannot: triangles, or a
+ * variant forced by mpet_set_spmv_variant.
  * Takes effect at the next mpet_assemble, which must follow.  No reference
  * counterpart (engine option and test hook). */
 int mpet_set_element_product(mpet_ctx* ctx, int32_t mode);

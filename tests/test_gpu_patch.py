@@ -101,12 +101,17 @@ def test_coefficients_follow_the_last_assembly_and_forced_variants_stay_stored()
     _check(s, dt, elements=0)
 
 
-def test_robin_matrix_keeps_the_stored_product():
+@pytest.mark.parametrize("n,J", [(3, 1), (12, 2)])
+def test_robin_matrix_in_the_element_product(n, J):
+    """Robin terms on one side for one network, on two sides for another; Dirichlet rows elsewhere."""
     from waterscapes_gb300 import CompiledSubDomain, Expression, MPETSolver
-    problem, dt = make_problem(3, 1)
-    CompiledSubDomain(lambda x: np.abs(x[:, 1] - 1.0) < 1e-12).mark(problem.continuity_boundary_markers[0], 2)
-    problem.beta = [Expression(lambda x, t: 1.5 + x[:, 2])]
+    problem, dt = make_problem(n, J)
+    side = lambda k, v: CompiledSubDomain(lambda x: np.abs(x[:, k] - v) < 1e-12)  # noqa: E731
+    side(1, 1.0).mark(problem.continuity_boundary_markers[0], 2)
+    side(0, 0.0).mark(problem.continuity_boundary_markers[J - 1], 2)
+    side(2, 1.0).mark(problem.continuity_boundary_markers[J - 1], 1)
+    problem.beta = [Expression(lambda x, t: 150.0 + x[:, 2]) for _ in range(J)]
     s = MPETSolver(problem, dict(dt=dt, T=1.0, precision="mixed"))
     s.ctx.call("mpet_set_element_product", 1)
     s.step(dt)
-    _check(s, dt, elements=0)
+    _check(s, dt)

@@ -224,7 +224,8 @@ int mpet_setup(mpet_ctx* c, const mpet_params* p) {
         MPET_CUDA(cudaMemsetAsync(c->A.v32, 0, sizeof(float) * c->nnz, c->stream));
     }
     if (!mixed || c->A.v32) build_sell(c, c->A, c->A.v32 != nullptr, true);
-    refresh_system_copies(c);
+    c->stale = COPY_ALL;
+    need_copies(c, COPY_ALL);
     autotune_system(c);
     MPET_CUDA(cudaStreamSynchronize(c->stream));
     c->setup_done = true;
@@ -281,11 +282,13 @@ int mpet_assemble(mpet_ctx* c, double dt, int32_t apply_bc) {
     API_BEGIN(c)
     require(c->setup_done, MPET_ERR_STATE, "mpet_setup must come first");
     require(dt > 0.0, MPET_ERR_INVALID, "dt must be positive");
-    launch_assemble_matrix(c, dt, apply_bc != 0, c->A.v32 != nullptr);
+    launch_assemble_matrix(c, dt, apply_bc != 0);
     launch_robin_matrix(c, dt);
-    refresh_system_copies(c);
-    build_patches(c);
+    c->stale = COPY_ALL;
+    // (the patches come with the preconditioner: a program that only assembles does without)
+    if (c->sys_patch_mode == 1) build_patches(c);
     set_patch_coefficients(c, dt, apply_bc != 0);
+    c->asm_bc = apply_bc != 0;
     MPET_CUDA(cudaStreamSynchronize(c->stream));
     c->assembled = true;
     c->bc_cols_zeroed = false;
@@ -551,6 +554,10 @@ int mpet_setup_preconditioner(mpet_ctx* c, double dt) {
     require(c->setup_done, MPET_ERR_STATE, "mpet_setup must come first");
     require(dt > 0.0, MPET_ERR_INVALID, "dt must be positive");
     destroy_minres_graph(c);
+    if (!c->patch.tried && c->sys_patch_mode != 0) {
+        build_patches(c);
+        if (c->assembled) set_patch_coefficients(c, c->asm_dt, c->asm_bc);
+    }
     using clk = std::chrono::steady_clock;
     auto since = [](clk::time_point t) { return std::chrono::duration<double, std::milli>(clk::now() - t).count(); };
     auto t0 = clk::now();
@@ -898,8 +905,7 @@ int mpet_apply_symmetric(mpet_ctx* c, double* b, const double* xbc) {
     require(c->assembled, MPET_ERR_STATE, "mpet_assemble must come first");
     launch_zero_bc_columns(c, b, xbc);
     c->bc_cols_zeroed = true;
-    convert_values_to_f32(c);
-    refresh_system_copies(c);
+    c->stale = COPY_ALL;
     MPET_CUDA(cudaStreamSynchronize(c->stream));
     API_END(c)
 }

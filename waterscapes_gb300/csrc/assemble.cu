@@ -158,10 +158,11 @@ struct AsmArgs {
     const double* geo;
     const uint8_t* dof_bc;
     double* v64;
-    float* v32;
     double* dinv;
     int apply_bc;
     const double* Mst;  // per-cell displacement blocks (k_elem_uu) or null
+    int64_t first, last;  // P2 nodes of this launch
+    int wbuf;             // doubles of shared memory per warp
 };
 
 // Number of node pairs m <= j of a cell and the index of pair (m, j), m <= j.
@@ -238,15 +239,22 @@ __global__ void __launch_bounds__(128) k_elem_uu(int64_t nc, const double* __res
 // displacement-pressure couplings (k, vertex w), and for a vertex node
 // NN*D pressure-displacement couplings (j, l) and NV pressure-pressure
 // entries (w): 30/42/72/76 on tetrahedra, 12/18/30/33 on triangles.
+//
+// A node's rows are added up in the warp's part of shared memory and written once: a
+// read-modify-write of global memory costs an L2 round trip in each of a cell's rounds
+// (33^3 A=4: 6.06 ms that way, 4.44 here).  Rows that do not fit there (wbuf doubles) are added up in place.
+// Vertices and edge nodes go in two launches, each with the room that its rows need.
 template <int D>
 __global__ void __launch_bounds__(256) k_assemble_matrix(AsmArgs A, MatCoef P) {
     constexpr int NV = Simplex<D>::NV, NN = Simplex<D>::NN;
     constexpr int X0 = (NN * D + 31) / 32 * 32;  // first coupling task
+    extern __shared__ double asm_rows[];
+    double* const buf = asm_rows + (size_t)(threadIdx.x >> 5) * A.wbuf;
     const int lane = threadIdx.x & 31;
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const int J = P.J;
-    for (int64_t i = warp; i < A.nnodes; i += nwarps) {
+    for (int64_t i = A.first + warp; i < A.last; i += nwarps) {
         const bool isv = i < A.nv;
         const int64_t s2 = A.n2_ptr[i], s1 = A.n1_ptr[i];
         const int d2 = (int)(A.n2_ptr[i + 1] - s2), d1 = (int)(A.n1_ptr[i + 1] - s1);
@@ -257,8 +265,15 @@ __global__ void __launch_bounds__(256) k_assemble_matrix(AsmArgs A, MatCoef P) {
         for (int a = 0; a < J; ++a) rows[D + a] = A.Nu + (int64_t)a * A.nv + i;
         int64_t rp[3 + MPET_MAX_NETWORKS];
         for (int q = 0; q < nrows; ++q) rp[q] = A.row_ptr[rows[q]];
-        for (int q = 0; q < nrows; ++q)
-            for (int e = lane; e < L; e += 32) A.v64[rp[q] + e] = 0.0;
+        const bool local = nrows * L <= A.wbuf;
+        // entry `off` of the node's row q
+        auto at = [&](int q, int64_t off) -> double& { return local ? buf[q * L + off] : A.v64[rp[q] + off]; };
+        if (local) {
+            for (int e = lane; e < nrows * L; e += 32) buf[e] = 0.0;
+        } else {
+            for (int q = 0; q < nrows; ++q)
+                for (int e = lane; e < L; e += 32) A.v64[rp[q] + e] = 0.0;
+        }
         __syncwarp();
         for (int64_t it = A.inc_ptr[i]; it < A.inc_ptr[i + 1]; ++it) {
             const int32_t packed = A.inc[it];
@@ -279,7 +294,7 @@ __global__ void __launch_bounds__(256) k_assemble_matrix(AsmArgs A, MatCoef P) {
                 if (t < X0) {
                     if (t >= NN * D) continue;
                     const int j = t / D, k = t % D;
-                    const int64_t base = rp[k] + D * (int64_t)rk2[j];
+                    const int64_t base = D * (int64_t)rk2[j];
                     if (A.Mst) {
                         // row k of B_mj (stored, or the transpose of the stored B_jm)
                         constexpr int DD = D * D;
@@ -287,7 +302,7 @@ __global__ void __launch_bounds__(256) k_assemble_matrix(AsmArgs A, MatCoef P) {
                         const bool up = m <= j;
                         src += pair_index<D>(up ? m : j, up ? j : m) * DD;
 #pragma unroll
-                        for (int l = 0; l < D; ++l) A.v64[base + l] += src[up ? k * D + l : l * D + k];
+                        for (int l = 0; l < D; ++l) at(k, base + l) += src[up ? k * D + l : l * D + k];
                         continue;
                     }
                     double M[3][3];
@@ -312,7 +327,7 @@ __global__ void __launch_bounds__(256) k_assemble_matrix(AsmArgs A, MatCoef P) {
                     for (int l = 0; l < D; ++l) {
                         double v = P.mu * M[l][k] + P.lmbda * M[k][l];
                         if (l == k) v += P.mu * tr;
-                        A.v64[base + l] += v;
+                        at(k, base + l) += v;
                     }
                 } else if (t < X0 + nx) {
                     // coupling value w20 (grad phi_node at vertex + s_node)[comp]: u row k with
@@ -332,27 +347,27 @@ __global__ void __launch_bounds__(256) k_assemble_matrix(AsmArgs A, MatCoef P) {
                         C = w20 * (g[comp] + sg[comp]);
                     }
                     for (int a = 0; a < J; ++a) {
-                        const int64_t pos = urow ? rp[comp] + D * (int64_t)d2 + (int64_t)a * d1 + rk1[gvert]
-                                                 : rp[D + a] + D * (int64_t)rk2[gnode] + comp;
-                        A.v64[pos] += P.cpl[a] * C;
+                        const int64_t pos = urow ? D * (int64_t)d2 + (int64_t)a * d1 + rk1[gvert]
+                                                 : D * (int64_t)rk2[gnode] + comp;
+                        at(urow ? comp : D + a, pos) += P.cpl[a] * C;
                     }
                 } else {
                     const int q = t - X0 - nx, a = q / NV, w = q % NV;
                     const double M1 = w20 * (m == w ? 2.0 : 1.0);
                     const double L1 = G.vol * (G.b[m][0] * G.b[w][0] + G.b[m][1] * G.b[w][1] + G.b[m][2] * G.b[w][2]);
-                    const int64_t base = rp[D + a] + D * (int64_t)d2 + rk1[w];
+                    const int64_t base = D * (int64_t)d2 + rk1[w];
                     if (P.coef_const) {
                         for (int b = 0; b < J; ++b) {
                             double v = P.Cm[a * MPET_MAX_NETWORKS + b] * M1;
                             if (a == b) v += P.Kd[a] * L1;
-                            A.v64[base + (int64_t)b * d1] += v;
+                            at(D + a, base + (int64_t)b * d1) += v;
                         }
                     } else {
                         for (int b = 0; b < J; ++b) {
                             double v = -(P.dt_theta * ((a == b ? P.Ssumof(a, cell) : 0.0) - P.Sof(a, b, cell)) +
                                          P.rank_inv * P.rank_b[a] * P.rank_b[b]) * M1;
                             if (a == b) v += -P.cof(a, cell) * M1 - P.dt_theta * P.Kof(a, cell) * L1;
-                            A.v64[base + (int64_t)b * d1] += v;
+                            at(D + a, base + (int64_t)b * d1) += v;
                         }
                     }
                 }
@@ -363,22 +378,18 @@ __global__ void __launch_bounds__(256) k_assemble_matrix(AsmArgs A, MatCoef P) {
         int self2 = lb_i32(A.n2_col + s2, d2, (int32_t)i);
         int self1 = isv ? lb_i32(A.n1_col + s1, d1, (int32_t)i) : 0;
         for (int q = 0; q < nrows; ++q) {
-            const int64_t dpos = q < D ? rp[q] + D * self2 + q : rp[q] + D * (int64_t)d2 + (int64_t)(q - D) * d1 + self1;
-            if (A.apply_bc && A.dof_bc[rows[q]]) {
-                for (int e = lane; e < L; e += 32) A.v64[rp[q] + e] = 0.0;
-                __syncwarp();
-                if (lane == 0) A.v64[dpos] = 1.0;
-                __syncwarp();
+            const int64_t dpos = q < D ? D * self2 + q : D * (int64_t)d2 + (int64_t)(q - D) * d1 + self1;
+            const bool fixed = A.apply_bc && A.dof_bc[rows[q]];
+            if (local) {
+                for (int e = lane; e < L; e += 32)
+                    __stcs(A.v64 + rp[q] + e, fixed ? (e == dpos ? 1.0 : 0.0) : buf[q * L + e]);
+            } else if (fixed) {
+                for (int e = lane; e < L; e += 32) A.v64[rp[q] + e] = e == dpos ? 1.0 : 0.0;
             }
             if (lane == 0) {
-                double dg = fabs(A.v64[dpos]);
+                double dg = fixed ? 1.0 : fabs(at(q, dpos));
                 A.dinv[rows[q]] = dg > 0.0 ? 1.0 / dg : 1.0;
             }
-        }
-        __syncwarp();
-        if (A.v32) {
-            for (int q = 0; q < nrows; ++q)
-                for (int e = lane; e < L; e += 32) A.v32[rp[q] + e] = (float)A.v64[rp[q] + e];
         }
         __syncwarp();
     }
@@ -692,7 +703,7 @@ static inline int grid_for(int64_t n, int threads) {
     return (int)(g < 1 ? 1 : g);
 }
 
-void launch_assemble_matrix(mpet_ctx* c, double dt, bool apply_bc, bool write32) {
+void launch_assemble_matrix(mpet_ctx* c, double dt, bool apply_bc) {
     AsmArgs A{};
     A.nnodes = c->nnodes;
     A.nv = c->nv;
@@ -709,13 +720,9 @@ void launch_assemble_matrix(mpet_ctx* c, double dt, bool apply_bc, bool write32)
     A.geo = c->geo;
     A.dof_bc = c->dof_bc;
     A.v64 = c->A.v64;
-    A.v32 = write32 ? c->A.v32 : nullptr;
     A.dinv = c->dinv;
     A.apply_bc = apply_bc ? 1 : 0;
     MatCoef P = make_coef(c, dt);
-    int64_t warps_needed = c->nnodes;
-    int blocks = grid_for(warps_needed * 32, 256);
-    if (blocks > 152 * 64) blocks = 152 * 64;
     // staged element data when it fits beside everything else (a fifth of HBM stays free)
     const size_t mst_bytes = (size_t)c->nc * (c->dim == 2 ? elem_record<2>() : elem_record<3>()) * sizeof(double);
     // (kept for later assemblies; decided once per context)
@@ -733,9 +740,22 @@ void launch_assemble_matrix(mpet_ctx* c, double dt, bool apply_bc, bool write32)
             k_elem_uu<3><<<grid_for(c->nc, 128), 128, 0, c->stream>>>(c->nc, c->geo, P.mu, P.lmbda, c->elem_buf);
         MPET_CHECK_LAUNCH();
     }
-    if (c->dim == 2) k_assemble_matrix<2><<<blocks, 256, 0, c->stream>>>(A, P);
-    else k_assemble_matrix<3><<<blocks, 256, 0, c->stream>>>(A, P);
-    MPET_CHECK_LAUNCH();
+    for (int part = 0; part < 2; ++part) {
+        A.first = part == 0 ? 0 : c->nv;
+        A.last = part == 0 ? c->nv : c->nnodes;
+        if (A.first >= A.last) continue;
+        // room for every row group of the part, 24 KB a warp at most; four warps a block where a
+        // warp's room is large
+        A.wbuf = std::min(c->asm_rows[part], 3072);
+        const int threads = A.wbuf > 512 ? 128 : 256;
+        const size_t sm = (size_t)A.wbuf * (threads / 32) * sizeof(double);
+        int blocks = grid_for((A.last - A.first) * 32, threads);
+        if (blocks > 152 * 64) blocks = 152 * 64;
+        auto kern = c->dim == 2 ? k_assemble_matrix<2> : k_assemble_matrix<3>;
+        MPET_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * 3072 * 8));
+        kern<<<blocks, threads, sm, c->stream>>>(A, P);
+        MPET_CHECK_LAUNCH();
+    }
 }
 
 void launch_assemble_prec_blocks(mpet_ctx* c, double dt) {
@@ -935,10 +955,8 @@ void set_patch_coefficients(mpet_ctx* c, double dt, bool apply_bc) {
     // From 3e6 entries on: the two kernels of an element product take about 13 us however
     // small the mesh, the stored product 4.5 us at 0.2e6 entries (4^3 cube, A=2), 7.4 at 1.6e6
     // (8^3; a whole iteration 72 us stored, 77 by elements), 14.7 at 5.3e6 (12^3; 121 and 112)
-    // and 769 against 195 at 1.03e9 (64^3, A=4).  Boundary-facet terms of the matrix are not
-    // element products.
-    bool use = s.ready() && !(c->nf > 0 && c->f_beta_matrix) &&
-               (c->sys_patch_mode == 1 || (c->sys_patch_mode < 0 && c->nnz >= 3000000));
+    // and 769 against 195 at 1.03e9 (64^3, A=4).
+    bool use = s.ready() && (c->sys_patch_mode == 1 || (c->sys_patch_mode < 0 && c->nnz >= 3000000));
     float* const coef0 = s.coef;
     if (use) {
         q.mu = (float)C.mu;
@@ -950,6 +968,7 @@ void set_patch_coefficients(mpet_ctx* c, double dt, bool apply_bc) {
                 q.Cm[a * MPET_MAX_NETWORKS + b] = (float)C.Cm[a * MPET_MAX_NETWORKS + b];
         }
         q.bc = apply_bc ? 1 : 0;
+        q.robin = launch_robin_entries(c, dt) ? 1 : 0;
         q.ncell = C.coef_const ? 0 : (C.cc || C.Sc ? J + J * J : J);
         const int64_t need = s.np * s.P * q.ncell;
         if (need > s.ncoef) {

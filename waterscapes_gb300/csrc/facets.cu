@@ -369,4 +369,44 @@ void launch_robin_matrix(mpet_ctx* c, double dt) {
     MPET_CHECK_LAUNCH();
 }
 
+// The Robin matrix once more, entry by entry (facet of a vertex, vertex of the facet), for the
+// element products of the system: -dt theta |F| sum_v beta_v T[v][m][w], zero for facets of other
+// kinds.
+__global__ void k_robin_entries(int64_t nq, int64_t nf, int J, const int32_t* __restrict__ bn_list,
+                                const int32_t* __restrict__ fnodes, const double* __restrict__ fgeo,
+                                const int32_t* __restrict__ markers, const double* __restrict__ beta, double dt_theta,
+                                int32_t* col, float* val) {
+    const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (q >= nq) return;
+    const int64_t f = bn_list[q] >> 3;
+    const int m = bn_list[q] & 7;
+    for (int w = 0; w < 3; ++w) {
+        col[3 * q + w] = fnodes[6 * f + w];
+        for (int a = 0; a < J; ++a) {
+            double t = 0.0;
+            if (m < 3 && markers[(int64_t)(1 + a) * nf + f] == 2) {
+                const double* bv = beta + ((int64_t)a * nf + f) * 3;
+                for (int v = 0; v < 3; ++v) t += bv[v] * ft1<3>(v, m, w);
+            }
+            val[a * 3 * nq + 3 * q + w] = (float)(-dt_theta * fgeo[4 * f] * t);
+        }
+    }
+}
+
+bool launch_robin_entries(mpet_ctx* c, double dt) {
+    if (c->dim != 3 || c->nf == 0 || !c->bn_ptr || !c->f_beta_matrix) return false;
+    if (!c->rob_col) {
+        MPET_CUDA(cudaMemcpyAsync(&c->rob_n, c->bn_ptr + c->nnodes, sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream));
+        MPET_CUDA(cudaStreamSynchronize(c->stream));
+        c->rob_col = c->pool.alloc<int32_t>(3 * c->rob_n);
+        c->rob_val = c->pool.alloc<float>(3 * c->rob_n * c->J);
+    }
+    if (c->rob_n == 0) return false;
+    k_robin_entries<<<grid_for(c->rob_n, 128), 128, 0, c->stream>>>(c->rob_n, c->nf, c->J, c->bn_list, c->fnodes, c->fgeo,
+                                                                    c->markers, c->f_beta_matrix, dt * c->prm.theta,
+                                                                    c->rob_col, c->rob_val);
+    MPET_CHECK_LAUNCH();
+    return true;
+}
+
 }  // namespace mpet

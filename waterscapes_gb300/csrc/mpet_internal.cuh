@@ -122,6 +122,7 @@ struct NodeBlocks {
     int64_t ncols = 0, nvals = 0;  // stored (with padding)
     int64_t nblocks = 0;           // blocks of the matrix (without padding)
     int32_t* skl = nullptr;        // batches: lowest and highest instance of each slice's lanes
+    bool have_cols = false;        // cols is filled
 };
 
 // Row tiles of a level operator (tile.cuh, variant 64)
@@ -172,6 +173,7 @@ struct Csr {
     int64_t nslices = 0;
     int64_t* s_off = nullptr;
     int32_t* s_ci = nullptr;
+    bool s_cols = false;       // s_ci is filled
     float* s_v32 = nullptr;
     double* s_v64 = nullptr;
     // half-precision SELL values (variant 32, FP32 products of a first AMG
@@ -225,6 +227,7 @@ struct PatchCoef {
     float cpl[MPET_MAX_NETWORKS], Cm[MPET_MAX_NETWORKS * MPET_MAX_NETWORKS], Kd[MPET_MAX_NETWORKS];
     int ncell;  // values per cell in PatchSet::coef: 0 none, J the Kd_a, J + J J the Kd_a and Cm_ab
     int bc;     // Dirichlet rows are unit rows
+    int robin;  // pressure rows with the entries of the Robin matrix (rob_col, rob_val)
 };
 
 struct AmgLevel {
@@ -357,6 +360,8 @@ struct mpet_ctx {
     int64_t N = 0, Nu = 0, nnz = 0;
     mpet::Csr A;                  // rp/ci/v64/v32
     mpet::NodeBlocks A_nb;        // node-block copy of A
+    unsigned stale = 0;           // copies of A that do not hold its values yet (COPY_*)
+    int asm_rows[2] = {0, 0};     // most entries of a vertex's / an edge node's rows
     double* dinv = nullptr;       // |diag|^-1 (1 where 0), FP64
 
     // Dirichlet data
@@ -427,6 +432,12 @@ struct mpet_ctx {
     mpet::PatchCoef patch_coef{};
     bool sys_patch = false;
     int sys_patch_mode = -1;
+    bool asm_bc = false;          // apply_bc of the last assembly
+    // Robin matrix of the last assembly, in FP32: entries 3 q + w of boundary-vertex incidence q
+    // (bn_ptr), columns (vertices) and J planes of values
+    int32_t* rob_col = nullptr;
+    float* rob_val = nullptr;
+    int64_t rob_n = 0;
     bool gmres = false;           // solves by restarted GMRES (non-symmetric system)
     // constant-pressure constraints (int p_k = 0, multiplier p_null_k): networks, the P1
     // load vector (int phi_v), W_k = A^-1 B_k^T (nq x N), the inverse of B W, multipliers
@@ -616,9 +627,11 @@ const int32_t* node_order(mpet_ctx* c);
 void build_facets(mpet_ctx* c);
 void launch_facet_rhs(mpet_ctx* c, double dt, const double* up_prev, double* b);
 void launch_robin_matrix(mpet_ctx* c, double dt);
+// its entries for the element products (c->rob_*); false without Robin data
+bool launch_robin_entries(mpet_ctx* c, double dt);
 
 // assemble.cu
-void launch_assemble_matrix(mpet_ctx* c, double dt, bool apply_bc, bool write32);
+void launch_assemble_matrix(mpet_ctx* c, double dt, bool apply_bc);
 void launch_assemble_prec_blocks(mpet_ctx* c, double dt);
 // per-cell data of the matrix-free first displacement level (c->mf_cell, c->mf_tab);
 // leaves c->mf_cell null when HBM is short
@@ -695,16 +708,21 @@ void build_tiles(mpet_ctx* c, Csr& A, const int64_t* rp_host);
 void build_sell(mpet_ctx* c, Csr& A, bool fp32, bool with64);
 // the FP16 SELL values of A (after build_sell; needs A.v64)
 void build_sell_half(mpet_ctx* c, Csr& A);
-void fill_sell(mpet_ctx* c, Csr& A);
+void fill_sell(mpet_ctx* c, Csr& A, bool f32, bool f64);
 void build_node_blocks(mpet_ctx* c);
 bool device_fits(mpet_ctx* c, size_t bytes);
-void refresh_system_copies(mpet_ctx* c);
+// the system matrix's copies are filled from A.v64 when a product needs them: after a change of
+// the values all are stale; need_system_copy<T> fills the one that the tuned products in T read,
+// need_copies any set of them
+enum { COPY_CSR32 = 1, COPY_SELL32 = 2, COPY_SELL64 = 4, COPY_NB32 = 8, COPY_NB64 = 16, COPY_ALL = 31 };
+void need_copies(mpet_ctx* c, unsigned which);
+template <typename T>
+void need_system_copy(mpet_ctx* c);
 // y = A x (FP32) as the inner Krylov iterations form it
 void krylov_product_f32(mpet_ctx* c, const float* x, float* y);
 bool spmv_variant_available(const Csr& A, int variant);
 constexpr int SPMV_TILE = 2048;  // entries per staged tile
 constexpr int TILE_MAX_COLS = 2048;  // distinct columns of a row tile
 void destroy_minres_graph(mpet_ctx* c);
-void convert_values_to_f32(mpet_ctx* c);
 
 }  // namespace mpet

@@ -128,7 +128,20 @@ struct PatchDims {
     const uint8_t* dof_bc;
     const float* geo;   // (p * 10 + q) * P + l: b_1, b_2, b_3, |T| / 20
     const float* coef;  // per-cell coefficients, (p * nc + q) * P + l, or null
+    const int64_t* bn_ptr;  // Robin matrix: entries 3 bn_ptr[v] .. 3 bn_ptr[v + 1] - 1 of vertex v
+    const int32_t* rob_col;
+    const float* rob_val;   // J planes of rob_n
+    int64_t rob_n;
 };
+
+// the Robin matrix's part of network a's row at vertex v
+__device__ __forceinline__ float patch_robin(const PatchDims& D, int a, int64_t v, const float* __restrict__ x) {
+    const int64_t e1 = 3 * __ldg(D.bn_ptr + v + 1);
+    float s = 0.f;
+    for (int64_t e = 3 * __ldg(D.bn_ptr + v); e < e1; ++e)
+        s += __ldg(D.rob_val + a * D.rob_n + e) * x[D.Nu + a * D.nv + __ldg(D.rob_col + e)];
+    return s;
+}
 
 template <int J, bool DOT>
 __global__ void __launch_bounds__(256, J <= 4 ? 3 : 2) k_patch_sys(PatchArgs A, PatchDims D, PatchCoef C,
@@ -323,6 +336,7 @@ __global__ void __launch_bounds__(256, J <= 4 ? 3 : 2) k_patch_sys(PatchArgs A, 
                 D.part_p[net * D.nslotv + (nd & 0x7fffffffu)] = a;
             } else {
                 const float xv = sp[net * V + i];
+                if (C.robin) a += patch_robin(D, net, nd & 0x3fffffffu, x);
                 patch_row<DOT>(O, row, C.bc && D.dof_bc[row] ? xv : a, r1, xv, cr, dot);
             }
         }
@@ -337,7 +351,7 @@ __global__ void __launch_bounds__(256, J <= 4 ? 3 : 2) k_patch_sys(PatchArgs A, 
 template <int J, bool DOT>
 __global__ void __launch_bounds__(256) k_patch_sys_shared(int64_t nsh, const int32_t* __restrict__ sh_node,
                                                           const int32_t* __restrict__ sh_ptr,
-                                                          const float4* __restrict__ part, PatchDims D, int bc,
+                                                          const float4* __restrict__ part, PatchDims D, int bc, int robin,
                                                           const float* __restrict__ x, PatchOut O, double* partials,
                                                           int first, unsigned* cnt,
                                                           const int32_t* __restrict__ node_inst,
@@ -387,6 +401,7 @@ __global__ void __launch_bounds__(256) k_patch_sys_shared(int64_t nsh, const int
             const float r1 = DOT ? O.r1[row] : 0.f, xv = x[row];
             float a = 0.f;
             for (int r = 0; r < n; ++r) a += D.part_p[net * D.nslotv + b + r];
+            if (robin) a += patch_robin(D, net, nd, x);
             patch_row<DOT>(O, row, bc && D.dof_bc[row] ? xv : a, r1, xv, cr, dot);
         }
     }
@@ -399,7 +414,8 @@ static void launch_patch_sys_j(mpet_ctx* c, const float* x, const PatchOut& O) {
     const PatchSet& s = c->patch;
     const size_t sm = sizeof(float) * ((size_t)5 * s.max_pn + (size_t)J * s.max_pv + (size_t)(30 + 4 * J) * s.P);
     const double* skip = s.inst ? c->skip_done : nullptr;
-    const PatchDims D{c->nv, c->Nu, (int)s.nshv, s.nslotv, s.part_p, c->dof_bc, s.sys, s.coef};
+    const PatchDims D{c->nv, c->Nu, (int)s.nshv, s.nslotv, s.part_p, c->dof_bc, s.sys, s.coef, c->bn_ptr, c->rob_col,
+                      c->rob_val, 3 * c->rob_n};
     // (reduction partials: one per block, at most NB_RED over both kernels)
     const int64_t items = s.nsh + (int64_t)J * s.nshv;
     const int g1 = (int)std::min<int64_t>(s.np, 456);
@@ -407,7 +423,7 @@ static void launch_patch_sys_j(mpet_ctx* c, const float* x, const PatchOut& O) {
     MPET_CUDA(cudaFuncSetAttribute(k_patch_sys<J, DOT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     launch_k(c, k_patch_sys<J, DOT>, g1, s.P, sm, patch_args(c), D, c->patch_coef, x, O, c->partials, skip);
     launch_k(c, k_patch_sys_shared<J, DOT>, g2, 256, 0, s.nsh, s.sh_node, s.sh_ptr, (const float4*)s.part, D,
-                                                          c->patch_coef.bc, x, O, c->partials, g1, c->red_cnt,
+                                                          c->patch_coef.bc, c->patch_coef.robin, x, O, c->partials, g1, c->red_cnt,
                                                           c->node_inst, skip);
     MPET_CHECK_LAUNCH();
     c->n_launch += 2;
@@ -428,7 +444,7 @@ static void launch_patch_sys(mpet_ctx* c, const float* x, const PatchOut& O) {
 }
 
 // products of the system matrix in the Krylov iterations: element patches where they serve
-// (c->sys_patch: mixed precision, tetrahedra, no Robin matrix term, no forced SpMV variant),
+// (c->sys_patch: mixed precision, tetrahedra, no forced SpMV variant, not a small matrix),
 // else the stored matrix
 template <typename T>
 static void krylov_product(mpet_ctx* c, const T* x, T* y) {

@@ -468,6 +468,11 @@ void build_pattern(mpet_ctx* c) {
         MPET_CUDA(cudaMemcpyAsync(rp.data(), c->A.rp, sizeof(int64_t) * (N + 1), cudaMemcpyDeviceToHost, s));
         MPET_CUDA(cudaStreamSynchronize(s));
         build_tiles(c, c->A, rp.data());
+        for (int64_t i = 0; i < c->nnodes; ++i) {
+            const int64_t len = rp[c->dim * i + 1] - rp[c->dim * i], rows = c->dim + (i < c->nv ? J : 0);
+            int& m = c->asm_rows[i < c->nv ? 0 : 1];
+            m = (int)std::max<int64_t>(m, std::min<int64_t>(len * rows, 1 << 20));
+        }
     }
     // preconditioner block patterns: u-Laplacian on n2, P1 blocks on the vertex rows of n1
     c->Lu.n = c->Lu.m = c->nnodes;

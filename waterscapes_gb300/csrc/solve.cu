@@ -635,9 +635,10 @@ __global__ void k_sell_width(int64_t n, int64_t nslices, const int64_t* __restri
     w32[sl] = 32 * w;
 }
 
-template <typename T>
+// (sci null: the columns are there already)
+template <typename T, typename Tin>
 __global__ void k_sell_fill(int64_t n, int64_t nslices, const int64_t* __restrict__ rp,
-                            const int32_t* __restrict__ ci, const T* __restrict__ v,
+                            const int32_t* __restrict__ ci, const Tin* __restrict__ v,
                             const int64_t* __restrict__ soff, int32_t* sci, T* sv) {
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (t >= nslices * 32) return;
@@ -646,16 +647,11 @@ __global__ void k_sell_fill(int64_t n, int64_t nslices, const int64_t* __restric
     const int64_t e0 = row < n ? rp[row] : 0, len = row < n ? rp[row + 1] - e0 : 0;
     // padding repeats the row's last column (a valid index of x, and a line
     // the row has just read), or column 0 for an empty row
-    const int32_t pad = len > 0 ? ci[e0 + len - 1] : 0;
+    const int32_t pad = sci && len > 0 ? ci[e0 + len - 1] : 0;
     for (int64_t k = 0; k < w; ++k) {
         const int64_t q = soff[sl] + k * 32 + lane;
-        if (k < len) {
-            sci[q] = ci[e0 + k];
-            sv[q] = v[e0 + k];
-        } else {
-            sci[q] = pad;
-            sv[q] = T(0);
-        }
+        if (sci) sci[q] = k < len ? ci[e0 + k] : pad;
+        sv[q] = k < len ? (T)v[e0 + k] : T(0);
     }
 }
 
@@ -1081,18 +1077,23 @@ void build_sell(mpet_ctx* c, Csr& A, bool fp32, bool with64) {
     if (fp32) A.s_v32 = c->pool.alloc<float>(acc);
     if (!fp32 || with64) A.s_v64 = c->pool.alloc<double>(acc);
     MPET_CUDA(cudaStreamSynchronize(c->stream));
-    fill_sell(c, A);
+    fill_sell(c, A, true, true);
 }
 
-void fill_sell(mpet_ctx* c, Csr& A) {
+// the values of the SELL copies from A.v64, the columns with the first fill
+void fill_sell(mpet_ctx* c, Csr& A, bool f32, bool f64) {
     if (!A.s_off) return;
     const int64_t ns = A.nslices;
-    if (A.s_v32)
-        k_sell_fill<float><<<grid_for(ns * 32, 256), 256, 0, c->stream>>>(A.n, ns, A.rp, A.ci, A.v32, A.s_off,
-                                                                          A.s_ci, A.s_v32);
-    if (A.s_v64)
-        k_sell_fill<double><<<grid_for(ns * 32, 256), 256, 0, c->stream>>>(A.n, ns, A.rp, A.ci, A.v64, A.s_off,
-                                                                           A.s_ci, A.s_v64);
+    auto cols = [&] {
+        int32_t* p = A.s_cols ? nullptr : A.s_ci;
+        A.s_cols = true;
+        return p;
+    };
+    const int G = grid_for(ns * 32, 256);
+    if (f32 && A.s_v32)
+        k_sell_fill<float, double><<<G, 256, 0, c->stream>>>(A.n, ns, A.rp, A.ci, A.v64, A.s_off, cols(), A.s_v32);
+    if (f64 && A.s_v64)
+        k_sell_fill<double, double><<<G, 256, 0, c->stream>>>(A.n, ns, A.rp, A.ci, A.v64, A.s_off, cols(), A.s_v64);
     MPET_CHECK_LAUNCH();
 }
 
@@ -1161,35 +1162,41 @@ void build_node_blocks(mpet_ctx* c) {
     c->A.nb = &nb;
 }
 
-static void fill_node_blocks(mpet_ctx* c) {
+// the values of the node-block copies from A.v64, the columns with the first fill
+static void fill_node_blocks(mpet_ctx* c, bool f32, bool f64) {
     NodeBlocks& nb = c->A_nb;
     if (!nb.sl) return;
     const int64_t ns = nb.nsu + nb.nsp;
     const int G = grid_for(ns * 32, 128);
-    int first = 1;
-    if (nb.v32) {
-        // from the FP32 CSR values when they exist (same rounding as the CSR kernels), else from FP64
-        if (c->A.v32)
-            k_nb_fill<float, float><<<G, 128, 0, c->stream>>>(c->nnodes, c->nv, c->Nu, c->J, nb.nsu, ns, nb.sl,
-                                                              nb.perm, c->A.rp, c->A.v32, c->n2_ptr, c->n2_col,
-                                                              c->n1_ptr, c->n1_col, nb.cols, nb.v32, first);
-        else
-            k_nb_fill<float, double><<<G, 128, 0, c->stream>>>(c->nnodes, c->nv, c->Nu, c->J, nb.nsu, ns, nb.sl,
-                                                               nb.perm, c->A.rp, c->A.v64, c->n2_ptr, c->n2_col,
-                                                               c->n1_ptr, c->n1_col, nb.cols, nb.v32, first);
-        first = 0;
+    if (f32 && nb.v32) {
+        k_nb_fill<float, double><<<G, 128, 0, c->stream>>>(c->nnodes, c->nv, c->Nu, c->J, nb.nsu, ns, nb.sl, nb.perm,
+                                                           c->A.rp, c->A.v64, c->n2_ptr, c->n2_col, c->n1_ptr,
+                                                           c->n1_col, nb.cols, nb.v32, nb.have_cols ? 0 : 1);
+        nb.have_cols = true;
     }
-    if (nb.v64)
-        k_nb_fill<double, double><<<G, 128, 0, c->stream>>>(c->nnodes, c->nv, c->Nu, c->J, nb.nsu, ns, nb.sl,
-                                                            nb.perm, c->A.rp, c->A.v64, c->n2_ptr, c->n2_col,
-                                                            c->n1_ptr, c->n1_col, nb.cols, nb.v64, first);
+    if (f64 && nb.v64) {
+        k_nb_fill<double, double><<<G, 128, 0, c->stream>>>(c->nnodes, c->nv, c->Nu, c->J, nb.nsu, ns, nb.sl, nb.perm,
+                                                            c->A.rp, c->A.v64, c->n2_ptr, c->n2_col, c->n1_ptr,
+                                                            c->n1_col, nb.cols, nb.v64, nb.have_cols ? 0 : 1);
+        nb.have_cols = true;
+    }
     MPET_CHECK_LAUNCH();
 }
 
-// After every change of the system matrix values: its SELL and node-block copies.
-void refresh_system_copies(mpet_ctx* c) {
-    fill_sell(c, c->A);
-    fill_node_blocks(c);
+__global__ void k_f64_to_f32(int64_t n, const double* __restrict__ a, float* b);
+
+void need_copies(mpet_ctx* c, unsigned which) {
+    which &= c->stale;
+    if (!which) return;
+    c->stale &= ~which;
+    if ((which & COPY_CSR32) && c->A.v32) {
+        k_f64_to_f32<<<grid_for(c->nnz, 256), 256, 0, c->stream>>>(c->nnz, c->A.v64, c->A.v32);
+        MPET_CHECK_LAUNCH();
+    }
+    if (which & (COPY_SELL32 | COPY_SELL64))
+        fill_sell(c, c->A, (which & COPY_SELL32) != 0, (which & COPY_SELL64) != 0);
+    if (which & (COPY_NB32 | COPY_NB64))
+        fill_node_blocks(c, (which & COPY_NB32) != 0, (which & COPY_NB64) != 0);
 }
 
 template <typename T>
@@ -1265,6 +1272,7 @@ struct EpiAddRhs {
 
 bool rhs_div_from_matrix(mpet_ctx* c, const double* up_prev, double* b) {
     if (!c->A.nb || !c->A.nb->v64 || c->dim != 3) return false;
+    need_copies(c, COPY_NB64);
     const NodeBlocks& nb = *c->A.nb;
     const int64_t ns = nb.nsu + nb.nsp;
     int blocks = grid_for(nb.nsp * 32, 256);
@@ -1305,6 +1313,20 @@ template <>
 const double* sell_vals<double>(const Csr& A) { return A.s_v64; }
 template <>
 const float* sell_vals<float>(const Csr& A) { return A.s_v32; }
+
+// (the choices of launch_spmv)
+template <typename T>
+void need_system_copy(mpet_ctx* c) {
+    constexpr bool d = sizeof(T) == 8;
+    const Csr& A = c->A;
+    const int variant = d && A.variant64 >= 0 ? A.variant64 : A.variant;
+    if ((variant == 8 || variant == 9) && A.nb && nb_vals<T>(*A.nb)) need_copies(c, d ? COPY_NB64 : COPY_NB32);
+    else if ((variant & 4) && sell_vals<T>(A)) need_copies(c, d ? COPY_SELL64 : COPY_SELL32);
+    else if (!d) need_copies(c, COPY_CSR32);
+    if (c->u_elast) need_copies(c, d ? COPY_NB64 : COPY_NB32);  // (first level of the elasticity hierarchy)
+}
+template void need_system_copy<double>(mpet_ctx*);
+template void need_system_copy<float>(mpet_ctx*);
 
 #include "tile.cuh"
 
@@ -1491,7 +1513,10 @@ __device__ __forceinline__ double sum_partials_n(const double* p, int n, double*
 
 #include "patch.cuh"
 
-void krylov_product_f32(mpet_ctx* c, const float* x, float* y) { krylov_product<float>(c, x, y); }
+void krylov_product_f32(mpet_ctx* c, const float* x, float* y) {
+    if (!c->sys_patch) need_system_copy<float>(c);
+    krylov_product<float>(c, x, y);
+}
 
 // operator of an AMG level: its CSR copy, the matrix-free first displacement
 // level, or the displacement block of the system
@@ -1650,6 +1675,7 @@ static void autotune_hier(mpet_ctx* c, AmgHier& h) {
 
 template <typename T>
 void spmv(mpet_ctx* c, const Csr& A, int nvec, const T* x, T* y) {
+    if (&A == &c->A) need_system_copy<T>(c);
     if (nvec == 4) launch_spmv<T, 4>(c, A, vals<T>(A), x, EpiStore<T, 4>{y});
     else launch_spmv<T, 1>(c, A, vals<T>(A), x, EpiStore<T, 1>{y});
 }
@@ -2624,11 +2650,13 @@ static int solve_impl(mpet_ctx* c, const double* b, double* x, mpet_stats* st, b
 }
 
 void apply_preconditioner(mpet_ctx* c, int precision, const void* r, void* z) {
+    if (c->u_elast) need_copies(c, precision == MPET_PRECISION_MIXED ? COPY_NB32 : COPY_NB64);
     if (precision == MPET_PRECISION_MIXED) precond<float>(c, (const float*)r, (float*)z);
     else precond<double>(c, (const double*)r, (double*)z);
 }
 
 void residual_norms(mpet_ctx* c, const double* b, const double* x, double* r, double* norms) {
+    need_system_copy<double>(c);
     launch_spmv<double, 1>(c, c->A, c->A.v64, x, EpiResid64{r, b, c->dinv});
     k_outer_norms<<<1, 256, 0, c->stream>>>(c->sc, c->partials);
     MPET_CHECK_LAUNCH();
@@ -3758,6 +3786,10 @@ static int solve_constrained(mpet_ctx* c, const double* b, double* x, mpet_stats
 }
 
 int solve_system(mpet_ctx* c, const double* b, double* x, mpet_stats* st, bool homogeneous) {
+    // the stored copies that the products of this solve read
+    need_system_copy<double>(c);
+    if (c->prm.precision == MPET_PRECISION_MIXED && !c->sys_patch) need_system_copy<float>(c);
+    if (c->prm.precision == MPET_PRECISION_MIXED && c->u_elast) need_copies(c, COPY_NB32);
     MPET_CUDA(cudaEventRecord(c->ev_sv0, c->stream));
     int s;
     if (c->gmres && (c->ninst > 0 || c->nrigid > 0))
@@ -4135,6 +4167,7 @@ static double csr_rho(mpet_ctx* c, const Csr& A, const double* dinv) {
 }
 
 bool setup_u_elasticity(mpet_ctx* c, bool fp32) {
+    need_copies(c, fp32 ? COPY_NB32 : COPY_NB64);
     c->u_elast = false;
     if (c->dim != 3 || !c->A.nb || c->ninst > 0 || c->nrigid > 0) return false;
     if (fp32 ? !c->A.nb->v32 : !c->A.nb->v64) return false;
@@ -4297,10 +4330,5 @@ bool setup_u_elasticity(mpet_ctx* c, bool fp32) {
 
 // ---- public helpers used by the API ------------------------------------------------------
 
-void convert_values_to_f32(mpet_ctx* c) {
-    if (!c->A.v32) return;
-    k_f64_to_f32<<<grid_for(c->nnz, 256), 256, 0, c->stream>>>(c->nnz, c->A.v64, c->A.v32);
-    MPET_CHECK_LAUNCH();
-}
 
 }  // namespace mpet
