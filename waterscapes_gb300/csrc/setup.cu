@@ -1191,10 +1191,11 @@ void build_row_tiles(mpet_ctx* c, Csr& A, const int32_t* order, int nvec, bool f
     if (n == 0 || nnz == 0 || nnz >= 2147483647LL || !A.v64) return;
     const size_t ev = (fp32 ? 4 : 8) + 2;
     if (!device_fits(c, (size_t)nnz * (24 + ev + ev / 4) + (size_t)n * 24)) return;
-    // Rows per tile: 256 (the more rows, the fewer x entries per row: the displacement level at
-    // 64^3 takes 1650, 1237 and 1071 us with 64, 128 and 256, 1157 with 512), less on a small level
-    // so that every SM has two tiles.
-    int R = 256;
+    // Rows per tile: 256 on a large level (the more rows, the fewer x entries per row: the
+    // displacement level at 64^3 takes 1650, 1237 and 1071 us with 64, 128 and 256, 1157 with 512);
+    // 128 below 400,000 rows, where the tiles are few waves of blocks (24^3, 118,000 rows: 205 us
+    // per iteration against 237 with 256); less on a small level so that every SM has two tiles.
+    int R = n >= 400000 ? 256 : 128;
     while (R > 32 && n < (int64_t)R * 304) R >>= 1;
     for (; R >= 32; R >>= 1)
         if (build_tiles_of(c, A, order, nvec, fp32, R)) return;
