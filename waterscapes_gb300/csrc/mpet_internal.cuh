@@ -456,9 +456,12 @@ struct mpet_ctx {
     void* gm_w = nullptr;
     void* gm_r = nullptr;
     double* gm_part = nullptr;    // (restart + 1) * NB_RED reduction partials
-    double* gm_h = nullptr;       // restart + 1 device scalars
+    unsigned* gm_cnt = nullptr;   // arrival counters of the reductions
+    double* gm_h = nullptr;       // 2 restart + 3 device scalars
     double* gm_h_host = nullptr;  // pinned
     int gm_m = 0;                 // restart length the buffers hold
+    cudaGraphExec_t gm_graph = nullptr;  // w = M^-1 A v
+    int64_t gm_graph_launches = 0;
     bool elem_tried = false;
     int elem_kernel = 1;          // element blocks of tetrahedra: 1 tensor cores, 0 FP64 CUDA cores
     bool amg_device = true;       // Laplacian-form hierarchies built on the GPU (false: host set-up)
