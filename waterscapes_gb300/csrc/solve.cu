@@ -178,12 +178,40 @@ struct EpiAxpby {
     }
 };
 
-// One Chebyshev step on D^-1 A: d = c1 d + c2 D^-1 (b - A xin); xout = xin + d.
+// y = A x, and the first Chebyshev step from zero for the level whose right-hand side y is:
+// x0 = f D^-1 y.  One launch and one read of y less than a kernel of its own for the step.
+template <typename T, int NV>
+struct EpiStoreFirst {
+    T* y;
+    T* x0;
+    const T* dinv;
+    T f;
+    static constexpr bool kTile = false;  // runs with the row-tile kernel
+    static constexpr int kRed = 0;
+    static constexpr bool kSystem = false;
+    struct Pre {
+        T di;
+    };
+    __device__ __forceinline__ Pre pre(int64_t row) const { return Pre{dinv[row]}; }
+    __device__ __forceinline__ void apply(int64_t row, const T* acc, const Pre& p, double&, double&) const {
+        T v[NV] = {};
+#pragma unroll
+        for (int k = 0; k < ncomp<NV>(); ++k) v[k] = p.di * acc[k] * f;
+        VecIO<T, NV>::store(y, row, acc);
+        VecIO<T, NV>::store(x0, row, v);
+    }
+};
+
+// One Chebyshev step on D^-1 A: d = c1 din + c2 D^-1 (b - A xin); xout = xin + d.  din: null on the
+// first step from a given xin, xin itself on the second step from zero (the first step's d is its
+// result).  dout: null on the last step.  (With d read and written at every step a smoothing of
+// two steps moved four vectors more.)
 template <typename T, int NV>
 struct EpiCheb {
     const T* b;
     const T* xin;
-    T* d;
+    const T* din;
+    T* dout;
     T* xout;
     const T* dinv;
     T c1, c2;
@@ -197,7 +225,10 @@ struct EpiCheb {
         Pre p;
         p.di = dinv[row];
         VecIO<T, NV>::load(b, row, p.bb);
-        VecIO<T, NV>::load(d, row, p.dd);
+        if (din) VecIO<T, NV>::load(din, row, p.dd);
+        else
+#pragma unroll
+            for (int k = 0; k < NV; ++k) p.dd[k] = T(0);
         VecIO<T, NV>::load(xin, row, p.xx);
         return p;
     }
@@ -208,7 +239,7 @@ struct EpiCheb {
             dd[k] = c1 * p.dd[k] + c2 * p.di * (p.bb[k] - acc[k]);
             xx[k] = p.xx[k] + dd[k];
         }
-        VecIO<T, NV>::store(d, row, dd);
+        if (dout) VecIO<T, NV>::store(dout, row, dd);
         VecIO<T, NV>::store(xout, row, xx);
     }
 };
@@ -1661,7 +1692,7 @@ static void autotune_hier(mpet_ctx* c, AmgHier& h) {
         for (void* p : {L.x, L.b, L.r, L.d, L.t0}) MPET_CUDA(cudaMemsetAsync(p, 0, bytes, c->stream));
         const T* dinv = dinv_of<T>(L);
         autotune_matrix<T, NV>(c, L.A, (const T*)L.x,
-                               EpiCheb<T, NV>{(const T*)L.b, (const T*)L.x, (T*)L.d, (T*)L.t0, dinv, T(0.5), T(0.5)});
+                               EpiCheb<T, NV>{(const T*)L.b, (const T*)L.x, (const T*)L.d, (T*)L.d, (T*)L.t0, dinv, T(0.5), T(0.5)});
         if (k + 1 < h.lev.size()) {
             AmgLevel& C = h.lev[k + 1];
             MPET_CUDA(cudaMemsetAsync(C.x, 0, sizeof(double) * C.A.n * NV, c->stream));
@@ -1685,14 +1716,12 @@ template void spmv<float>(mpet_ctx*, const Csr&, int, const float*, float*);
 // ---- vector kernels ----------------------------------------------------------------
 
 template <typename T>
-__global__ void k_cheb_first(int64_t n, int nvec, const T* __restrict__ b, const T* __restrict__ dinv, T* d, T* x,
+__global__ void k_cheb_first(int64_t n, int nvec, const T* __restrict__ b, const T* __restrict__ dinv, T* x,
                              T inv_theta) {
     pdl_wait();
     int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
-    T v = dinv[i / nvec] * b[i] * inv_theta;
-    d[i] = v;
-    x[i] = v;
+    x[i] = dinv[i / nvec] * b[i] * inv_theta;
 }
 
 // Coarsest level: a warp per row of the dense FP64 inverse, every component of the row from one
@@ -1861,7 +1890,7 @@ __device__ __forceinline__ double sum_partials_n(const double* p, int n, double*
 // itself, without packing).
 //
 // k_mr_lanczos: y -= c_r2 r2, and the displacement rows of y in the padded layout that the
-// preconditioner's first level takes.  k_mr_dot: the preconditioned vector z from that layout,
+// preconditioner's first level takes, with that level's first smoothing step.  k_mr_dot: the preconditioned vector z from that layout,
 // the partial sums of r . z, and in the block that arrives last the scalar step of the iteration.
 // k_mr_direction: w = (v - oldeps w1 - delta w2) / gamma, d += phi w, v = z / beta (the next
 // Lanczos vector).  Against one kernel per operation (nine a iteration with two single-block ones)
@@ -1870,6 +1899,7 @@ __device__ __forceinline__ double sum_partials_n(const double* p, int n, double*
 template <typename T>
 __global__ void __launch_bounds__(256) k_mr_lanczos(int64_t nodes, int dim, int64_t n, T* y,
                                                     const T* __restrict__ r2, T* packed,
+                                                    T* first, const T* __restrict__ dinv, T inv_theta,
                                                     const int32_t* __restrict__ perm, const MinresScalars* sc) {
     pdl_wait();
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -1882,7 +1912,14 @@ __global__ void __launch_bounds__(256) k_mr_lanczos(int64_t nodes, int dim, int6
 #pragma unroll
         for (int k = 0; k < 3; ++k)
             if (k < dim) y[dim * i + k] = v[k];
-        VecIO<T, 4>::store(packed, perm ? perm[i] : i, v);
+        const int64_t p = perm ? perm[i] : i;
+        VecIO<T, 4>::store(packed, p, v);
+        if (first) {
+            const T f = dinv[p] * inv_theta;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) v[k] *= f;
+            VecIO<T, 4>::store(first, p, v);
+        }
     } else {
         const int64_t row = dim * nodes + (i - nodes);
         if (row < n) y[row] -= c * r2[row];
@@ -1970,41 +2007,61 @@ __global__ void k_f64_to_f32(int64_t n, const double* __restrict__ a, float* b) 
 
 // ---- AMG V-cycle -------------------------------------------------------------------------
 
-template <typename T, int NV>
-static void cheb(mpet_ctx* c, AmgHier& h, AmgLevel& L, const T* b, const T* xin, T* xout) {
-    const int nv = NV;
-    const int64_t n = L.A.n * nv;
+static int cheb_degree(const AmgHier& h, size_t k) {
+    return k == 0 ? h.cheb_degree0 : ((int64_t)k >= h.cheb_level_c ? h.cheb_degree_c : h.cheb_degree);
+}
+// centre of the interval of D^-1 A that the smoother of a level damps
+static double cheb_theta(const AmgLevel& L) {
     const double hi = 1.1 * L.rho, lo = hi / 30.0;
-    const double theta = 0.5 * (hi + lo), delta = 0.5 * (hi - lo);
+    return 0.5 * (hi + lo);
+}
+// where the first step from zero of level k's smoothing leaves its result
+template <typename T>
+static T* cheb_start(const AmgHier& h, size_t k) {
+    const AmgLevel& L = h.lev[k];
+    return (T*)(cheb_degree(h, k) == 1 ? L.x : L.t0);
+}
+
+// started: the first step from zero is in cheb_start already
+template <typename T, int NV>
+static void cheb(mpet_ctx* c, AmgHier& h, size_t k, const T* b, const T* xin, T* xout, bool started = false) {
+    AmgLevel& L = h.lev[k];
+    const int64_t n = L.A.n * NV;
+    const double hi = 1.1 * L.rho, lo = hi / 30.0;
+    const double theta = cheb_theta(L), delta = 0.5 * (hi - lo);
     const double sigma = theta / delta;
     double rho_old = 1.0 / sigma;
-    const int64_t lk = &L - &h.lev[0];
-    const int s = lk == 0 ? h.cheb_degree0 : (lk >= h.cheb_level_c ? h.cheb_degree_c : h.cheb_degree);
+    const int s = cheb_degree(h, k);
     T* d = (T*)L.d;
     T* t0 = (T*)L.t0;
     T* t1 = (T*)L.t1;
     const T* dinv = dinv_of<T>(L);
     T* cur = (s == 1) ? xout : t0;
+    const T* din = cur;
     if (!xin) {
-        launch_k(c, k_cheb_first<T>, grid_for(n, 256), 256, 0, n, nv, b, dinv, d, cur, (T)(1.0 / theta));
-        MPET_CHECK_LAUNCH();
-        c->n_launch++;
+        if (!started) {
+            launch_k(c, k_cheb_first<T>, grid_for(n, 256), 256, 0, n, NV, b, dinv, cur, (T)(1.0 / theta));
+            MPET_CHECK_LAUNCH();
+            c->n_launch++;
+        }
     } else {
-        const EpiCheb<T, NV> e{b, xin, d, cur, dinv, T(0), (T)(1.0 / theta)};
-        level_spmv<T, NV>(c, L, xin, e);
+        T* dout = s == 1 ? nullptr : d;
+        level_spmv<T, NV>(c, L, xin, EpiCheb<T, NV>{b, xin, nullptr, dout, cur, dinv, T(0), (T)(1.0 / theta)});
+        din = d;
     }
     for (int j = 1; j < s; ++j) {
         const double rho_new = 1.0 / (2.0 * sigma - rho_old);
         const T c1 = (T)(rho_new * rho_old), c2 = (T)(2.0 * rho_new / delta);
         T* nxt = (j == s - 1) ? xout : (cur == t0 ? t1 : t0);
-        level_spmv<T, NV>(c, L, cur, EpiCheb<T, NV>{b, cur, d, nxt, dinv, c1, c2});
+        level_spmv<T, NV>(c, L, cur, EpiCheb<T, NV>{b, cur, din, j == s - 1 ? nullptr : d, nxt, dinv, c1, c2});
         cur = nxt;
+        din = d;
         rho_old = rho_new;
     }
 }
 
 template <typename T, int NV>
-static void vcycle(mpet_ctx* c, AmgHier& h, size_t k, const T* b, T* x) {
+static void vcycle(mpet_ctx* c, AmgHier& h, size_t k, const T* b, T* x, bool started = false) {
     if (k + 1 == h.lev.size()) {
         launch_k(c, k_dense_coarse<T, NV>, grid_for(h.ncoarse * 32, 64), 64, 0, h.ncoarse, h.cinv, b, x);
         MPET_CHECK_LAUNCH();
@@ -2015,14 +2072,21 @@ static void vcycle(mpet_ctx* c, AmgHier& h, size_t k, const T* b, T* x) {
     AmgLevel& C = h.lev[k + 1];
     T* xs = (T*)L.x;
     T* r = (T*)L.r;
-    cheb<T, NV>(c, h, L, b, nullptr, xs);
+    cheb<T, NV>(c, h, k, b, nullptr, xs, started);
     level_spmv<T, NV>(c, L, xs, EpiAxpby<T, NV>{r, b, T(-1), T(1)});
     const Csr& R = L.tiled() ? L.Rt : L.R;
     const Csr& P = L.tiled() ? L.Pt : L.P;
-    launch_spmv<T, NV>(c, R, vals<T>(R), r, EpiStore<T, NV>{(T*)C.b});
-    vcycle<T, NV>(c, h, k + 1, (const T*)C.b, (T*)C.x);
+    // The restriction starts the coarse level's smoothing.  Not where batch instances are skipped:
+    // a smoothing that went on from a skipped row's old iterate could grow from cycle to cycle.
+    const bool start = k + 2 < h.lev.size() && !c->skip_done;
+    if (start)
+        launch_spmv<T, NV>(c, R, vals<T>(R), r, EpiStoreFirst<T, NV>{(T*)C.b, cheb_start<T>(h, k + 1), dinv_of<T>(C),
+                                                                     (T)(1.0 / cheb_theta(C))});
+    else
+        launch_spmv<T, NV>(c, R, vals<T>(R), r, EpiStore<T, NV>{(T*)C.b});
+    vcycle<T, NV>(c, h, k + 1, (const T*)C.b, (T*)C.x, start);
     launch_spmv<T, NV>(c, P, vals<T>(P), (const T*)C.x, EpiAxpby<T, NV>{xs, xs, T(1), T(1)});
-    cheb<T, NV>(c, h, L, b, xs, x);
+    cheb<T, NV>(c, h, k, b, xs, x);
 }
 
 // Per-level profile of one hierarchy: ms[k] = median time of a V-cycle
@@ -2061,7 +2125,7 @@ static void profile_levels(mpet_ctx* c, AmgHier& h, int reps, double* ms, double
             bytes[k] = (double)h.ncoarse * h.ncoarse * 8.0 + 2.0 * h.ncoarse * NV * sv;
             continue;
         }
-        const int s = k == 0 ? h.cheb_degree0 : ((int)k >= h.cheb_level_c ? h.cheb_degree_c : h.cheb_degree);
+        const int s = cheb_degree(h, k);
         const double nc = (double)h.lev[k + 1].A.n, vecc = nc * NV * sv;
         // a product with A: the CSR entries and row pointers, or (matrix-free) the
         // incidence and per-cell node ids (NN each), the per-cell data, the row
@@ -2069,8 +2133,9 @@ static void profile_levels(mpet_ctx* c, AmgHier& h, int reps, double* ms, double
         const double nn_cell = c->dim == 3 ? 10.0 : 6.0;
         const double mA = L.mf ? (double)c->nc * (2.0 * nn_cell * 4.0 + 8.0 * sv) + n + (n + 1) * 8.0
                                : L.A.nnz * (sv + 4.0) + (n + 1) * 8.0;
-        double b = 3 * vec + dv;                              // first Chebyshev step (no product)
-        b += (2 * s - 1) * (mA + 5 * vec + dv);               // the other 2s - 1 smoothing products
+        double b = 2 * vec + dv;                              // first Chebyshev step (no product)
+        b += (2 * s - 1) * (mA + 3 * vec + dv);               // the other 2s - 1 smoothing products
+        b += (2 * (s > 2 ? s - 2 : 0) + 2 * (s - 1)) * vec;   // ... the direction, between two of them
         b += mA + 3 * vec;                                    // residual
         b += L.R.nnz * (sv + 4.0) + (nc + 1) * 8.0 + vec + vecc;  // restriction
         b += L.P.nnz * (sv + 4.0) + (n + 1) * 8.0 + vecc + 2 * vec;  // prolongation + correction
@@ -2141,8 +2206,8 @@ static const int32_t* first_level_perm(const mpet_ctx* c) {
 // transforms) are forked onto side streams and run concurrently with the
 // displacement V-cycle on the main stream (inside a CUDA graph capture they
 // become parallel branches); the main stream joins them at the end.
-// packed: the displacement rows of r are already in the first level's input, and those of z are
-// left in its output (k_mr_lanczos, k_mr_dot).
+// packed: the displacement rows of r are already in the first level's input and its smoothing is
+// started, and those of z are left in its output (k_mr_lanczos, k_mr_dot).
 template <typename T>
 static void precond(mpet_ctx* c, const T* r, T* z, bool packed = false) {
     cudaStream_t main = c->stream;
@@ -2180,7 +2245,7 @@ static void precond(mpet_ctx* c, const T* r, T* z, bool packed = false) {
             k_pack34<T><<<grid_for(nodes, 256), 256, 0, main>>>(nodes, c->dim, r, bin, perm);
             c->n_launch++;
         }
-        vcycle<T, 4>(c, hu, 0, bin, xout);
+        vcycle<T, 4>(c, hu, 0, bin, xout, packed && hu.lev.size() > 1);
         if (!packed) {
             k_unpack43<T><<<grid_for(nodes, 256), 256, 0, main>>>(nodes, c->dim, xout, z, perm);
             c->n_launch++;
@@ -2211,6 +2276,7 @@ static void minres_three(mpet_ctx* c) {
     const AmgHier& hu = c->amg_u;
     const int64_t nodes = pack ? c->nnodes : 0, items = nodes + (n - c->dim * nodes);
     const int32_t* perm = pack ? first_level_perm(c) : nullptr;
+    T* first = pack && hu.lev.size() > 1 ? cheb_start<T>(hu, 0) : nullptr;
     const int G = grid_for(items, 256);
     // two blocks per SM (each block's FP64 sum takes half a microsecond of its SM's FP64 pipe), more
     // where that leaves a thread more than 16 rows
@@ -2226,7 +2292,9 @@ static void minres_three(mpet_ctx* c) {
         T* y = (T*)c->kr[iy];
         minres_product<T>(c, EpiMinres<T>{y, r1, v, c->sc});
         c->n_spmv++;
-        launch_k(c, k_mr_lanczos<T>, G, 256, 0, nodes, c->dim, n, y, r2, (T*)hu.pack_in, perm, c->sc);
+        launch_k(c, k_mr_lanczos<T>, G, 256, 0, nodes, c->dim, n, y, r2, (T*)hu.pack_in, first,
+                 first ? dinv_of<T>(hu.lev[0]) : (const T*)nullptr, first ? (T)(1.0 / cheb_theta(hu.lev[0])) : T(0), perm,
+                 c->sc);
         MPET_CHECK_LAUNCH();
         const int old1 = ir1;
         ir1 = ir2;
@@ -3923,7 +3991,7 @@ static void choose_mf(mpet_ctx* c, AmgHier& h) {
     constexpr size_t kFlush = 256u << 20;
     if (!c->l2_flush) c->l2_flush = c->pool.alloc<unsigned char>(kFlush);
     const int64_t l0 = c->n_launch;
-    const EpiCheb<T, 4> e{(const T*)L.b, (const T*)L.x, (T*)L.d, (T*)L.t0, dinv_of<T>(L), T(0.5), T(0.5)};
+    const EpiCheb<T, 4> e{(const T*)L.b, (const T*)L.x, (const T*)L.d, (T*)L.d, (T*)L.t0, dinv_of<T>(L), T(0.5), T(0.5)};
     float med[2];
     for (int v = 0; v < 2; ++v) {
         L.mf = v == 1;
