@@ -521,7 +521,7 @@ struct mpet_ctx {
     double* bdone = nullptr;
     double* bdone_host = nullptr;             // pinned
     double* btarget = nullptr;
-    double* bval = nullptr;                   // per-instance reduced sums
+    unsigned* bcnt = nullptr;                 // per-instance arrivals of chunk sums
     cudaGraphExec_t bmr_graph = nullptr;
     int64_t bmr_graph_launches = 0;
     // instance of each P2 node (vertices first), the skip maps of the matrices

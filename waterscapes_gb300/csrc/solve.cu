@@ -1539,6 +1539,7 @@ static void launch_p2lap_mf(mpet_ctx* c, const T* x, const Epi& epi) {
 // (defined with the MINRES kernels)
 __device__ void mr_alfa_one(MinresScalars* s, double t);
 __global__ void k_mr_alfa(MinresScalars* s, const double* partials);
+__device__ __forceinline__ bool last_of(unsigned* cnt, unsigned blocks);
 __device__ __forceinline__ bool last_block(unsigned* cnt);
 __device__ __forceinline__ double sum_partials_n(const double* p, int n, double* sh);
 
@@ -1864,19 +1865,20 @@ __global__ void k_mr_alfa(MinresScalars* s, const double* partials) {
     double t = sum_partials(partials, sh);
     if (threadIdx.x == 0) mr_alfa_one(s, t);
 }
-// True in the block of this launch that arrives last (every block calls it once, after thread 0
-// has written the block's partial); that block may read the others' partials.  The counter wraps
-// to zero for the next launch.
-__device__ __forceinline__ bool last_block(unsigned* cnt) {
+// True in the block that arrives last of the `blocks` of this launch that count at cnt (each calls
+// it once, after thread 0 has written the block's partial); that block may read the others'
+// partials.  The counter wraps to zero for the next launch.
+__device__ __forceinline__ bool last_of(unsigned* cnt, unsigned blocks) {
     __shared__ bool last;
     if (threadIdx.x == 0) {
         __threadfence();
-        last = atomicInc(cnt, gridDim.x - 1) == gridDim.x - 1;
+        last = atomicInc(cnt, blocks - 1) == blocks - 1;
         __threadfence();
     }
     __syncthreads();
     return last;
 }
+__device__ __forceinline__ bool last_block(unsigned* cnt) { return last_of(cnt, gridDim.x); }
 
 // Sum of n partials by one 256-thread block (fixed order); for the last block of a launch.
 __device__ __forceinline__ double sum_partials_n(const double* p, int n, double* sh) {
@@ -2206,10 +2208,11 @@ static const int32_t* first_level_perm(const mpet_ctx* c) {
 // transforms) are forked onto side streams and run concurrently with the
 // displacement V-cycle on the main stream (inside a CUDA graph capture they
 // become parallel branches); the main stream joins them at the end.
-// packed: the displacement rows of r are already in the first level's input and its smoothing is
-// started, and those of z are left in its output (k_mr_lanczos, k_mr_dot).
+// packed: the displacement rows of r are already in the first level's input, and those of z are
+// left in its output (k_mr_lanczos, k_mr_dot; k_bmr_axpy, k_bmr_beta).  started: so is the first
+// step of that level's smoothing (k_mr_lanczos).
 template <typename T>
-static void precond(mpet_ctx* c, const T* r, T* z, bool packed = false) {
+static void precond(mpet_ctx* c, const T* r, T* z, bool packed = false, bool started = false) {
     cudaStream_t main = c->stream;
     const T* rp = r + c->Nu;
     T* zp = z + c->Nu;
@@ -2245,7 +2248,7 @@ static void precond(mpet_ctx* c, const T* r, T* z, bool packed = false) {
             k_pack34<T><<<grid_for(nodes, 256), 256, 0, main>>>(nodes, c->dim, r, bin, perm);
             c->n_launch++;
         }
-        vcycle<T, 4>(c, hu, 0, bin, xout, packed && hu.lev.size() > 1);
+        vcycle<T, 4>(c, hu, 0, bin, xout, started);
         if (!packed) {
             k_unpack43<T><<<grid_for(nodes, 256), 256, 0, main>>>(nodes, c->dim, xout, z, perm);
             c->n_launch++;
@@ -2300,7 +2303,7 @@ static void minres_three(mpet_ctx* c) {
         ir1 = ir2;
         ir2 = iy;
         iy = old1;
-        precond<T>(c, (const T*)c->kr[ir2], (T*)c->kr[iy], pack);
+        precond<T>(c, (const T*)c->kr[ir2], (T*)c->kr[iy], pack, first != nullptr);
         launch_k(c, k_mr_dot<T>, Gd, 256, 0, nodes, c->dim, n, (const T*)c->kr[ir2], (T*)c->kr[iy],
                                                (const T*)hu.pack_out, perm, c->partials, c->red_cnt, c->sc);
         const int oldw1 = iw1;
@@ -2765,26 +2768,6 @@ __global__ void k_seg_dot(const int64_t* __restrict__ lo, const int32_t* __restr
     if (threadIdx.x == 0) part[ch] = s;
 }
 
-// k_seg_dot for the batched iterations: a converged instance's chunks contribute 0
-template <typename T>
-__global__ void k_seg_dot_open(const int64_t* __restrict__ lo, const int32_t* __restrict__ len,
-                               const int32_t* __restrict__ inst, const T* __restrict__ a, const T* __restrict__ b,
-                               double* part, const double* __restrict__ done) {
-    __shared__ double sh[8];
-    const int64_t ch = blockIdx.x;
-    if (done[inst[ch]] != 0.0) {
-        if (threadIdx.x == 0) part[ch] = 0.0;
-        return;
-    }
-    T acc = T(0);  // a thread's 16 products in the working precision, then FP64
-    for (int i = threadIdx.x; i < len[ch]; i += 256) {
-        const int64_t r = lo[ch] + i;
-        acc += a[r] * b[r];
-    }
-    const double s = block_sum256((double)acc, sh);
-    if (threadIdx.x == 0) part[ch] = s;
-}
-
 // (r D^-1)^2 and (b D^-1)^2 per chunk
 __global__ void k_seg_norms(const int64_t* __restrict__ lo, const int32_t* __restrict__ len, int64_t nch,
                             const double* __restrict__ r, const double* __restrict__ b,
@@ -2893,9 +2876,18 @@ __global__ void k_batch_status(int ninst, double* iv, double rtol, int first) {
 //
 // The vectors hold all instances; every scalar (alpha, beta, the Givens
 // rotation) is per instance, and the dots are per-instance chunk sums.  An
-// instance that reaches its target is frozen: its scalars are zeroed at the
-// start of the next iteration, so its Lanczos vectors and its correction
-// stop changing while the others continue.
+// instance that reaches its target is frozen: its scalars are zeroed in the
+// next iteration, so its Lanczos vectors and its correction stop changing
+// while the others continue.
+//
+// done: 0 open, 2 converged in this or the previous iteration (the update still counts), 1
+// settled; the chunks of instances that are not open are skipped.
+//
+// An iteration's vector work is four kernels, a block per chunk: y -= c_r1 r1 with v . y, y -= c_r2
+// r2 into the layout of the preconditioner's first level, z out of that layout with r . z, and the
+// update with the next v.  The block of an instance that arrives last sums its chunks and takes
+// the instance's scalar step.  (24 cubes of 6^3..16^3: 338 us per iteration, 346 with twelve kernels
+// and the sums of an instance in one thread.)
 
 template <typename T>
 __global__ void k_bmr_v(const int64_t* __restrict__ lo, const int32_t* __restrict__ len,
@@ -2905,58 +2897,6 @@ __global__ void k_bmr_v(const int64_t* __restrict__ lo, const int32_t* __restric
     if (done[inst[ch]] != 0.0) return;  // a converged instance's chunks are left as they are
     const T ib = msc<T>(sc[inst[ch]].inv_beta, sc[inst[ch]].f_inv_beta);
     for (int i = threadIdx.x; i < len[ch]; i += 256) v[lo[ch] + i] = y[lo[ch] + i] * ib;
-}
-
-// y -= c_r1 r1 and the chunk sums of v . y
-template <typename T>
-__global__ void k_bmr_axpy_dot(const int64_t* __restrict__ lo, const int32_t* __restrict__ len,
-                               const int32_t* __restrict__ inst, T* y, const T* __restrict__ r1,
-                               const T* __restrict__ v, const MinresScalars* __restrict__ sc, double* part,
-                               const double* __restrict__ done) {
-    __shared__ double sh[8];
-    const int64_t ch = blockIdx.x;
-    if (done[inst[ch]] != 0.0) {
-        if (threadIdx.x == 0) part[ch] = 0.0;
-        return;
-    }
-    const T c1 = msc<T>(sc[inst[ch]].c_r1, sc[inst[ch]].f_c_r1);
-    T acc = T(0);  // a thread's 16 products in the working precision, then FP64
-    for (int i = threadIdx.x; i < len[ch]; i += 256) {
-        const int64_t r = lo[ch] + i;
-        const T yy = y[r] - c1 * r1[r];
-        y[r] = yy;
-        acc += v[r] * yy;
-    }
-    const double s = block_sum256((double)acc, sh);
-    if (threadIdx.x == 0) part[ch] = s;
-}
-
-template <typename T>
-__global__ void k_bmr_axpy(const int64_t* __restrict__ lo, const int32_t* __restrict__ len,
-                           const int32_t* __restrict__ inst, T* y, const T* __restrict__ r2,
-                           const MinresScalars* __restrict__ sc, const double* __restrict__ done) {
-    const int64_t ch = blockIdx.x;
-    if (done[inst[ch]] != 0.0) return;
-    const T c2 = msc<T>(sc[inst[ch]].c_r2, sc[inst[ch]].f_c_r2);
-    for (int i = threadIdx.x; i < len[ch]; i += 256) y[lo[ch] + i] -= c2 * r2[lo[ch] + i];
-}
-
-template <typename T>
-__global__ void k_bmr_update(const int64_t* __restrict__ lo, const int32_t* __restrict__ len,
-                             const int32_t* __restrict__ inst, const T* __restrict__ v, const T* __restrict__ w1,
-                             const T* __restrict__ w2, T* w, T* d, const MinresScalars* __restrict__ sc,
-                             const double* __restrict__ done) {
-    const int64_t ch = blockIdx.x;
-    if (done[inst[ch]] == 1.0) return;  // 2: converged by this iteration's beta, its update still counts
-    const MinresScalars& s = sc[inst[ch]];
-    const T oe = msc<T>(s.oldeps, s.f_oldeps), de = msc<T>(s.delta, s.f_delta);
-    const T ig = msc<T>(s.inv_gamma, s.f_inv_gamma), ph = msc<T>(s.phi, s.f_phi);
-    for (int i = threadIdx.x; i < len[ch]; i += 256) {
-        const int64_t r = lo[ch] + i;
-        const T wn = (v[r] - oe * w1[r] - de * w2[r]) * ig;
-        w[r] = wn;
-        d[r] += ph * wn;
-    }
 }
 
 __device__ void mr_freeze(MinresScalars* s) {
@@ -2969,6 +2909,134 @@ __device__ void mr_freeze(MinresScalars* s) {
     s->delta = 0.0;
     s->alfa = 0.0;
     mr_mirror(s);
+}
+
+// sum of the chunk partials of an instance by its last block (fixed order)
+__device__ __forceinline__ double sum_chunks(const double* part, const int32_t* __restrict__ chunks, int n, double* sh) {
+    double v = 0.0;
+    for (int k = threadIdx.x; k < n; k += 256) v += __ldcg(part + chunks[k]);
+    return block_sum256(v, sh);
+}
+
+// y -= c_r1 r1, alfa = v . y
+template <typename T>
+__global__ void __launch_bounds__(256) k_bmr_alfa(const int64_t* __restrict__ lo, const int32_t* __restrict__ len,
+                                                  const int32_t* __restrict__ inst, const int32_t* __restrict__ cptr,
+                                                  const int32_t* __restrict__ chunks, T* y, const T* __restrict__ r1,
+                                                  const T* __restrict__ v, MinresScalars* sc, double* part,
+                                                  unsigned* cnt, double* done) {
+    pdl_wait();
+    __shared__ double sh[8];
+    const int64_t ch = blockIdx.x;
+    const int in = inst[ch], c0 = cptr[in], nc = cptr[in + 1] - c0;
+    const double dn = done[in];
+    if (dn != 0.0) {
+        // converged in the previous iteration: settled once every block of the instance has seen it
+        if (dn == 2.0 && threadIdx.x == 0 && atomicInc(cnt + in, nc - 1) == (unsigned)(nc - 1)) {
+            mr_freeze(&sc[in]);
+            done[in] = 1.0;
+        }
+        return;
+    }
+    const T c1 = msc<T>(sc[in].c_r1, sc[in].f_c_r1);
+    T acc = T(0);  // a thread's 16 products in the working precision, then FP64
+    for (int i = threadIdx.x; i < len[ch]; i += 256) {
+        const int64_t r = lo[ch] + i;
+        const T yy = y[r] - c1 * r1[r];
+        y[r] = yy;
+        acc += v[r] * yy;
+    }
+    const double s = block_sum256((double)acc, sh);
+    if (threadIdx.x == 0) part[ch] = s;
+    if (!last_of(cnt + in, nc)) return;
+    const double t = sum_chunks(part, chunks + c0, nc, sh);
+    if (threadIdx.x == 0) mr_alfa_one(&sc[in], t);
+}
+
+// y -= c_r2 r2; its displacement rows (r < Nu; Nu = 0: none) also in the padded layout that the
+// preconditioner's first level takes, zeros there for a converged instance
+template <typename T>
+__global__ void __launch_bounds__(256) k_bmr_axpy(const int64_t* __restrict__ lo, const int32_t* __restrict__ len,
+                                                  const int32_t* __restrict__ inst, T* y, const T* __restrict__ r2,
+                                                  int64_t Nu, T* packed, const int32_t* __restrict__ perm,
+                                                  const MinresScalars* __restrict__ sc,
+                                                  const double* __restrict__ done) {
+    pdl_wait();
+    const int64_t ch = blockIdx.x;
+    const int in = inst[ch];
+    const bool open = done[in] == 0.0;
+    const T c2 = msc<T>(sc[in].c_r2, sc[in].f_c_r2);
+    for (int i = threadIdx.x; i < len[ch]; i += 256) {
+        const int64_t r = lo[ch] + i;
+        T yy = T(0);
+        if (open) {
+            yy = y[r] - c2 * r2[r];
+            y[r] = yy;
+        }
+        if (r < Nu) {
+            const int64_t node = r / 3;
+            packed[4 * (perm ? perm[node] : node) + (r - 3 * node)] = yy;
+        }
+    }
+}
+
+// beta^2 = r . z, the displacement rows of z from the padded layout of the first level's output;
+// the rotation of the iteration and the instance's convergence
+template <typename T>
+__global__ void __launch_bounds__(256) k_bmr_beta(const int64_t* __restrict__ lo, const int32_t* __restrict__ len,
+                                                  const int32_t* __restrict__ inst, const int32_t* __restrict__ cptr,
+                                                  const int32_t* __restrict__ chunks, const T* __restrict__ rr, T* z,
+                                                  int64_t Nu, const T* __restrict__ packed,
+                                                  const int32_t* __restrict__ perm, MinresScalars* sc, double* part,
+                                                  unsigned* cnt, const double* __restrict__ target, double* done) {
+    pdl_wait();
+    __shared__ double sh[8];
+    const int64_t ch = blockIdx.x;
+    const int in = inst[ch], c0 = cptr[in], nc = cptr[in + 1] - c0;
+    if (done[in] != 0.0) return;
+    T acc = T(0);
+    for (int i = threadIdx.x; i < len[ch]; i += 256) {
+        const int64_t r = lo[ch] + i;
+        T zz;
+        if (r < Nu) {
+            const int64_t node = r / 3;
+            zz = packed[4 * (perm ? perm[node] : node) + (r - 3 * node)];
+            z[r] = zz;
+        } else
+            zz = z[r];
+        acc += rr[r] * zz;
+    }
+    const double s = block_sum256((double)acc, sh);
+    if (threadIdx.x == 0) part[ch] = s;
+    if (!last_of(cnt + in, nc)) return;
+    const double t = sum_chunks(part, chunks + c0, nc, sh);
+    if (threadIdx.x != 0) return;
+    mr_beta_one(&sc[in], t);
+    if (sc[in].rel <= target[in] || sc[in].flag != 0.0) done[in] = 2.0;  // the update of this iteration still runs
+}
+
+// w = (v - oldeps w1 - delta w2) / gamma, d += phi w; v = z / beta for the next iteration
+template <typename T>
+__global__ void __launch_bounds__(256) k_bmr_update(const int64_t* __restrict__ lo, const int32_t* __restrict__ len,
+                                                    const int32_t* __restrict__ inst, const T* __restrict__ z, T* v,
+                                                    const T* __restrict__ w1, const T* __restrict__ w2, T* w, T* d,
+                                                    const MinresScalars* __restrict__ sc,
+                                                    const double* __restrict__ done) {
+    pdl_wait();
+    const int64_t ch = blockIdx.x;
+    const double dn = done[inst[ch]];
+    if (dn == 1.0) return;
+    const MinresScalars& s = sc[inst[ch]];
+    const T oe = msc<T>(s.oldeps, s.f_oldeps), de = msc<T>(s.delta, s.f_delta);
+    const T ig = msc<T>(s.inv_gamma, s.f_inv_gamma), ph = msc<T>(s.phi, s.f_phi);
+    const T ib = msc<T>(s.inv_beta, s.f_inv_beta);
+    for (int i = threadIdx.x; i < len[ch]; i += 256) {
+        const int64_t r = lo[ch] + i;
+        const T wn = (v[r] - oe * w1[r] - de * w2[r]) * ig;
+        w[r] = wn;
+        d[r] += ph * wn;
+        if (dn == 0.0) v[r] = z[r] * ib;
+    }
 }
 
 // start: q_i = rhs_i . M^-1 rhs_i; instances with active_i == 0 start frozen
@@ -2984,33 +3052,9 @@ __global__ void k_bmr_init(int ni, MinresScalars* sc, const double* q, const dou
     done[i] = on ? 0.0 : 1.0;
 }
 
-// done: 0 open, 2 converged in the previous iteration (its last update was still
-// applied), 1 settled; settled instances' chunks are skipped by the vector kernels
-__global__ void k_bmr_freeze(int ni, MinresScalars* sc, double* done) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < ni && done[i] != 0.0) {
-        mr_freeze(&sc[i]);
-        done[i] = 1.0;
-    }
-}
-
-__global__ void k_bmr_alfa(int ni, MinresScalars* sc, const double* t, const double* done) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < ni && done[i] == 0.0) mr_alfa_one(&sc[i], t[i]);
-}
-
-__global__ void k_bmr_beta(int ni, MinresScalars* sc, const double* t, const double* target, double* done) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= ni || done[i] != 0.0) return;
-    mr_beta_one(&sc[i], t[i]);
-    if (sc[i].rel <= target[i] || sc[i].flag != 0.0) done[i] = 2.0;  // the update of this iteration still runs
-}
-
 template <typename T>
 static void bminres_three(mpet_ctx* c) {
-    const int ni = c->ninst;
-    const int64_t nch = c->nchunks;
-    const int gi = grid_for(ni, 128);
+    const int nch = (int)c->nchunks;
     T* v = (T*)c->kv;
     T* d = (T*)c->kd;
     int ir1 = 0, ir2 = 1, iy = 2;
@@ -3022,40 +3066,35 @@ static void bminres_three(mpet_ctx* c) {
         ~SkipScope() { c->skip_done = nullptr; }
     } scope{c};
     c->skip_done = (c->batch_skip && c->skip_maps) ? c->bdone : nullptr;
+    const bool pack = !c->u_elast;  // (elasticity form: the hierarchy works on the rows as they are)
+    const int64_t Nu = pack ? c->Nu : 0;
+    const int32_t* perm = pack ? first_level_perm(c) : nullptr;
+    T* pin = (T*)c->amg_u.pack_in;
+    const T* pout = (const T*)c->amg_u.pack_out;
     for (int q = 0; q < 3; ++q) {
         T* r1 = (T*)c->kr[ir1];
         T* r2 = (T*)c->kr[ir2];
         T* y = (T*)c->kr[iy];
-        k_bmr_freeze<<<gi, 128, 0, c->stream>>>(ni, c->bsc, c->bdone);
-        k_bmr_v<T><<<(unsigned)nch, 256, 0, c->stream>>>(c->ch_lo, c->ch_len, c->ch_inst, y, v, c->bsc, c->bdone);
-        MPET_CHECK_LAUNCH();
         krylov_product<T>(c, v, y);
         c->n_spmv++;
-        k_bmr_axpy_dot<T><<<(unsigned)nch, 256, 0, c->stream>>>(c->ch_lo, c->ch_len, c->ch_inst, y, r1, v, c->bsc,
-                                                                 c->ch_part, c->bdone);
-        k_seg_finish<<<gi, 128, 0, c->stream>>>(ni, c->inst_cptr, c->inst_chunks, c->ch_part, nch, 1, c->bval);
-        k_bmr_alfa<<<gi, 128, 0, c->stream>>>(ni, c->bsc, c->bval, c->bdone);
-        k_bmr_axpy<T><<<(unsigned)nch, 256, 0, c->stream>>>(c->ch_lo, c->ch_len, c->ch_inst, y, r2, c->bsc,
-                                                             c->bdone);
+        launch_k(c, k_bmr_alfa<T>, nch, 256, 0, c->ch_lo, c->ch_len, c->ch_inst, c->inst_cptr, c->inst_chunks, y, r1, v,
+                 c->bsc, c->ch_part, c->bcnt, c->bdone);
+        launch_k(c, k_bmr_axpy<T>, nch, 256, 0, c->ch_lo, c->ch_len, c->ch_inst, y, r2, Nu, pin, perm, c->bsc, c->bdone);
         MPET_CHECK_LAUNCH();
-        c->n_launch += 6;
         const int old1 = ir1;
         ir1 = ir2;
         ir2 = iy;
         iy = old1;
-        precond<T>(c, (const T*)c->kr[ir2], (T*)c->kr[iy]);
-        k_seg_dot_open<T><<<(unsigned)nch, 256, 0, c->stream>>>(c->ch_lo, c->ch_len, c->ch_inst,
-                                                                (const T*)c->kr[ir2], (const T*)c->kr[iy],
-                                                                c->ch_part, c->bdone);
-        k_seg_finish<<<gi, 128, 0, c->stream>>>(ni, c->inst_cptr, c->inst_chunks, c->ch_part, nch, 1, c->bval);
-        k_bmr_beta<<<gi, 128, 0, c->stream>>>(ni, c->bsc, c->bval, c->btarget, c->bdone);
+        T* z = (T*)c->kr[iy];
+        precond<T>(c, (const T*)c->kr[ir2], z, pack, false);
+        launch_k(c, k_bmr_beta<T>, nch, 256, 0, c->ch_lo, c->ch_len, c->ch_inst, c->inst_cptr, c->inst_chunks,
+                 (const T*)c->kr[ir2], z, Nu, pout, perm, c->bsc, c->ch_part, c->bcnt, c->btarget, c->bdone);
         const int oldw1 = iw1;
         iw1 = iw2;
         iw2 = iw;
         iw = oldw1;
-        k_bmr_update<T><<<(unsigned)nch, 256, 0, c->stream>>>(c->ch_lo, c->ch_len, c->ch_inst, v,
-                                                              (const T*)c->kw[iw1], (const T*)c->kw[iw2],
-                                                              (T*)c->kw[iw], d, c->bsc, c->bdone);
+        launch_k(c, k_bmr_update<T>, nch, 256, 0, c->ch_lo, c->ch_len, c->ch_inst, z, v, (const T*)c->kw[iw1],
+                 (const T*)c->kw[iw2], (T*)c->kw[iw], d, c->bsc, c->bdone);
         MPET_CHECK_LAUNCH();
         c->n_launch += 4;
     }
@@ -3079,6 +3118,11 @@ static int bminres_run(mpet_ctx* c, int max_iters, int* iters_done) {
             },
             &c->bmr_graph, &c->bmr_graph_launches, "batched MINRES");
     const int ni = c->ninst;
+    // the Lanczos vector that the captured iterations start from
+    k_bmr_v<T><<<(unsigned)c->nchunks, 256, 0, c->stream>>>(c->ch_lo, c->ch_len, c->ch_inst, (const T*)c->kr[2],
+                                                            (T*)c->kv, c->bsc, c->bdone);
+    MPET_CHECK_LAUNCH();
+    c->n_launch++;
     run_while_graph(c, c->bmr_graph, 0.0, max_iters);
     MPET_CUDA(cudaMemcpyAsync(c->bdone_host, c->bdone, sizeof(double) * ni, cudaMemcpyDeviceToHost, c->stream));
     MPET_CUDA(cudaMemcpyAsync(c->bsc_host, c->bsc, sizeof(MinresScalars) * ni, cudaMemcpyDeviceToHost, c->stream));
@@ -3274,7 +3318,8 @@ void setup_batch(mpet_ctx* c, int ninst, const int32_t* vertex_inst) {
     c->bsc = c->pool.alloc<MinresScalars>(ninst);
     c->bdone = c->pool.alloc<double>(ninst);
     c->btarget = c->pool.alloc<double>(ninst);
-    c->bval = c->pool.alloc<double>(ninst);
+    c->bcnt = c->pool.alloc<unsigned>(ninst);
+    MPET_CUDA(cudaMemsetAsync(c->bcnt, 0, sizeof(unsigned) * ninst, c->stream));
     MPET_CUDA(cudaMallocHost(&c->bsc_host, sizeof(MinresScalars) * ninst));
     MPET_CUDA(cudaMallocHost(&c->bdone_host, sizeof(double) * ninst));
     c->node_inst = c->pool.alloc<int32_t>(c->nnodes);
