@@ -2954,7 +2954,9 @@ __global__ void __launch_bounds__(256) k_bmr_alfa(const int64_t* __restrict__ lo
 }
 
 // y -= c_r2 r2; its displacement rows (r < Nu; Nu = 0: none) also in the padded layout that the
-// preconditioner's first level takes, zeros there for a converged instance
+// preconditioner's first level takes.  The preconditioner's input of a converged instance is zero:
+// products in slices that it shares with an open one go on computing its rows, and z, the next
+// iteration's y, would grow through them until 0 * inf in a padded entry reached open instances.
 template <typename T>
 __global__ void __launch_bounds__(256) k_bmr_axpy(const int64_t* __restrict__ lo, const int32_t* __restrict__ len,
                                                   const int32_t* __restrict__ inst, T* y, const T* __restrict__ r2,
@@ -2968,11 +2970,8 @@ __global__ void __launch_bounds__(256) k_bmr_axpy(const int64_t* __restrict__ lo
     const T c2 = msc<T>(sc[in].c_r2, sc[in].f_c_r2);
     for (int i = threadIdx.x; i < len[ch]; i += 256) {
         const int64_t r = lo[ch] + i;
-        T yy = T(0);
-        if (open) {
-            yy = y[r] - c2 * r2[r];
-            y[r] = yy;
-        }
+        const T yy = open ? y[r] - c2 * r2[r] : T(0);
+        if (open || r >= Nu) y[r] = yy;
         if (r < Nu) {
             const int64_t node = r / 3;
             packed[4 * (perm ? perm[node] : node) + (r - 3 * node)] = yy;
