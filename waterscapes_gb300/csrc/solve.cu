@@ -1636,7 +1636,11 @@ static void autotune_matrix(mpet_ctx* c, Csr& A, const T* x, const Epi& epi, dou
             // median; a variant replaces the incumbent only when clearly faster,
             // so near-ties do not flip from one set-up to the next
             const float med = t[3];
-            const float ms = med * ((v == 0 && lpr == lpr0) ? 0.97f : 1.0f);
+            // Row tiles of a large matrix win ties within 4%: from a flushed L2 they tie with SELL
+            // between 250,000 and 400,000 rows, but the products of a cycle follow one another, and
+            // of the tiles' smaller copy more is still in L2 (24 cubes of 6^3..16^3: 335 us per
+            // iteration with SELL, 307 with tiles; 32^3, A=4: 375 and 357).
+            const float ms = med * ((v == 0 && lpr == lpr0) ? 0.97f : v == 64 && flush ? 0.94f : 1.0f);
             // (slot 6: the faster node-block kernel)
             if (ms_out && lpr == lpr0 && (v <= 5 || v == 8)) ms_out[v == 8 ? 6 : v] = med;
             if (ms_out && lpr == lpr0 && v == 9 && (ms_out[6] <= 0.0 || med < ms_out[6])) ms_out[6] = med;
