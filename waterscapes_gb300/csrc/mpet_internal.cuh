@@ -478,6 +478,7 @@ struct mpet_ctx {
     // error-indicator scratch: per-facet terms, per-cell R4p density, its sum, bad-index flag
     double* est_fval = nullptr;
     int64_t est_fval_cap = 0;
+    double* est_h = nullptr;      // cell diameters
     double* est_r4 = nullptr;
     double* est_sum = nullptr;
     int32_t* est_bad = nullptr;
