@@ -1259,7 +1259,6 @@ static void launch_nb(mpet_ctx* c, const NodeBlocks& nb, const T* x, const Epi& 
         blocks = wave;
     }
     const int J = c->J;
-    cudaStream_t st = c->stream;
     const T* v = nb_vals<T>(nb);
     const int32_t* skl = c->skip_done ? nb.skl : nullptr;
     if (occ && sizeof(T) == 4) {
@@ -1309,7 +1308,6 @@ bool rhs_div_from_matrix(mpet_ctx* c, const double* up_prev, double* b) {
     int blocks = grid_for(nb.nsp * 32, 256);
     if (blocks > 152 * 16) blocks = 152 * 16;
     const int J = c->J;
-    cudaStream_t st = c->stream;
     if (J <= 2)
         launch_k(c, k_spmv_nb<double, 2, EpiAddRhs, false, false, true>, blocks, 256, 0, 
             c->nnodes, c->nv, c->Nu, J, nb.nsu, ns, nb.sl, nb.perm, nb.cols, nb.v64, up_prev, EpiAddRhs{b},
@@ -1441,7 +1439,6 @@ static void launch_spmv(mpet_ctx* c, const Csr& A, const T* va, const T* x, cons
         if (blocks > 152 * 16) blocks = 152 * 16;
     }
     double* part = c->partials;
-    cudaStream_t s = c->stream;
     switch (lpr) {
         case 32:
             if (deep) launch_k(c, k_spmv<T, NV, 32, 8, Epi>, blocks, 256, 0, A.n, A.rp, A.ci, va, x, epi, part, skl, skip);
