@@ -4231,105 +4231,118 @@ double device_rho(mpet_ctx* c, const Csr& A, const double* dinv) { return csr_rh
 // reached by the P1-in-P2 embedding of each component; below it smoothed
 // aggregation with the six rigid-body modes (amg_setup_block_host).
 
+// Lanczos on D^-1/2 A D^-1/2 with its scalars on the device (sc: the norms beta_0.. at sc[k], alpha_k
+// at sc[32 + k]); a step is the product and three kernels.  With both dot products of a step read
+// back by the host a radius took 1.8 ms on a level of a few thousand rows, nearly all of it waits
+// (12.8 ms of two rebuilds of the pressure hierarchies at 16^3, A=2).
 __global__ void k_lz_init(int64_t n, const double* __restrict__ dinv, const uint8_t* __restrict__ bc, double* s,
-                          double* v) {
+                          double* w, double* v) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
     s[i] = dinv[i] > 0.0 ? sqrt(dinv[i]) : 0.0;
-    v[i] = (bc && bc[i]) ? 0.0 : 0.5 + (double)((7919LL * i) % 1009LL) / 1009.0;
+    w[i] = (bc && bc[i]) ? 0.0 : 0.5 + (double)((7919LL * i) % 1009LL) / 1009.0;
+    v[i] = 0.0;
 }
+// w = s t - beta vprev, alpha = w . v
 template <typename T>
-__global__ void k_lz_mul(int64_t n, const double* __restrict__ s, const double* __restrict__ v, T* w) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i < n) w[i] = (T)(s[i] * v[i]);
+__global__ void __launch_bounds__(256) k_lz_alpha(int64_t n, const double* __restrict__ s, const T* __restrict__ t,
+                                                  const double* __restrict__ vprev, const double* __restrict__ v,
+                                                  double* w, const double* beta, double* partials, unsigned* cnt,
+                                                  double* alpha) {
+    __shared__ double sh[8];
+    const double b = *beta;
+    double acc = 0.0;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const double x = s[i] * (double)t[i] - b * vprev[i];
+        w[i] = x;
+        acc += x * v[i];
+    }
+    acc = block_sum256(acc, sh);
+    if (threadIdx.x == 0) partials[blockIdx.x] = acc;
+    if (!last_block(cnt)) return;
+    acc = sum_partials_n(partials, gridDim.x, sh);
+    if (threadIdx.x == 0) *alpha = acc;
 }
+// w -= alpha v (alpha null: 0), beta = |w|
+__global__ void __launch_bounds__(256) k_lz_beta(int64_t n, const double* __restrict__ v, double* w,
+                                                 const double* alpha, double* partials, unsigned* cnt, double* beta) {
+    __shared__ double sh[8];
+    const double a = alpha ? *alpha : 0.0;
+    double acc = 0.0;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const double x = w[i] - a * v[i];
+        w[i] = x;
+        acc += x * x;
+    }
+    acc = block_sum256(acc, sh);
+    if (threadIdx.x == 0) partials[blockIdx.x] = acc;
+    if (!last_block(cnt)) return;
+    acc = sum_partials_n(partials, gridDim.x, sh);
+    if (threadIdx.x == 0) *beta = sqrt(acc);
+}
+// vprev = v, v = w / beta, xin = s v
 template <typename T>
-__global__ void k_lz_w(int64_t n, const double* __restrict__ s, const T* __restrict__ t, double beta,
-                       const double* __restrict__ vprev, double* w) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i < n) w[i] = s[i] * (double)t[i] - beta * vprev[i];
-}
-__global__ void k_lz_axpy(int64_t n, double* w, double a, const double* __restrict__ v) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i < n) w[i] += a * v[i];
-}
-__global__ void k_lz_next(int64_t n, const double* __restrict__ w, double ib, double* vprev, double* v) {
+__global__ void k_lz_next(int64_t n, const double* __restrict__ w, const double* __restrict__ s, const double* beta,
+                          double* vprev, double* v, T* xin) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
+    const double x = w[i] * (1.0 / *beta);
     vprev[i] = v[i];
-    v[i] = w[i] * ib;
+    v[i] = x;
+    xin[i] = (T)(s[i] * x);
 }
 
-// Spectral radius of D^-1 A_uu: 30 Lanczos steps on D^-1/2 A_uu D^-1/2 from the fixed
-// start vector of the host setup with the Dirichlet rows zeroed (the iterates stay
+// Largest Ritz value of 30 steps from the fixed start vector of the host set-up, rows of bc zeroed;
+// product(xin, t): t = A xin.  A step whose beta vanishes ends the recurrence: the host drops what
+// the later steps computed from it.
+template <typename T, class Product>
+static double device_lanczos(mpet_ctx* c, int64_t n, const double* dinv, const uint8_t* bc, Product product) {
+    constexpr int STEPS = 30;
+    const int64_t pad = (n + 31) & ~(int64_t)31;
+    TmpBuf buf(sizeof(double) * (6 * pad + 64));
+    double *s = buf.as<double>(), *v = s + pad, *vp = v + pad, *w = vp + pad, *sc = w + 3 * pad;
+    T *t = (T*)(w + pad), *xin = (T*)(w + 2 * pad);
+    const int G = grid_for(n, 256);
+    const int Gd = (int)std::min<int64_t>(NB_RED, std::max<int64_t>(std::min<int64_t>(G, 304), grid_for(n, 4096)));
+    const int steps = n < STEPS ? (int)n : STEPS;
+    k_lz_init<<<G, 256, 0, c->stream>>>(n, dinv, bc, s, w, v);
+    k_lz_beta<<<Gd, 256, 0, c->stream>>>(n, v, w, nullptr, c->partials, c->red_cnt, sc);
+    k_lz_next<T><<<G, 256, 0, c->stream>>>(n, w, s, sc, vp, v, xin);
+    MPET_CHECK_LAUNCH();
+    for (int k = 0; k < steps; ++k) {
+        product(xin, t);
+        k_lz_alpha<T><<<Gd, 256, 0, c->stream>>>(n, s, t, vp, v, w, sc + k, c->partials, c->red_cnt, sc + 32 + k);
+        k_lz_beta<<<Gd, 256, 0, c->stream>>>(n, v, w, sc + 32 + k, c->partials, c->red_cnt, sc + k + 1);
+        if (k + 1 < steps) k_lz_next<T><<<G, 256, 0, c->stream>>>(n, w, s, sc + k + 1, vp, v, xin);
+        MPET_CHECK_LAUNCH();
+    }
+    double h[64];
+    MPET_CUDA(cudaMemcpyAsync(h, sc, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
+    MPET_CUDA(cudaStreamSynchronize(c->stream));
+    if (!(h[0] > 0.0)) return 1.0;
+    std::vector<double> al, be(1, 0.0);
+    for (int k = 0; k < steps; ++k) {
+        al.push_back(h[32 + k]);
+        if (h[k + 1] <= 1e-14 * fabs(h[32 + k]) || k + 1 == steps) break;
+        be.push_back(h[k + 1]);
+    }
+    return tridiag_max_eig_host(al, be);
+}
+
+// Spectral radius of D^-1 A_uu, the Dirichlet rows zeroed in the start vector (the iterates stay
 // where the row-replaced block acts symmetrically).
 template <typename T>
 static double nb_uu_rho(mpet_ctx* c, const double* dinv) {
-    const int64_t n = c->Nu;
-    TmpBuf bs(sizeof(double) * n), bv(sizeof(double) * n), bp(sizeof(double) * n), bw(sizeof(double) * n),
-        bt(sizeof(double) * n);
-    double *s = bs.as<double>(), *v = bv.as<double>(), *vp = bp.as<double>(), *w = bw.as<double>();
-    T* t = bt.as<T>();
-    const int G = grid_for(n, 256);
-    k_lz_init<<<G, 256, 0, c->stream>>>(n, dinv, c->dof_bc, s, v);
-    MPET_CUDA(cudaMemsetAsync(vp, 0, sizeof(double) * n, c->stream));
-    MPET_CHECK_LAUNCH();
-    double nrm = sqrt(dot_host(c, v, v, n));
-    if (!(nrm > 0.0)) return 1.0;
-    k_lz_next<<<G, 256, 0, c->stream>>>(n, v, 1.0 / nrm, w, v);  // v /= |v| (w scratch)
-    MPET_CUDA(cudaMemsetAsync(vp, 0, sizeof(double) * n, c->stream));
-    std::vector<double> al, be(1, 0.0);
-    double beta = 0.0;
-    TmpBuf bx(sizeof(double) * n);
-    T* xin = bx.as<T>();
-    for (int k = 0; k < 30; ++k) {
-        k_lz_mul<T><<<G, 256, 0, c->stream>>>(n, s, v, xin);
-        launch_nb_uu<T>(c, *c->A.nb, xin, EpiStore<T, 1>{t});
-        k_lz_w<T><<<G, 256, 0, c->stream>>>(n, s, t, beta, vp, w);
-        MPET_CHECK_LAUNCH();
-        const double alpha = dot_host(c, w, v, n);
-        al.push_back(alpha);
-        k_lz_axpy<<<G, 256, 0, c->stream>>>(n, w, -alpha, v);
-        beta = sqrt(dot_host(c, w, w, n));
-        if (beta <= 1e-14 * fabs(alpha) || k + 1 == 30) break;
-        be.push_back(beta);
-        k_lz_next<<<G, 256, 0, c->stream>>>(n, w, 1.0 / beta, vp, v);
-    }
-    return tridiag_max_eig_host(al, be);
+    return device_lanczos<T>(c, c->Nu, dinv, c->dof_bc,
+                             [c](const T* x, T* t) { launch_nb_uu<T>(c, *c->A.nb, x, EpiStore<T, 1>{t}); });
 }
 
 // Spectral radius of D^-1 A for a CSR level on the device (FP64 values): the host
-// set-up's Lanczos iteration (lanczos_rho, amg_setup.cpp) with the same start vector,
-// 30 steps on D^-1/2 A D^-1/2, largest Ritz value.
+// set-up's Lanczos iteration (lanczos_rho, amg_setup.cpp) with the same start vector.
 static double csr_rho(mpet_ctx* c, const Csr& A, const double* dinv) {
-    const int64_t n = A.n;
-    TmpBuf bs(sizeof(double) * n), bv(sizeof(double) * n), bp(sizeof(double) * n), bw(sizeof(double) * n),
-        bt(sizeof(double) * n), bx(sizeof(double) * n);
-    double *s = bs.as<double>(), *v = bv.as<double>(), *vp = bp.as<double>(), *w = bw.as<double>();
-    double *t = bt.as<double>(), *xin = bx.as<double>();
-    const int G = grid_for(n, 256);
-    k_lz_init<<<G, 256, 0, c->stream>>>(n, dinv, nullptr, s, v);
-    MPET_CHECK_LAUNCH();
-    double nrm = sqrt(dot_host(c, v, v, n));
-    if (!(nrm > 0.0)) return 1.0;
-    k_lz_next<<<G, 256, 0, c->stream>>>(n, v, 1.0 / nrm, w, v);  // v /= |v| (w scratch)
-    MPET_CUDA(cudaMemsetAsync(vp, 0, sizeof(double) * n, c->stream));
-    std::vector<double> al, be(1, 0.0);
-    double beta = 0.0;
-    for (int k = 0; k < 30 && k < n; ++k) {
-        k_lz_mul<double><<<G, 256, 0, c->stream>>>(n, s, v, xin);
-        launch_spmv<double, 1>(c, A, A.v64, xin, EpiStore<double, 1>{t});
-        k_lz_w<double><<<G, 256, 0, c->stream>>>(n, s, t, beta, vp, w);
-        MPET_CHECK_LAUNCH();
-        const double alpha = dot_host(c, w, v, n);
-        al.push_back(alpha);
-        k_lz_axpy<<<G, 256, 0, c->stream>>>(n, w, -alpha, v);
-        beta = sqrt(dot_host(c, w, w, n));
-        if (beta <= 1e-14 * fabs(alpha) || k + 1 == 30 || k + 1 == n) break;
-        be.push_back(beta);
-        k_lz_next<<<G, 256, 0, c->stream>>>(n, w, 1.0 / beta, vp, v);
-    }
-    return tridiag_max_eig_host(al, be);
+    return device_lanczos<double>(c, A.n, dinv, nullptr, [c, &A](const double* x, double* t) {
+        launch_spmv<double, 1>(c, A, A.v64, x, EpiStore<double, 1>{t});
+    });
 }
 
 bool setup_u_elasticity(mpet_ctx* c, bool fp32) {
