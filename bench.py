@@ -182,6 +182,23 @@ def time_spmv(solver, torch, lib, reps=20):
     return out
 
 
+def time_inner_product(solver, torch, lib, reps=20):
+    """The FP32 product of the inner iterations (from the elements, or the stored matrix)."""
+    import ctypes
+    x = torch.randn(solver.N, dtype=torch.float32, device=solver.device)
+    y = torch.empty_like(x)
+    elements = ctypes.c_int32()
+    e0, e1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+    for k in range(reps + 3):
+        if k == 3:
+            torch.cuda.synchronize()
+            e0.record(solver._stream)
+        solver.ctx.call("mpet_krylov_product", lib._ptr(x), lib._ptr(y), ctypes.byref(elements))
+    e1.record(solver._stream)
+    torch.cuda.synchronize()
+    return {"ms": e0.elapsed_time(e1) / reps, "from": "elements" if elements.value else "stored matrix"}
+
+
 def run_steps(solver, torch, steps, warmup, dt):
     """solve_direct steps with the state on the device; returns (ms total, iterations, states)."""
     problem = solver.problem
@@ -871,6 +888,7 @@ def main():
     torch.cuda.synchronize()
     asm_ms = e0.elapsed_time(e1)
     spmv = time_spmv(sol, torch, lib)
+    inner_product = time_inner_product(sol, torch, lib) if sol.params["precision"] == "mixed" else None
     precond_ms = time_precond(sol, torch, lib)
 
     clk = ClockSampler(local_rank)
@@ -987,12 +1005,13 @@ def main():
         "preconditioner_u_block": prec_form(sol),
         "preconditioner_level_variants": level_variants(sol),
         "iteration_breakdown_ms": dict(split, spmv_fp32=(spmv.get("fp32") or spmv["fp64"])["ms"],
-                                       preconditioner=precond_ms),
+                                       inner_product=inner_product, preconditioner=precond_ms),
         "fp64_iteration_breakdown_ms": res.get("fp64", {}).get("iteration_breakdown_ms"),
         "roofline": {"kernel": ROOFLINE_KERNEL[sp32["layout"]] + (" FP32" if "fp32" in spmv else " FP64")
                      + (", 64-register kernel" if tuning.get("chosen") == "node-block/64 registers" else ""),
                      "bound": "hbm", "achieved": sp32["gbs"], "peak": hbm, "unit": "GB/s",
                      "frac": sp32["gbs"] / hbm, "peak_kind": peak_kind,
+                     "note": "the product with the stored matrix; see inner_product for the inner iterations'",
                      "alg_bytes_per_launch": sp32["alg_bytes"],
                      "traffic": (sp32["alg_bytes"] * TRAFFIC_RATIO[sp32["layout"]]
                                  if sp32["layout"] in TRAFFIC_RATIO else None),
