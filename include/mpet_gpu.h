@@ -179,8 +179,12 @@ int mpet_get_edges(mpet_ctx* ctx, int64_t* edges_host);
 
 /* Matrix assembly: assemble(self.a) + Robin axpy + bc.apply(A)
  * (mpetsolver.py:335-344 / 412-419).  apply_bc != 0 replaces Dirichlet
- * rows by unit rows (DirichletBC.apply).  In mixed precision an FP32 copy
- * of the values is written in the same pass. */
+ * rows by unit rows (DirichletBC.apply).  Products read copies of the values
+ * in layouts of their own (FP32 in mixed precision): those that earlier
+ * products have read are written before this call returns, any other one
+ * before the first product that reads it is issued.  A product captured in a
+ * CUDA graph therefore runs on the values of the last mpet_assemble (or
+ * mpet_apply_symmetric) before each replay. */
 int mpet_assemble(mpet_ctx* ctx, double dt, int32_t apply_bc);
 int mpet_get_values(mpet_ctx* ctx, double* values_host);
 

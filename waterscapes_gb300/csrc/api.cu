@@ -224,9 +224,10 @@ int mpet_setup(mpet_ctx* c, const mpet_params* p) {
         MPET_CUDA(cudaMemsetAsync(c->A.v32, 0, sizeof(float) * c->nnz, c->stream));
     }
     if (!mixed || c->A.v32) build_sell(c, c->A, c->A.v32 != nullptr, true);
-    c->stale = COPY_ALL;
-    need_copies(c, COPY_ALL);
+    c->used = COPY_ALL;  // (for the autotuner)
+    values_changed(c);
     autotune_system(c);
+    c->used = 0;
     MPET_CUDA(cudaStreamSynchronize(c->stream));
     c->setup_done = true;
     API_END(c)
@@ -282,14 +283,14 @@ int mpet_assemble(mpet_ctx* c, double dt, int32_t apply_bc) {
     API_BEGIN(c)
     require(c->setup_done, MPET_ERR_STATE, "mpet_setup must come first");
     require(dt > 0.0, MPET_ERR_INVALID, "dt must be positive");
+    c->stale = COPY_ALL;
     launch_assemble_matrix(c, dt, apply_bc != 0);
     launch_robin_matrix(c, dt);
-    c->stale = COPY_ALL;
     // (the patches come with the preconditioner: a program that only assembles does without)
     if (c->sys_patch_mode == 1) build_patches(c);
     set_patch_coefficients(c, dt, apply_bc != 0);
     c->asm_bc = apply_bc != 0;
-    MPET_CUDA(cudaStreamSynchronize(c->stream));
+    values_changed(c);
     c->assembled = true;
     c->bc_cols_zeroed = false;
     c->q_dirty = true;
@@ -903,10 +904,10 @@ int mpet_krylov_product(mpet_ctx* c, const float* x, float* y, int32_t* elements
 int mpet_apply_symmetric(mpet_ctx* c, double* b, const double* xbc) {
     API_BEGIN(c)
     require(c->assembled, MPET_ERR_STATE, "mpet_assemble must come first");
+    c->stale = COPY_ALL;
     launch_zero_bc_columns(c, b, xbc);
     c->bc_cols_zeroed = true;
-    c->stale = COPY_ALL;
-    MPET_CUDA(cudaStreamSynchronize(c->stream));
+    values_changed(c);
     API_END(c)
 }
 

@@ -361,6 +361,7 @@ struct mpet_ctx {
     mpet::Csr A;                  // rp/ci/v64/v32
     mpet::NodeBlocks A_nb;        // node-block copy of A
     unsigned stale = 0;           // copies of A that do not hold its values yet (COPY_*)
+    unsigned used = 0;            // copies that products have read since the set-up
     int asm_rows[2] = {0, 0};     // most entries of a vertex's / an edge node's rows
     double* dinv = nullptr;       // |diag|^-1 (1 where 0), FP64
 
@@ -712,14 +713,17 @@ void build_tiles(mpet_ctx* c, Csr& A, const int64_t* rp_host);
 void build_sell(mpet_ctx* c, Csr& A, bool fp32, bool with64);
 // the FP16 SELL values of A (after build_sell; needs A.v64)
 void build_sell_half(mpet_ctx* c, Csr& A);
-void fill_sell(mpet_ctx* c, Csr& A, bool f32, bool f64);
+void fill_sell(Csr& A, bool f32, bool f64, cudaStream_t st);
 void build_node_blocks(mpet_ctx* c);
 bool device_fits(mpet_ctx* c, size_t bytes);
-// the system matrix's copies are filled from A.v64 when a product needs them: after a change of
-// the values all are stale; need_system_copy<T> fills the one that the tuned products in T read,
-// need_copies any set of them
+// The system matrix's copies are filled from A.v64 for the products that read them.  A copy is
+// filled, and the fill waited for, before the first product that reads it (need_copies;
+// need_system_copy<T>: the copy of the tuned products in T), and from then on with every change of
+// the values (values_changed): a product may have been captured in a caller's graph or may be
+// issued on another stream, and finds the values of the last mpet_assemble all the same.
 enum { COPY_CSR32 = 1, COPY_SELL32 = 2, COPY_SELL64 = 4, COPY_NB32 = 8, COPY_NB64 = 16, COPY_ALL = 31 };
 void need_copies(mpet_ctx* c, unsigned which);
+void values_changed(mpet_ctx* c);
 template <typename T>
 void need_system_copy(mpet_ctx* c);
 // y = A x (FP32) as the inner Krylov iterations form it

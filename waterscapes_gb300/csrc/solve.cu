@@ -1108,24 +1108,26 @@ void build_sell(mpet_ctx* c, Csr& A, bool fp32, bool with64) {
     if (fp32) A.s_v32 = c->pool.alloc<float>(acc);
     if (!fp32 || with64) A.s_v64 = c->pool.alloc<double>(acc);
     MPET_CUDA(cudaStreamSynchronize(c->stream));
-    fill_sell(c, A, true, true);
+    fill_sell(A, true, true, c->stream);
 }
 
 // the values of the SELL copies from A.v64, the columns with the first fill
-void fill_sell(mpet_ctx* c, Csr& A, bool f32, bool f64) {
+void fill_sell(Csr& A, bool f32, bool f64, cudaStream_t st) {
     if (!A.s_off) return;
     const int64_t ns = A.nslices;
-    auto cols = [&] {
-        int32_t* p = A.s_cols ? nullptr : A.s_ci;
-        A.s_cols = true;
-        return p;
-    };
     const int G = grid_for(ns * 32, 256);
-    if (f32 && A.s_v32)
-        k_sell_fill<float, double><<<G, 256, 0, c->stream>>>(A.n, ns, A.rp, A.ci, A.v64, A.s_off, cols(), A.s_v32);
-    if (f64 && A.s_v64)
-        k_sell_fill<double, double><<<G, 256, 0, c->stream>>>(A.n, ns, A.rp, A.ci, A.v64, A.s_off, cols(), A.s_v64);
-    MPET_CHECK_LAUNCH();
+    if (f32 && A.s_v32) {
+        k_sell_fill<float, double><<<G, 256, 0, st>>>(A.n, ns, A.rp, A.ci, A.v64, A.s_off, A.s_cols ? nullptr : A.s_ci,
+                                                      A.s_v32);
+        MPET_CHECK_LAUNCH();
+        A.s_cols = true;
+    }
+    if (f64 && A.s_v64) {
+        k_sell_fill<double, double><<<G, 256, 0, st>>>(A.n, ns, A.rp, A.ci, A.v64, A.s_off,
+                                                       A.s_cols ? nullptr : A.s_ci, A.s_v64);
+        MPET_CHECK_LAUNCH();
+        A.s_cols = true;
+    }
 }
 
 // Node-block layout of the system matrix: slice widths from the node and
@@ -1194,40 +1196,63 @@ void build_node_blocks(mpet_ctx* c) {
 }
 
 // the values of the node-block copies from A.v64, the columns with the first fill
-static void fill_node_blocks(mpet_ctx* c, bool f32, bool f64) {
+static void fill_node_blocks(mpet_ctx* c, bool f32, bool f64, cudaStream_t st) {
     NodeBlocks& nb = c->A_nb;
     if (!nb.sl) return;
     const int64_t ns = nb.nsu + nb.nsp;
     const int G = grid_for(ns * 32, 128);
     if (f32 && nb.v32) {
-        k_nb_fill<float, double><<<G, 128, 0, c->stream>>>(c->nnodes, c->nv, c->Nu, c->J, nb.nsu, ns, nb.sl, nb.perm,
+        k_nb_fill<float, double><<<G, 128, 0, st>>>(c->nnodes, c->nv, c->Nu, c->J, nb.nsu, ns, nb.sl, nb.perm,
                                                            c->A.rp, c->A.v64, c->n2_ptr, c->n2_col, c->n1_ptr,
                                                            c->n1_col, nb.cols, nb.v32, nb.have_cols ? 0 : 1);
+        MPET_CHECK_LAUNCH();
         nb.have_cols = true;
     }
     if (f64 && nb.v64) {
-        k_nb_fill<double, double><<<G, 128, 0, c->stream>>>(c->nnodes, c->nv, c->Nu, c->J, nb.nsu, ns, nb.sl, nb.perm,
+        k_nb_fill<double, double><<<G, 128, 0, st>>>(c->nnodes, c->nv, c->Nu, c->J, nb.nsu, ns, nb.sl, nb.perm,
                                                             c->A.rp, c->A.v64, c->n2_ptr, c->n2_col, c->n1_ptr,
                                                             c->n1_col, nb.cols, nb.v64, nb.have_cols ? 0 : 1);
+        MPET_CHECK_LAUNCH();
         nb.have_cols = true;
     }
-    MPET_CHECK_LAUNCH();
 }
 
 __global__ void k_f64_to_f32(int64_t n, const double* __restrict__ a, float* b);
 
-void need_copies(mpet_ctx* c, unsigned which) {
-    which &= c->stale;
-    if (!which) return;
-    c->stale &= ~which;
+static void fill_copies(mpet_ctx* c, unsigned which, cudaStream_t st) {
     if ((which & COPY_CSR32) && c->A.v32) {
-        k_f64_to_f32<<<grid_for(c->nnz, 256), 256, 0, c->stream>>>(c->nnz, c->A.v64, c->A.v32);
+        k_f64_to_f32<<<grid_for(c->nnz, 256), 256, 0, st>>>(c->nnz, c->A.v64, c->A.v32);
         MPET_CHECK_LAUNCH();
     }
     if (which & (COPY_SELL32 | COPY_SELL64))
-        fill_sell(c, c->A, (which & COPY_SELL32) != 0, (which & COPY_SELL64) != 0);
+        fill_sell(c->A, (which & COPY_SELL32) != 0, (which & COPY_SELL64) != 0, st);
     if (which & (COPY_NB32 | COPY_NB64))
-        fill_node_blocks(c, (which & COPY_NB32) != 0, (which & COPY_NB64) != 0);
+        fill_node_blocks(c, (which & COPY_NB32) != 0, (which & COPY_NB64) != 0, st);
+}
+
+void values_changed(mpet_ctx* c) {
+    c->stale = COPY_ALL;
+    fill_copies(c, c->used, c->stream);
+    MPET_CUDA(cudaStreamSynchronize(c->stream));
+    c->stale &= ~c->used;
+}
+
+void need_copies(mpet_ctx* c, unsigned which) {
+    c->used |= which;
+    which &= c->stale;
+    if (!which) return;
+    // The values are finished (every change of them ends with a wait), so the fill needs no order
+    // with c->stream: it runs on the context's own stream, is never captured with a caller's graph and
+    // is over before the product that reads the copy is issued on whatever stream.
+    struct RelaxedCapture {
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        RelaxedCapture() { MPET_CUDA(cudaThreadExchangeStreamCaptureMode(&mode)); }
+        ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    } relaxed;
+    if (!c->cap_stream) MPET_CUDA(cudaStreamCreateWithFlags(&c->cap_stream, cudaStreamNonBlocking));
+    fill_copies(c, which, c->cap_stream);
+    MPET_CUDA(cudaStreamSynchronize(c->cap_stream));
+    c->stale &= ~which;
 }
 
 template <typename T>
