@@ -288,8 +288,8 @@ int mpet_assemble(mpet_ctx* c, double dt, int32_t apply_bc) {
     launch_robin_matrix(c, dt);
     // (the patches come with the preconditioner: a program that only assembles does without)
     if (c->sys_patch_mode == 1) build_patches(c);
-    set_patch_coefficients(c, dt, apply_bc != 0);
-    c->asm_bc = apply_bc != 0;
+    take_patch_coefficients(c, dt, apply_bc != 0);
+    use_patches(c);
     values_changed(c);
     c->assembled = true;
     c->bc_cols_zeroed = false;
@@ -557,7 +557,7 @@ int mpet_setup_preconditioner(mpet_ctx* c, double dt) {
     destroy_minres_graph(c);
     if (!c->patch.tried && c->sys_patch_mode != 0) {
         build_patches(c);
-        if (c->assembled) set_patch_coefficients(c, c->asm_dt, c->asm_bc);
+        if (c->assembled) use_patches(c);  // with the coefficients of that assembly
     }
     using clk = std::chrono::steady_clock;
     auto since = [](clk::time_point t) { return std::chrono::duration<double, std::milli>(clk::now() - t).count(); };

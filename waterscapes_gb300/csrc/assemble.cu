@@ -925,65 +925,99 @@ void launch_patch_geometry(mpet_ctx* c) {
     MPET_CHECK_LAUNCH();
 }
 
-__global__ void k_patch_coef(int64_t nslots, int P, const int32_t* __restrict__ cell, int ncell, MatCoef C,
-                             float* out) {
-    const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (s >= nslots) return;
-    const int64_t p = s / P;
-    const int l = (int)(s % P);
-    const int32_t c = cell[s];
+// per-cell coefficients of the assembled matrix, ncell planes of nc
+__global__ void k_cell_coef(int64_t nc, int ncell, MatCoef C, float* out) {
+    const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (c >= nc) return;
     const int J = C.J;
     for (int q = 0; q < ncell; ++q) {
-        double v = 0.0;
-        if (c >= 0 && q < J) {
+        double v;
+        if (q < J) {
             v = -C.dt_theta * C.Kof(q, c);
-        } else if (c >= 0) {
+        } else {
             const int a = (q - J) / J, b = (q - J) % J;
             v = -(C.dt_theta * ((a == b ? C.Ssumof(a, c) : 0.0) - C.Sof(a, b, c)) +
                   C.rank_inv * C.rank_b[a] * C.rank_b[b]) -
                 (a == b ? C.cof(a, c) : 0.0);
         }
-        out[(p * ncell + q) * P + l] = (float)v;
+        out[q * nc + c] = (float)v;
     }
 }
 
-void set_patch_coefficients(mpet_ctx* c, double dt, bool apply_bc) {
-    PatchSet& s = c->patch;
+// ... in the slots of the patches (padding: zeros)
+__global__ void k_patch_coef(int64_t nslots, int P, const int32_t* __restrict__ cell, int ncell, int64_t nc,
+                             const float* __restrict__ in, float* out) {
+    const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (s >= nslots) return;
+    const int64_t p = s / P;
+    const int l = (int)(s % P);
+    const int32_t c = cell[s];
+    for (int q = 0; q < ncell; ++q) out[(p * ncell + q) * P + l] = c >= 0 ? in[q * nc + c] : 0.f;
+}
+
+// From 3e6 entries on: the two kernels of an element product take about 13 us however
+// small the mesh, the stored product 4.5 us at 0.2e6 entries (4^3 cube, A=2), 7.4 at 1.6e6
+// (8^3; a whole iteration 72 us stored, 77 by elements), 14.7 at 5.3e6 (12^3; 121 and 112)
+// and 769 against 195 at 1.03e9 (64^3, A=4).
+static bool wants_patches(const mpet_ctx* c) {
+    return c->dim == 3 && c->prm.precision == MPET_PRECISION_MIXED &&
+           (c->sys_patch_mode == 1 || (c->sys_patch_mode < 0 && c->nnz >= 3000000));
+}
+
+void take_patch_coefficients(mpet_ctx* c, double dt, bool apply_bc) {
+    c->asm_coef = PatchCoef{};
+    c->asm_taken = false;
+    if (!wants_patches(c) || (c->patch.tried && !c->patch.ready())) return;
     const MatCoef C = make_coef(c, dt);
     const int J = c->J;
-    PatchCoef q{};
-    // From 3e6 entries on: the two kernels of an element product take about 13 us however
-    // small the mesh, the stored product 4.5 us at 0.2e6 entries (4^3 cube, A=2), 7.4 at 1.6e6
-    // (8^3; a whole iteration 72 us stored, 77 by elements), 14.7 at 5.3e6 (12^3; 121 and 112)
-    // and 769 against 195 at 1.03e9 (64^3, A=4).
-    bool use = s.ready() && (c->sys_patch_mode == 1 || (c->sys_patch_mode < 0 && c->nnz >= 3000000));
+    PatchCoef& q = c->asm_coef;
+    q.mu = (float)C.mu;
+    q.lam = (float)C.lmbda;
+    for (int a = 0; a < J; ++a) {
+        q.cpl[a] = (float)C.cpl[a];
+        q.Kd[a] = (float)C.Kd[a];
+        for (int b = 0; b < J; ++b) q.Cm[a * MPET_MAX_NETWORKS + b] = (float)C.Cm[a * MPET_MAX_NETWORKS + b];
+    }
+    q.bc = apply_bc ? 1 : 0;
+    q.robin = launch_robin_entries(c, dt) ? 1 : 0;
+    q.ncell = C.coef_const ? 0 : (C.cc || C.Sc ? J + J * J : J);
+    if (q.ncell > 0) {
+        const int64_t need = c->nc * q.ncell;
+        if (need > c->asm_ncell) {
+            if (!device_fits(c, (size_t)need * sizeof(float))) return;
+            c->pool.release(c->asm_cell);
+            c->asm_cell = nullptr;
+            c->asm_ncell = 0;
+            c->asm_cell = c->pool.alloc<float>(need);
+            c->asm_ncell = need;
+        }
+        k_cell_coef<<<grid_for(c->nc, 256), 256, 0, c->stream>>>(c->nc, q.ncell, C, c->asm_cell);
+        MPET_CHECK_LAUNCH();
+    }
+    c->asm_taken = true;
+}
+
+void use_patches(mpet_ctx* c) {
+    PatchSet& s = c->patch;
+    bool use = s.ready() && c->asm_taken && wants_patches(c);
     float* const coef0 = s.coef;
-    if (use) {
-        q.mu = (float)C.mu;
-        q.lam = (float)C.lmbda;
-        for (int a = 0; a < J; ++a) {
-            q.cpl[a] = (float)C.cpl[a];
-            q.Kd[a] = (float)C.Kd[a];
-            for (int b = 0; b < J; ++b)
-                q.Cm[a * MPET_MAX_NETWORKS + b] = (float)C.Cm[a * MPET_MAX_NETWORKS + b];
+    const int64_t need = s.np * s.P * c->asm_coef.ncell;
+    if (use && need > s.ncoef) {
+        if (device_fits(c, (size_t)need * sizeof(float))) {
+            c->pool.release(s.coef);
+            s.coef = nullptr;
+            s.ncoef = 0;
+            s.coef = c->pool.alloc<float>(need);
+            s.ncoef = need;
+        } else {
+            use = false;
         }
-        q.bc = apply_bc ? 1 : 0;
-        q.robin = launch_robin_entries(c, dt) ? 1 : 0;
-        q.ncell = C.coef_const ? 0 : (C.cc || C.Sc ? J + J * J : J);
-        const int64_t need = s.np * s.P * q.ncell;
-        if (need > s.ncoef) {
-            if (device_fits(c, (size_t)need * sizeof(float))) {
-                c->pool.release(s.coef);
-                s.coef = c->pool.alloc<float>(need);
-                s.ncoef = need;
-            } else {
-                use = false;
-            }
-        }
-        if (use && q.ncell > 0) {
-            k_patch_coef<<<grid_for(s.np * s.P, 256), 256, 0, c->stream>>>(s.np * s.P, s.P, s.cell, q.ncell, C, s.coef);
-            MPET_CHECK_LAUNCH();
-        }
+    }
+    const PatchCoef q = use ? c->asm_coef : PatchCoef{};
+    if (use && q.ncell > 0) {
+        k_patch_coef<<<grid_for(s.np * s.P, 256), 256, 0, c->stream>>>(s.np * s.P, s.P, s.cell, q.ncell, c->nc,
+                                                                       c->asm_cell, s.coef);
+        MPET_CHECK_LAUNCH();
     }
     // captured iterations hold the coefficients and the choice
     if (use != c->sys_patch || (use && (s.coef != coef0 || memcmp(&q, &c->patch_coef, sizeof(q)) != 0)))

@@ -433,7 +433,12 @@ struct mpet_ctx {
     mpet::PatchCoef patch_coef{};
     bool sys_patch = false;
     int sys_patch_mode = -1;
-    bool asm_bc = false;          // apply_bc of the last assembly
+    // what the last assembly took from the parameters and the caller's arrays for them (per-cell
+    // values: planes of nc)
+    bool asm_taken = false;
+    mpet::PatchCoef asm_coef{};
+    float* asm_cell = nullptr;
+    int64_t asm_ncell = 0;
     // Robin matrix of the last assembly, in FP32: entries 3 q + w of boundary-vertex incidence q
     // (bn_ptr), columns (vertices) and J planes of values
     int32_t* rob_col = nullptr;
@@ -641,10 +646,14 @@ void launch_assemble_prec_blocks(mpet_ctx* c, double dt);
 // per-cell data of the matrix-free first displacement level (c->mf_cell, c->mf_tab);
 // leaves c->mf_cell null when HBM is short
 void launch_mf_cells(mpet_ctx* c, double dt);
-// per-cell geometry of the patch products (once per patch set), and their coefficients for
-// this assembly (sets c->patch_coef and c->sys_patch)
+// per-cell geometry of the patch products (once per patch set)
 void launch_patch_geometry(mpet_ctx* c);
-void set_patch_coefficients(mpet_ctx* c, double dt, bool apply_bc);
+// The coefficients of the patch products are those of the assembled matrix: mpet_assemble takes
+// them, Robin entries and per-cell values with it, into the context's own memory, so that nothing of
+// the caller's is read again when the patches are built later.  use_patches decides whether the
+// inner products go by patches (c->sys_patch) and hands them the coefficients.
+void take_patch_coefficients(mpet_ctx* c, double dt, bool apply_bc);
+void use_patches(mpet_ctx* c);
 void setup_network_modes(mpet_ctx* c, double dt);
 void set_instances(mpet_ctx* c, int ninst, const int32_t* vertex_inst_host);
 void launch_rhs(mpet_ctx* c, double dt, const double* up_prev, double* b);
