@@ -135,7 +135,7 @@ struct PatchDims {
 };
 
 // the Robin matrix's part of network a's row at vertex v
-__device__ __forceinline__ float patch_robin(const PatchDims& D, int a, int64_t v, const float* __restrict__ x) {
+__device__ __forceinline__ float patch_robin(const PatchDims& D, int a, int64_t v, const float* x) {
     const int64_t e1 = 3 * __ldg(D.bn_ptr + v + 1);
     float s = 0.f;
     for (int64_t e = 3 * __ldg(D.bn_ptr + v); e < e1; ++e)
@@ -145,8 +145,8 @@ __device__ __forceinline__ float patch_robin(const PatchDims& D, int a, int64_t 
 
 template <int J, bool DOT>
 __global__ void __launch_bounds__(256, J <= 4 ? 3 : 2) k_patch_sys(PatchArgs A, PatchDims D, PatchCoef C,
-                                                      const float* __restrict__ x, PatchOut O, double* partials,
-                                                      const double* __restrict__ skip) {
+                                                      const float* x, PatchOut O, double* partials,
+                                                      const double* skip) {
     extern __shared__ float psm[];
     const int P = A.P, t = threadIdx.x, M = A.max_pn, V = A.max_pv;
     float* sx = psm;                // three planes of max_pn: u
@@ -351,11 +351,11 @@ __global__ void __launch_bounds__(256, J <= 4 ? 3 : 2) k_patch_sys(PatchArgs A, 
 template <int J, bool DOT>
 __global__ void __launch_bounds__(256) k_patch_sys_shared(int64_t nsh, const int32_t* __restrict__ sh_node,
                                                           const int32_t* __restrict__ sh_ptr,
-                                                          const float4* __restrict__ part, PatchDims D, int bc, int robin,
-                                                          const float* __restrict__ x, PatchOut O, double* partials,
+                                                          const float4* part, PatchDims D, int bc, int robin,
+                                                          const float* x, PatchOut O, double* partials,
                                                           int first, unsigned* cnt,
                                                           const int32_t* __restrict__ node_inst,
-                                                          const double* __restrict__ skip) {
+                                                          const double* skip) {
     pdl_wait();
     const float cr = DOT ? O.sc->f_c_r1 : 0.f;
     DotAcc dot;

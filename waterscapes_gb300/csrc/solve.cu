@@ -66,6 +66,9 @@ int choose_lpr(int64_t n, int64_t nnz) {
 // while they waited (16^3 FP64: 303 us per iteration without, 313 to 329 at once, 278 late; 28^3
 // A=4 FP64: 856, 882, 793; 64^3: 1910, 1887, 1820; 24^3 total pressure: 227, 220, 205).  Outside a
 // capture, after a change of stream and after a wait for an event the launch is an ordinary one.
+// Vectors, scalars and flags, which earlier kernels of an iteration write, are parameters without
+// __restrict__: the kernel is alive while its predecessor still writes them, and a read-only load
+// may take only what nothing writes meanwhile.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -300,7 +303,7 @@ struct EpiResid64 {
 // store, when every one of them has converged (done != 0).  The products of a
 // converged instance are never read again in the inner solve.
 __device__ __forceinline__ bool slice_frozen(const int32_t* __restrict__ skl, int64_t s,
-                                             const double* __restrict__ done) {
+                                             const double* done) {
     const int lo = skl[2 * s], hi = skl[2 * s + 1];
     for (int i = lo; i <= hi; ++i)
         if (done[i] == 0.0) return false;
@@ -310,9 +313,9 @@ __device__ __forceinline__ bool slice_frozen(const int32_t* __restrict__ skl, in
 template <typename T, int NV, int LPR, int U, class Epi>
 __global__ void __launch_bounds__(256) k_spmv(int64_t n, const int64_t* __restrict__ rp,
                                               const int32_t* __restrict__ ci, const T* __restrict__ va,
-                                              const T* __restrict__ x, Epi epi, double* partials,
+                                              const T* x, Epi epi, double* partials,
                                               const int32_t* __restrict__ skl = nullptr,
-                                              const double* __restrict__ skip = nullptr) {
+                                              const double* skip = nullptr) {
     constexpr int RPW = 32 / LPR;  // rows per warp per pass
     const int lane = threadIdx.x & 31;
     const int sub = lane & (LPR - 1);
@@ -416,9 +419,9 @@ __global__ void __launch_bounds__(256) k_spmv(int64_t n, const int64_t* __restri
 template <typename T, int NV, int U, class Epi, bool LATE>
 __device__ __forceinline__ void spmv_sell_body(int64_t n, int64_t nslices, const int64_t* __restrict__ soff,
                                                    const int32_t* __restrict__ sci, const T* __restrict__ sva,
-                                                   const T* __restrict__ x, Epi epi, double* partials,
+                                                   const T* x, Epi epi, double* partials,
                                                    const int32_t* __restrict__ skl,
-                                                   const double* __restrict__ skip) {
+                                                   const double* skip) {
     const int lane = threadIdx.x & 31;
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -504,9 +507,9 @@ __device__ __forceinline__ void spmv_sell_body(int64_t n, int64_t nslices, const
 template <typename T, int NV, int U, class Epi>
 __global__ void __launch_bounds__(256) k_spmv_sell(int64_t n, int64_t nslices, const int64_t* __restrict__ soff,
                                                    const int32_t* __restrict__ sci, const T* __restrict__ sva,
-                                                   const T* __restrict__ x, Epi epi, double* partials,
+                                                   const T* x, Epi epi, double* partials,
                                                    const int32_t* __restrict__ skl = nullptr,
-                                                   const double* __restrict__ skip = nullptr) {
+                                                   const double* skip = nullptr) {
     spmv_sell_body<T, NV, U, Epi, false>(n, nslices, soff, sci, sva, x, epi, partials, skl, skip);
 }
 
@@ -514,10 +517,10 @@ template <typename T, int NV, int U, class Epi>
 __global__ void __launch_bounds__(256, 8) k_spmv_sell_late(int64_t n, int64_t nslices,
                                                           const int64_t* __restrict__ soff,
                                                           const int32_t* __restrict__ sci,
-                                                          const T* __restrict__ sva, const T* __restrict__ x,
+                                                          const T* __restrict__ sva, const T* x,
                                                           Epi epi, double* partials,
                                                           const int32_t* __restrict__ skl = nullptr,
-                                                          const double* __restrict__ skip = nullptr) {
+                                                          const double* skip = nullptr) {
     spmv_sell_body<T, NV, U, Epi, true>(n, nslices, soff, sci, sva, x, epi, partials, skl, skip);
 }
 
@@ -529,9 +532,9 @@ template <int NV, int U, class Epi>
 __global__ void __launch_bounds__(256) k_spmv_sell_h(int64_t n, int64_t nslices, const int64_t* __restrict__ soff,
                                                      const int32_t* __restrict__ sci, const __half* __restrict__ sva,
                                                      const float* __restrict__ dg, float hs,
-                                                     const float* __restrict__ x, Epi epi, double* partials,
+                                                     const float* x, Epi epi, double* partials,
                                                      const int32_t* __restrict__ skl,
-                                                     const double* __restrict__ skip) {
+                                                     const double* skip) {
     pdl_wait();
     const int lane = threadIdx.x & 31;
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
@@ -704,9 +707,9 @@ template <typename T, int JM, class Epi, bool UU = false, bool OCC = false, bool
 __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 3 : (OCC ? 4 : 1)) k_spmv_nb(int64_t nnodes, int64_t nv, int64_t Nu, int J, int64_t nsu,
                                                  int64_t ns, const NbSlice* __restrict__ sl,
                                                  const int32_t* __restrict__ perm, const int32_t* __restrict__ cols,
-                                                 const T* __restrict__ vals, const T* __restrict__ x, Epi epi,
+                                                 const T* __restrict__ vals, const T* x, Epi epi,
                                                  double* partials, const int32_t* __restrict__ skl = nullptr,
-                                                 const double* __restrict__ skip = nullptr) {
+                                                 const double* skip = nullptr) {
     pdl_wait();
     const int lane = threadIdx.x & 31;
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
@@ -1494,7 +1497,7 @@ __global__ void __launch_bounds__(256) k_p2lap_mf(int64_t nnodes, const int64_t*
                                                   const int32_t* __restrict__ inc,
                                                   const int32_t* __restrict__ cell_nodes, const T* __restrict__ cdat,
                                                   const uint8_t* __restrict__ node_bc, const float* __restrict__ tab,
-                                                  const T* __restrict__ x, Epi epi) {
+                                                  const T* x, Epi epi) {
     pdl_wait();
     constexpr int NN = Simplex<D>::NN, NQ = D * (D + 1) / 2, NP = NN * (NN + 1) / 2;
     __shared__ float s_t6[NP * NQ];
@@ -1743,7 +1746,7 @@ template void spmv<float>(mpet_ctx*, const Csr&, int, const float*, float*);
 // ---- vector kernels ----------------------------------------------------------------
 
 template <typename T>
-__global__ void k_cheb_first(int64_t n, int nvec, const T* __restrict__ b, const T* __restrict__ dinv, T* x,
+__global__ void k_cheb_first(int64_t n, int nvec, const T* b, const T* __restrict__ dinv, T* x,
                              T inv_theta) {
     pdl_wait();
     int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -1754,7 +1757,7 @@ __global__ void k_cheb_first(int64_t n, int nvec, const T* __restrict__ b, const
 // Coarsest level: a warp per row of the dense FP64 inverse, every component of the row from one
 // pass over it.
 template <typename T, int NV>
-__global__ void k_dense_coarse(int64_t n, const double* __restrict__ cinv, const T* __restrict__ b, T* x) {
+__global__ void k_dense_coarse(int64_t n, const double* __restrict__ cinv, const T* b, T* x) {
     pdl_wait();
     constexpr int NC = ncomp<NV>();
     const int lane = threadIdx.x & 31;
@@ -1926,7 +1929,7 @@ __device__ __forceinline__ double sum_partials_n(const double* p, int n, double*
 // iteration on the 4^3 cube (A=2, FP32), 256 -> 230 at 24^3 (total pressure).
 template <typename T>
 __global__ void __launch_bounds__(256) k_mr_lanczos(int64_t nodes, int dim, int64_t n, T* y,
-                                                    const T* __restrict__ r2, T* packed,
+                                                    const T* r2, T* packed,
                                                     T* first, const T* __restrict__ dinv, T inv_theta,
                                                     const int32_t* __restrict__ perm, const MinresScalars* sc) {
     pdl_wait();
@@ -1955,8 +1958,8 @@ __global__ void __launch_bounds__(256) k_mr_lanczos(int64_t nodes, int dim, int6
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) k_mr_dot(int64_t nodes, int dim, int64_t n, const T* __restrict__ r, T* z,
-                                                const T* __restrict__ packed, const int32_t* __restrict__ perm,
+__global__ void __launch_bounds__(256) k_mr_dot(int64_t nodes, int dim, int64_t n, const T* r, T* z,
+                                                const T* packed, const int32_t* __restrict__ perm,
                                                 double* partials, unsigned* cnt, MinresScalars* sc) {
     pdl_wait();
     __shared__ double sh[8];
@@ -1986,8 +1989,8 @@ __global__ void __launch_bounds__(256) k_mr_dot(int64_t nodes, int dim, int64_t 
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) k_mr_direction(int64_t n, const T* __restrict__ z, T* v,
-                                                      const T* __restrict__ w1, const T* __restrict__ w2, T* w, T* d,
+__global__ void __launch_bounds__(256) k_mr_direction(int64_t n, const T* z, T* v,
+                                                      const T* w1, const T* w2, T* w, T* d,
                                                       const MinresScalars* sc) {
     pdl_wait();
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -2209,7 +2212,7 @@ __global__ void k_unpack43(int64_t nodes, int dim, const T* __restrict__ b4, T* 
 // with the Q of the vertex's instance
 template <typename T, bool FWD>
 __global__ void k_modes(int64_t nv, int J, const int32_t* __restrict__ vinst, const double* __restrict__ Q,
-                        const T* __restrict__ in, T* out) {
+                        const T* in, T* out) {
     pdl_wait();
     const int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (v >= nv) return;
@@ -2948,8 +2951,8 @@ __device__ __forceinline__ double sum_chunks(const double* part, const int32_t* 
 template <typename T>
 __global__ void __launch_bounds__(256) k_bmr_alfa(const int64_t* __restrict__ lo, const int32_t* __restrict__ len,
                                                   const int32_t* __restrict__ inst, const int32_t* __restrict__ cptr,
-                                                  const int32_t* __restrict__ chunks, T* y, const T* __restrict__ r1,
-                                                  const T* __restrict__ v, MinresScalars* sc, double* part,
+                                                  const int32_t* __restrict__ chunks, T* y, const T* r1,
+                                                  const T* v, MinresScalars* sc, double* part,
                                                   unsigned* cnt, double* done) {
     pdl_wait();
     __shared__ double sh[8];
@@ -2985,10 +2988,10 @@ __global__ void __launch_bounds__(256) k_bmr_alfa(const int64_t* __restrict__ lo
 // iteration's y, would grow through them until 0 * inf in a padded entry reached open instances.
 template <typename T>
 __global__ void __launch_bounds__(256) k_bmr_axpy(const int64_t* __restrict__ lo, const int32_t* __restrict__ len,
-                                                  const int32_t* __restrict__ inst, T* y, const T* __restrict__ r2,
+                                                  const int32_t* __restrict__ inst, T* y, const T* r2,
                                                   int64_t Nu, T* packed, const int32_t* __restrict__ perm,
-                                                  const MinresScalars* __restrict__ sc,
-                                                  const double* __restrict__ done) {
+                                                  const MinresScalars* sc,
+                                                  const double* done) {
     pdl_wait();
     const int64_t ch = blockIdx.x;
     const int in = inst[ch];
@@ -3010,8 +3013,8 @@ __global__ void __launch_bounds__(256) k_bmr_axpy(const int64_t* __restrict__ lo
 template <typename T>
 __global__ void __launch_bounds__(256) k_bmr_beta(const int64_t* __restrict__ lo, const int32_t* __restrict__ len,
                                                   const int32_t* __restrict__ inst, const int32_t* __restrict__ cptr,
-                                                  const int32_t* __restrict__ chunks, const T* __restrict__ rr, T* z,
-                                                  int64_t Nu, const T* __restrict__ packed,
+                                                  const int32_t* __restrict__ chunks, const T* rr, T* z,
+                                                  int64_t Nu, const T* packed,
                                                   const int32_t* __restrict__ perm, MinresScalars* sc, double* part,
                                                   unsigned* cnt, const double* __restrict__ target, double* done) {
     pdl_wait();
@@ -3043,10 +3046,10 @@ __global__ void __launch_bounds__(256) k_bmr_beta(const int64_t* __restrict__ lo
 // w = (v - oldeps w1 - delta w2) / gamma, d += phi w; v = z / beta for the next iteration
 template <typename T>
 __global__ void __launch_bounds__(256) k_bmr_update(const int64_t* __restrict__ lo, const int32_t* __restrict__ len,
-                                                    const int32_t* __restrict__ inst, const T* __restrict__ z, T* v,
-                                                    const T* __restrict__ w1, const T* __restrict__ w2, T* w, T* d,
-                                                    const MinresScalars* __restrict__ sc,
-                                                    const double* __restrict__ done) {
+                                                    const int32_t* __restrict__ inst, const T* z, T* v,
+                                                    const T* w1, const T* w2, T* w, T* d,
+                                                    const MinresScalars* sc,
+                                                    const double* done) {
     pdl_wait();
     const int64_t ch = blockIdx.x;
     const double dn = done[inst[ch]];

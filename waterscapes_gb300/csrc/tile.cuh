@@ -85,8 +85,8 @@ struct Pair<double> {
 
 template <typename T, int NV, int LPR, class Epi>
 __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 4 : 5) k_spmv_tile(TileArgs A, const T* __restrict__ va,
-                                                                          const T* __restrict__ x, Epi epi,
-                                                                          const double* __restrict__ skip) {
+                                                                          const T* x, Epi epi,
+                                                                          const double* skip) {
     constexpr int RW = 32 / LPR, R = 256 / LPR, NC = ncomp<NV>(), PF = 4, CQ = TILE_MAX_COLS / 256;
     extern __shared__ __align__(128) unsigned char smem[];
     typedef typename Pair<T>::type P2;
