@@ -740,6 +740,11 @@ void krylov_product_f32(mpet_ctx* c, const float* x, float* y);
 bool spmv_variant_available(const Csr& A, int variant);
 constexpr int SPMV_TILE = 2048;  // entries per staged tile
 constexpr int TILE_MAX_COLS = 2048;  // distinct columns of a row tile
+// most dynamic shared memory of a row-tile block and of a patch block.  A kernel's limit is one for
+// all contexts of the process, so it is always set to these: set to a launch's own need, another
+// thread's smaller one could come between the call and the launch
+constexpr int TILE_SMEM = 72 * 1024;
+constexpr int PATCH_SMEM = 200 * 1024;
 void destroy_minres_graph(mpet_ctx* c);
 
 }  // namespace mpet

@@ -420,7 +420,7 @@ static void launch_patch_sys_j(mpet_ctx* c, const float* x, const PatchOut& O) {
     const int64_t items = s.nsh + (int64_t)J * s.nshv;
     const int g1 = (int)std::min<int64_t>(s.np, 456);
     const int g2 = (int)std::min<int64_t>(std::max<int64_t>((items + 255) / 256, 1), NB_RED - 456);
-    MPET_CUDA(cudaFuncSetAttribute(k_patch_sys<J, DOT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    MPET_CUDA(cudaFuncSetAttribute(k_patch_sys<J, DOT>, cudaFuncAttributeMaxDynamicSharedMemorySize, PATCH_SMEM));
     launch_k(c, k_patch_sys<J, DOT>, g1, s.P, sm, patch_args(c), D, c->patch_coef, x, O, c->partials, skip);
     launch_k(c, k_patch_sys_shared<J, DOT>, g2, 256, 0, s.nsh, s.sh_node, s.sh_ptr, (const float4*)s.part, D,
                                                           c->patch_coef.bc, c->patch_coef.robin, x, O, c->partials, g1, c->red_cnt,

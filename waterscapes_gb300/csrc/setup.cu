@@ -934,7 +934,7 @@ void build_patches(mpet_ctx* c) {
     }
     c->pool.release(key);
     // shared memory of a block (patch.cuh): x at the nodes and the contributions
-    if (4 * (5 * s.max_pn + J * s.max_pv + (30 + 4 * J) * P) > 200 * 1024) {
+    if (4 * (5 * s.max_pn + J * s.max_pv + (30 + 4 * J) * P) > PATCH_SMEM) {
         release_patches(c);
         c->patch.tried = true;
         return;
@@ -1156,7 +1156,7 @@ static bool build_tiles_of(mpet_ctx* c, Csr& A, const int32_t* order, int nvec, 
     for (int64_t t = 0; t < nt; ++t) r.mc = std::max(r.mc, cp[t + 1] - cp[t]);
     r.mc = (r.mc + 31) / 32 * 32;
     // (x in shared memory: three blocks per SM at least)
-    if ((size_t)r.mc * nvec * (fp32 ? 4 : 8) > 72 * 1024 || r.mc > TILE_MAX_COLS) {
+    if ((size_t)r.mc * nvec * (fp32 ? 4 : 8) > TILE_SMEM || r.mc > TILE_MAX_COLS) {
         c->pool.release(key);
         release_row_tiles(c, r);
         return false;

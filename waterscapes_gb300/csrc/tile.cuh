@@ -178,7 +178,7 @@ template <typename T, int NV, int LPR, class Epi>
 static void launch_tile_l(mpet_ctx* c, const RowTiles& r, int64_t n, const T* x, const Epi& epi) {
     const size_t sm = (size_t)r.mc * NV * sizeof(T);
     auto kern = k_spmv_tile<T, NV, LPR, Epi>;
-    if (sm > 48 * 1024) MPET_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    if (sm > 48 * 1024) MPET_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TILE_SMEM));
     const TileArgs A{n, r.perm ? nullptr : r.row, r.col, r.eoff, r.steps, r.lc, r.skl, r.mc};
     launch_k(c, kern, r.nt, 256, sm, A, (const T*)r.v, x, epi, r.skl ? c->skip_done : (const double*)nullptr);
     MPET_CHECK_LAUNCH();
