@@ -34,7 +34,7 @@ def _compile(src, extra=()):
     out = os.path.join(BUILD, os.path.splitext(src)[0] + ".o")
     path = os.path.join(CSRC, src)
     deps = [path, os.path.join(CSRC, "mpet_internal.cuh"), os.path.join(CSRC, "patch.cuh"),
-            os.path.join(CSRC, "tile.cuh"),
+            os.path.join(CSRC, "tile.cuh"), os.path.join(CSRC, "dot_acc.cuh"),
             os.path.join(HERE, "..", "include", "mpet_gpu.h")]
     if os.path.exists(out) and all(os.path.getmtime(out) >= os.path.getmtime(d) for d in deps):
         return out

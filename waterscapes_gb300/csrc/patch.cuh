@@ -72,22 +72,6 @@ __device__ __forceinline__ void patch_scatter(float (&F)[4][4], float* sc, const
         for (int b = a + 1; b < 4; ++b) sc[pos[edge_node(a, b)]] = 4.f * (F[a][b] + F[b][a]);
 }
 
-// Sum of products of FP32 values to about twice FP32 precision, without the FP64 pipe (an
-// FP64 sum of the 64^3 case's 7.5e6 products costs 40 us there): the products and the sums are
-// split into their rounded values and the exact errors, and the errors are summed apart.
-struct DotAcc {
-    float hi = 0.f, lo = 0.f;
-    __device__ __forceinline__ void add(float a, float b) {
-        const float p = __fmul_rn(a, b);
-        const float e = __fmaf_rn(a, b, -p);
-        const float s = __fadd_rn(hi, p);
-        const float z = __fsub_rn(s, hi);
-        lo += __fadd_rn(__fadd_rn(__fsub_rn(hi, __fsub_rn(s, z)), __fsub_rn(p, z)), e);
-        hi = s;
-    }
-    __device__ __forceinline__ double value() const { return (double)hi + (double)lo; }
-};
-
 // y = A x; DOT: y = A x - (beta / oldb) r1 with the partial sums of x . y (EpiMinres)
 struct PatchOut {
     float* y;

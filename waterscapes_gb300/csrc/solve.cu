@@ -28,6 +28,7 @@
 #include <cstring>
 #include <utility>
 
+#include "dot_acc.cuh"
 #include "mpet_internal.cuh"
 
 namespace mpet {
@@ -1963,8 +1964,7 @@ __global__ void __launch_bounds__(256) k_mr_dot(int64_t nodes, int dim, int64_t 
                                                 double* partials, unsigned* cnt, MinresScalars* sc) {
     pdl_wait();
     __shared__ double sh[8];
-    // a thread's products are summed in the working precision (a few dozen terms), then in FP64
-    T acc = T(0);
+    typename DotOf<T>::type acc;
     const int64_t items = nodes + (n - dim * nodes);
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < items; i += (int64_t)gridDim.x * blockDim.x) {
         if (i < nodes) {
@@ -1974,14 +1974,14 @@ __global__ void __launch_bounds__(256) k_mr_dot(int64_t nodes, int dim, int64_t 
             for (int k = 0; k < 3; ++k)
                 if (k < dim) {
                     z[dim * i + k] = v[k];
-                    acc += r[dim * i + k] * v[k];
+                    acc.add(r[dim * i + k], v[k]);
                 }
         } else {
             const int64_t row = dim * nodes + (i - nodes);
-            acc += r[row] * z[row];
+            acc.add(r[row], z[row]);
         }
     }
-    const double s = block_sum256((double)acc, sh);
+    const double s = block_sum256(acc.value(), sh);
     if (threadIdx.x == 0) partials[blockIdx.x] = s;
     if (!last_block(cnt)) return;
     const double t = sum_partials_n(partials, gridDim.x, sh);
