@@ -53,3 +53,30 @@ def test_the_coefficients_are_those_of_the_assembly(what):
     torch.cuda.synchronize()
     s.ctx.call("mpet_setup_preconditioner", dt)
     _check_product(s, 1)
+
+
+def test_small_cells_keep_their_terms():
+    """Cells of 5e-8 (metres, say) with K dt of 1e-19 and 1e-20: entries K dt h of 5e-27 are well inside
+    FP32's range, but the product of the cell's volume and K dt, 2e-42, is not."""
+    from waterscapes_gb300 import Mesh, MPETProblem, MPETSolver, UnitCubeMesh, Constant, _lib
+    from helpers import cfg_params
+    unit = UnitCubeMesh(4)
+    mesh = Mesh(unit.coordinates() * 2e-7, unit.cells())
+    params, _ = cfg_params(2)
+    params.update(K=(1e-17, 1e-18), c=(0.0, 0.0), S=((0.0, 0.0), (0.0, 0.0)))
+    s = MPETSolver(MPETProblem(mesh, Constant(0.0), params=params), dict(dt=1e-2, precision="mixed"))
+    s.ctx.call("mpet_set_element_product", 1)
+    s.ctx.call("mpet_assemble", 1e-2, 1)
+    import scipy.sparse as sp
+    rp, ci = s.pattern()
+    A = sp.csr_matrix((s.matrix_values(), ci, rp), shape=(s.N, s.N))
+    x = np.random.default_rng(6).standard_normal(s.N)
+    x[:s.Nu] = 0.0  # the stiffness term alone in the pressure rows
+    x = torch.tensor(x, dtype=torch.float32, device=s.device)
+    y = torch.full_like(x, float("nan"))
+    s.ctx.call("mpet_krylov_product", _lib._ptr(x), _lib._ptr(y), None)
+    torch.cuda.synchronize()
+    xd, yd = x.double().cpu().numpy(), y.double().cpu().numpy()
+    err, scale = np.abs(yd - A @ xd), abs(A) @ np.abs(xd)
+    for b in [slice(0, s.Nu)] + [slice(s.Nu + a * s.nv, s.Nu + (a + 1) * s.nv) for a in range(2)]:
+        assert np.linalg.norm(err[b]) <= 2e-6 * np.linalg.norm(scale[b])

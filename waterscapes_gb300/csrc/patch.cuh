@@ -17,6 +17,15 @@
 // a cell needs the stress at its four vertices and the P1 mass matrix between them: about 700
 // operations with four networks, for 40 bytes of geometry, 40 bytes of local numbering and
 // the cell's share of its nodes, where the stored node-block matrix costs 2900 bytes per cell.
+//
+// Rounding: FP32 like the stored copy that it replaces, in other places.  Differences of u and p are
+// taken before anything is scaled, so smooth vectors, whose products cancel, come out closer than from
+// rounded entries.  Error against the FP64 matrix relative to || A x || (48^3, A=4; elements, stored):
+// Lanczos-like vectors (M^-1 A)^5 v, displacement rows 4.9e-6, 1.7e-5, pressure rows 1e-7, 2e-6; smooth
+// interpolants 2.7e-5, 7.0e-5 and 9e-12, 2.5e-11; random vectors 1.0e-7, 1.2e-7 and 4e-11, 6e-11.
+// Further off only in the displacement rows of vectors that are nearly all pressure, where the stress is
+// the pressure's rounding: M^-1 of random vectors 2.1e-7, 1.1e-7, of smooth ones 1.4e-6, 4.5e-7 (their
+// pressure rows 8e-8, 2.4e-6).
 #pragma once
 
 struct PatchArgs {
@@ -59,17 +68,29 @@ __device__ __forceinline__ void patch_u16x10(const uint32_t* __restrict__ w, int
     }
 }
 
-// The contributions of one component of a cell from F_cv (v = 1..3; F_c0 = -(F_c1 + F_c2 + F_c3)):
-// vertex v: 4 F_vv - sum_c F_cv, edge (a, b): 4 (F_ab + F_ba)
-__device__ __forceinline__ void patch_scatter(float (&F)[4][4], float* sc, const int (&pos)[10]) {
+// The contributions of one component of a cell.  With T_c = R_c + s and F_cv = T_c . b_v (b_0 = -(b_1 +
+// b_2 + b_3)): edge (a, b): 4 w (F_ab + F_ba); vertex v: w (4 F_vv - sum_c F_cv) = w (4 R_v - s) . b_v, in
+// the second form, whose large parts cancel before they are rounded.
+__device__ __forceinline__ void patch_scatter(const float (&R)[4][3], const float (&s)[3], const float (&b)[3][3],
+                                              float w, float* sc, const int (&pos)[10]) {
+    float F[4][4];
 #pragma unroll
-    for (int c = 0; c < 4; ++c) F[c][0] = -(F[c][1] + F[c][2] + F[c][3]);
+    for (int c = 0; c < 4; ++c) {
+        float g[3];
 #pragma unroll
-    for (int v = 0; v < 4; ++v) sc[pos[v]] = 4.f * F[v][v] - (F[0][v] + F[1][v] + F[2][v] + F[3][v]);
+        for (int l = 0; l < 3; ++l)
+            g[l] = c > 0 ? b[c > 0 ? c - 1 : 0][l] : -(b[0][l] + b[1][l] + b[2][l]);
+        sc[pos[c]] = w * ((4.f * R[c][0] - s[0]) * g[0] + (4.f * R[c][1] - s[1]) * g[1] + (4.f * R[c][2] - s[2]) * g[2]);
+        const float t0 = R[c][0] + s[0], t1 = R[c][1] + s[1], t2 = R[c][2] + s[2];
+#pragma unroll
+        for (int v = 1; v < 4; ++v) F[c][v] = t0 * b[v - 1][0] + t1 * b[v - 1][1] + t2 * b[v - 1][2];
+        F[c][0] = -(F[c][1] + F[c][2] + F[c][3]);
+    }
+    const float w4 = 4.f * w;
 #pragma unroll
     for (int a = 0; a < 4; ++a)
 #pragma unroll
-        for (int b = a + 1; b < 4; ++b) sc[pos[edge_node(a, b)]] = 4.f * (F[a][b] + F[b][a]);
+        for (int e = a + 1; e < 4; ++e) sc[pos[edge_node(a, e)]] = w4 * (F[a][e] + F[e][a]);
 }
 
 // y = A x; DOT: y = A x - (beta / oldb) r1 with the partial sums of x . y (EpiMinres)
@@ -213,35 +234,23 @@ __global__ void __launch_bounds__(256, J <= 4 ? 3 : 2) k_patch_sys(PatchArgs A, 
                 S[c][5] = C.mu * (H[c][1][2] + H[c][2][1]);
             }
         }
-        // the P1 mass matrix between the vertices: |T| / 20 (1 + delta)
-#pragma unroll
-        for (int q = 0; q < 6; ++q) {
-            const float s = S[0][q] + S[1][q] + S[2][q] + S[3][q];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) S[c][q] = w * (S[c][q] + s);
-        }
-        {
-            const float s = tr[0] + tr[1] + tr[2] + tr[3];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) tr[c] = w * (tr[c] + s);
-        }
+        // The P1 mass matrix between the vertices is |T| / 20 (1 + delta); the factor w comes last, as
+        // on a small cell it is far smaller than the products that it scales.
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            const int q0 = k, q1 = k == 0 ? 3 : k == 1 ? 3 : 4, q2 = k == 0 ? 4 : 5;
-            float F[4][4];
+            float R[4][3], s[3];  // row k of the stress at the vertices and its sum over them
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const float s0 = k == 0 ? S[c][0] : S[c][q1];
-                const float s1 = k == 1 ? S[c][1] : (k == 0 ? S[c][3] : S[c][5]);
-                const float s2 = k == 2 ? S[c][2] : S[c][q2];
-                (void)q0;
+            for (int l = 0; l < 3; ++l) {
+                const int q = k == l ? k : k + l + 2;
 #pragma unroll
-                for (int v = 1; v < 4; ++v) F[c][v] = s0 * b[v - 1][0] + s1 * b[v - 1][1] + s2 * b[v - 1][2];
+                for (int c = 0; c < 4; ++c) R[c][l] = S[c][q];
+                s[l] = R[0][l] + R[1][l] + R[2][l] + R[3][l];
             }
-            if (live) patch_scatter(F, sc + k * 10 * P, pos);
+            if (live) patch_scatter(R, s, b, w, sc + k * 10 * P, pos);
         }
         // pressure rows: coupling, mass-type and stiffness terms
         {
+            const float ts = tr[0] + tr[1] + tr[2] + tr[3];
             float pv[J][4], ps[J];
 #pragma unroll
             for (int a = 0; a < J; ++a) {
@@ -254,7 +263,7 @@ __global__ void __launch_bounds__(256, J <= 4 ? 3 : 2) k_patch_sys(PatchArgs A, 
                 const float d1 = pv[a][1] - pv[a][0], d2 = pv[a][2] - pv[a][0], d3 = pv[a][3] - pv[a][0];
                 float kd = C.Kd[a];
                 if (C.ncell > 0) kd = __ldg(D.coef + (p * C.ncell + a) * P + t);
-                kd *= 20.f * w;
+                kd *= 20.f;
                 float gr[3];
 #pragma unroll
                 for (int l = 0; l < 3; ++l) gr[l] = kd * (d1 * b[0][l] + d2 * b[1][l] + d3 * b[2][l]);
@@ -263,18 +272,17 @@ __global__ void __launch_bounds__(256, J <= 4 ? 3 : 2) k_patch_sys(PatchArgs A, 
                 for (int v = 1; v < 4; ++v) o[v] = gr[0] * b[v - 1][0] + gr[1] * b[v - 1][1] + gr[2] * b[v - 1][2];
                 o[0] = -(o[1] + o[2] + o[3]);
 #pragma unroll
-                for (int c = 0; c < 4; ++c) o[c] += C.cpl[a] * tr[c];
+                for (int c = 0; c < 4; ++c) o[c] += C.cpl[a] * (tr[c] + ts);
 #pragma unroll
-                for (int e = 0; e < J; ++e) {
+                for (int e = 0; e < J; ++e) {  // (p_e, lambda_c) = w (p_e(c) + sum)
                     float cm = C.Cm[a * MPET_MAX_NETWORKS + e];
                     if (C.ncell > J) cm = __ldg(D.coef + (p * C.ncell + J + a * J + e) * P + t);
-                    cm *= w;  // (p_e, lambda_c) = |T| / 20 (p_e(c) + sum)
 #pragma unroll
                     for (int c = 0; c < 4; ++c) o[c] += cm * (pv[e][c] + ps[e]);
                 }
                 if (live)
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) scp[a * 4 * P + pos[c]] = o[c];
+                    for (int c = 0; c < 4; ++c) scp[a * 4 * P + pos[c]] = w * o[c];
             }
         }
         __syncthreads();
