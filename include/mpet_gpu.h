@@ -402,8 +402,8 @@ int mpet_set_row_tiles(mpet_ctx* ctx, int32_t mode);
 /* How the inner FP32 iterations of a mixed-precision solve form A x: cell by
  * cell from the geometry and the coefficients of the last mpet_assemble (1),
  * from the stored FP32 copy (0), or by the size of the matrix (-1, default).
- * The stored copy serves wherever the element product cannot: triangles, or a
- * variant forced by mpet_set_spmv_variant.
+ * The stored copy serves wherever the element product cannot (triangles)
+ * and, in every mode, once mpet_set_spmv_variant has forced a variant.
  * Takes effect at the next mpet_assemble, which must follow.  No reference
  * counterpart (engine option and test hook). */
 int mpet_set_element_product(mpet_ctx* ctx, int32_t mode);
@@ -441,7 +441,8 @@ int mpet_get_spmv_tuning_fp64(mpet_ctx* ctx, double* ms7_host, int32_t* chosen);
 int mpet_get_node_block_info(mpet_ctx* ctx, int64_t* blocks, int64_t* stored_values);
 
 /* Override the autotuned system-matrix SpMV variant (bits as above) for the
- * products of both precisions;
+ * products of both precisions, the inner iterations' among them, from now
+ * on (mpet_set_element_product keeps its mode but has no effect any more);
  * MPET_ERR_INVALID if the variant cannot run on this matrix.  Every variant
  * computes the same product (summation order differs).  No reference
  * counterpart (tuning and test hook). */

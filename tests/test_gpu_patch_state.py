@@ -80,3 +80,17 @@ def test_small_cells_keep_their_terms():
     err, scale = np.abs(yd - A @ xd), abs(A) @ np.abs(xd)
     for b in [slice(0, s.Nu)] + [slice(s.Nu + a * s.nv, s.Nu + (a + 1) * s.nv) for a in range(2)]:
         assert np.linalg.norm(err[b]) <= 2e-6 * np.linalg.norm(scale[b])
+
+
+@pytest.mark.parametrize("mode", [-1, 1])
+def test_a_forced_variant_stays_forced(mode):
+    from waterscapes_gb300 import MPETSolver
+    problem, dt = make_problem(12, 2)
+    s = MPETSolver(problem, dict(dt=dt, T=1.0, precision="mixed"))
+    s.ctx.call("mpet_set_spmv_variant", 0)
+    s.ctx.call("mpet_set_element_product", mode)
+    s.ctx.call("mpet_assemble", dt, 1)
+    s.ctx.call("mpet_setup_preconditioner", dt)
+    _check_product(s, 0)
+    s.ctx.call("mpet_assemble", 2.0 * dt, 1)
+    _check_product(s, 0)

@@ -963,8 +963,8 @@ int mpet_set_spmv_variant(mpet_ctx* c, int32_t variant) {
     destroy_minres_graph(c);
     c->A.variant = variant;
     c->A.variant64 = -1;  // the forced variant serves both precisions
-    c->sys_patch = false;  // ... and the inner iterations
-    c->sys_patch_mode = 0;
+    c->spmv_forced = true;  // ... and the inner iterations
+    c->sys_patch = false;
     API_END(c)
 }
 

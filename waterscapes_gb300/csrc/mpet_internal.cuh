@@ -433,6 +433,7 @@ struct mpet_ctx {
     mpet::PatchCoef patch_coef{};
     bool sys_patch = false;
     int sys_patch_mode = -1;
+    bool spmv_forced = false;     // mpet_set_spmv_variant: stored products everywhere
     // what the last assembly took from the parameters and the caller's arrays for them (per-cell
     // values: planes of nc)
     bool asm_taken = false;
