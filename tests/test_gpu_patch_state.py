@@ -94,3 +94,28 @@ def test_a_forced_variant_stays_forced(mode):
     _check_product(s, 0)
     s.ctx.call("mpet_assemble", 2.0 * dt, 1)
     _check_product(s, 0)
+
+
+@pytest.mark.parametrize("n,elements", [(12, 1), (4, 0)])
+def test_the_mode_takes_effect_at_the_next_assembly(n, elements):
+    """5.3e6 and 0.2e6 entries: by size, elements and the stored copy."""
+    from waterscapes_gb300 import MPETSolver
+    problem, dt = make_problem(n, 2)
+    s = MPETSolver(problem, dict(dt=dt, T=1.0, precision="mixed"))
+    s.ctx.call("mpet_set_element_product", 0)
+    s.ctx.call("mpet_assemble", dt, 1)
+    s.ctx.call("mpet_setup_preconditioner", dt)
+    _check_product(s, 0)
+    for mode, used in ((-1, elements), (1, 1), (0, 0), (-1, elements)):
+        s.ctx.call("mpet_set_element_product", mode)
+        s.ctx.call("mpet_assemble", dt, 1)
+        _check_product(s, used)
+
+
+def test_the_preconditioner_before_the_assembly():
+    from waterscapes_gb300 import MPETSolver
+    problem, dt = make_problem(12, 2)
+    s = MPETSolver(problem, dict(dt=dt, T=1.0, precision="mixed"))
+    s.ctx.call("mpet_setup_preconditioner", dt)
+    s.ctx.call("mpet_assemble", dt, 1)
+    _check_product(s, 1)

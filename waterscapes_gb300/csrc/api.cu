@@ -287,7 +287,7 @@ int mpet_assemble(mpet_ctx* c, double dt, int32_t apply_bc) {
     launch_assemble_matrix(c, dt, apply_bc != 0);
     launch_robin_matrix(c, dt);
     // (the patches come with the preconditioner: a program that only assembles does without)
-    if (c->sys_patch_mode == 1) build_patches(c);
+    if (wants_patches(c) && (c->sys_patch_mode == 1 || c->precond_ready)) build_patches(c);
     take_patch_coefficients(c, dt, apply_bc != 0);
     use_patches(c);
     values_changed(c);
@@ -555,7 +555,7 @@ int mpet_setup_preconditioner(mpet_ctx* c, double dt) {
     require(c->setup_done, MPET_ERR_STATE, "mpet_setup must come first");
     require(dt > 0.0, MPET_ERR_INVALID, "dt must be positive");
     destroy_minres_graph(c);
-    if (!c->patch.tried && c->sys_patch_mode != 0) {
+    if (wants_patches(c) && !c->patch.tried) {
         build_patches(c);
         if (c->assembled) use_patches(c);  // with the coefficients of that assembly
     }

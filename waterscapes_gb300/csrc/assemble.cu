@@ -959,7 +959,7 @@ __global__ void k_patch_coef(int64_t nslots, int P, const int32_t* __restrict__ 
 // small the mesh, the stored product 4.5 us at 0.2e6 entries (4^3 cube, A=2), 7.4 at 1.6e6
 // (8^3; a whole iteration 72 us stored, 77 by elements), 14.7 at 5.3e6 (12^3; 121 and 112)
 // and 769 against 195 at 1.03e9 (64^3, A=4).
-static bool wants_patches(const mpet_ctx* c) {
+bool wants_patches(const mpet_ctx* c) {
     return c->dim == 3 && c->prm.precision == MPET_PRECISION_MIXED && !c->spmv_forced &&
            (c->sys_patch_mode == 1 || (c->sys_patch_mode < 0 && c->nnz >= 3000000));
 }

@@ -653,6 +653,7 @@ void launch_patch_geometry(mpet_ctx* c);
 // them, Robin entries and per-cell values with it, into the context's own memory, so that nothing of
 // the caller's is read again when the patches are built later.  use_patches decides whether the
 // inner products go by patches (c->sys_patch) and hands them the coefficients.
+bool wants_patches(const mpet_ctx* c);  // by the mode, the size and the kind of system
 void take_patch_coefficients(mpet_ctx* c, double dt, bool apply_bc);
 void use_patches(mpet_ctx* c);
 void setup_network_modes(mpet_ctx* c, double dt);
