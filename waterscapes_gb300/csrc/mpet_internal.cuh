@@ -237,7 +237,8 @@ struct AmgLevel {
     Csr Pt, Rt;
     double* dinv64t = nullptr;
     float* dinv32t = nullptr;
-    bool tiled() const { return A.rt.perm && A.variant == 64 && !mf; }
+    // (not on a coarsest level: it has no transfers, and its dense inverse is in the rows' own order)
+    bool tiled() const { return A.rt.perm && dinv64t && A.variant == 64 && !mf; }
     double* dinv64 = nullptr;
     float* dinv32 = nullptr;
     double rho = 1.0;  // spectral radius estimate of D^-1 A
