@@ -4118,9 +4118,14 @@ void release_hier(mpet_ctx* c, AmgHier& h) {
 
 static void finish_device_csr(mpet_ctx* c, Csr& d, bool fp32);
 
-// P, R and the inverse diagonal of a level whose tiles have their own order
+// P, R and the inverse diagonal of a level whose tiles have their own order; where memory is short
+// (a CSR and a SELL copy of both, some 32 bytes an entry) the level does without its tiles
 static void tiled_transfers(mpet_ctx* c, AmgLevel& L, bool fp32) {
     if (!L.A.rt.perm) return;
+    if (!device_fits(c, (size_t)(L.P.nnz + L.R.nnz) * 32 + (size_t)(L.P.n + L.R.n) * 32)) {
+        release_row_tiles(c, L.A.rt);
+        return;
+    }
     permute_transfers(c, L.A.rt.perm, L.A.rt.row, L.P, L.R, L.dinv64, L.Pt, L.Rt, &L.dinv64t);
     finish_device_csr(c, L.Pt, fp32);
     finish_device_csr(c, L.Rt, fp32);
@@ -4128,6 +4133,22 @@ static void tiled_transfers(mpet_ctx* c, AmgLevel& L, bool fp32) {
         L.dinv32t = c->pool.alloc<float>(L.A.n);
         k_f64_to_f32<<<grid_for(L.A.n, 256), 256, 0, c->stream>>>(L.A.n, L.dinv64t, L.dinv32t);
         MPET_CHECK_LAUNCH();
+    }
+}
+
+// after the autotuner's choices: the tiles and transfers that no product will read
+static void drop_unused_tiles(mpet_ctx* c, AmgHier& h) {
+    for (size_t k = 0; k + 1 < h.lev.size(); ++k) {
+        AmgLevel& L = h.lev[k];
+        if (L.A.rt.perm && !L.tiled()) {
+            release_csr(c, L.Pt);
+            release_csr(c, L.Rt);
+            c->pool.release(L.dinv64t);
+            c->pool.release(L.dinv32t);
+            L.dinv64t = nullptr;
+            L.dinv32t = nullptr;
+        }
+        if (L.A.variant != 64 || L.mf) release_row_tiles(c, L.A.rt);
     }
 }
 
@@ -4186,6 +4207,7 @@ void upload_amg(mpet_ctx* c, AmgHier& h, const HostAmg& ha, int nvec, bool fp32)
     } else {
         if (fp32) autotune_hier<float, 1>(c, h); else autotune_hier<double, 1>(c, h);
     }
+    drop_unused_tiles(c, h);
     h.ncoarse = ha.ncoarse;
     h.cinv = c->pool.alloc<double>(ha.ncoarse * ha.ncoarse);
     MPET_CUDA(cudaMemcpyAsync(h.cinv, ha.cinv.data(), sizeof(double) * ha.ncoarse * ha.ncoarse,
@@ -4247,6 +4269,7 @@ void finish_device_hier(mpet_ctx* c, AmgHier& h, int nvec, bool fp32) {
     } else {
         if (fp32) autotune_hier<float, 1>(c, h); else autotune_hier<double, 1>(c, h);
     }
+    drop_unused_tiles(c, h);
     MPET_CUDA(cudaStreamSynchronize(c->stream));
 }
 
