@@ -324,7 +324,7 @@ __global__ void k_robin_matrix(int64_t nv, int64_t Nu, int64_t nf, int J, const 
                                const double* __restrict__ beta, const int64_t* __restrict__ row_ptr,
                                const int64_t* __restrict__ n2_ptr, const int64_t* __restrict__ n1_ptr,
                                const int32_t* __restrict__ n1_col, const uint8_t* __restrict__ dof_bc, double* v64,
-                               float* v32, double* dinv, double dt_theta) {
+                               double* dinv, double dt_theta) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= nv) return;
     const int64_t q0 = bn_ptr[i], q1 = bn_ptr[i + 1];
@@ -349,7 +349,6 @@ __global__ void k_robin_matrix(int64_t nv, int64_t Nu, int64_t nf, int J, const 
                 for (int v = 0; v < FV; ++v) t += bv[v] * ft1<D>(v, m, w);
                 const int64_t pos = base + lb_i32f(n1_col + s1, d1, fnodes[6 * f + w]);
                 v64[pos] += -dt_theta * area * t;
-                if (v32) v32[pos] = (float)v64[pos];
             }
             touched = true;
         }
@@ -365,7 +364,7 @@ void launch_robin_matrix(mpet_ctx* c, double dt) {
     auto kern = c->dim == 2 ? k_robin_matrix<2> : k_robin_matrix<3>;
     kern<<<grid_for(c->nv, 128), 128, 0, c->stream>>>(
         c->nv, c->Nu, c->nf, c->J, c->bn_ptr, c->bn_list, c->fnodes, c->fgeo, c->markers, c->f_beta_matrix,
-        c->A.rp, c->n2_ptr, c->n1_ptr, c->n1_col, c->dof_bc, c->A.v64, c->A.v32, c->dinv, dt * c->prm.theta);
+        c->A.rp, c->n2_ptr, c->n1_ptr, c->n1_col, c->dof_bc, c->A.v64, c->dinv, dt * c->prm.theta);
     MPET_CHECK_LAUNCH();
 }
 
