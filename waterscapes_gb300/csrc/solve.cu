@@ -144,7 +144,7 @@ __host__ __device__ constexpr int ncomp() { return NV == 4 ? 3 : NV; }
 template <typename T, int NV>
 struct EpiStore {
     T* y;
-    static constexpr bool kTile = false;  // runs with the row-tile kernel
+    static constexpr bool kTile = false;  // not built for the row-tile kernel
     static constexpr int kRed = 0;
     static constexpr bool kSystem = NV == 1;  // runs with the node-block system kernel
     struct Pre {};
@@ -190,7 +190,7 @@ struct EpiStoreFirst {
     T* x0;
     const T* dinv;
     T f;
-    static constexpr bool kTile = false;  // runs with the row-tile kernel
+    static constexpr bool kTile = false;  // not built for the row-tile kernel
     static constexpr int kRed = 0;
     static constexpr bool kSystem = false;
     struct Pre {
@@ -263,7 +263,7 @@ struct EpiMinres {
     const T* r1;
     const T* v;
     const MinresScalars* sc;
-    static constexpr bool kTile = false;  // runs with the row-tile kernel
+    static constexpr bool kTile = false;  // not built for the row-tile kernel
     static constexpr int kRed = 1;
     static constexpr bool kSystem = true;
     struct Pre {
@@ -283,7 +283,7 @@ struct EpiResid64 {
     double* r;
     const double* b;
     const double* dinv;
-    static constexpr bool kTile = false;  // runs with the row-tile kernel
+    static constexpr bool kTile = false;  // not built for the row-tile kernel
     static constexpr int kRed = 2;
     static constexpr bool kSystem = true;
     struct Pre {
@@ -1319,7 +1319,7 @@ static void launch_nb(mpet_ctx* c, const NodeBlocks& nb, const T* x, const Epi& 
 // b += the pressure rows' displacement-column products (FP64 right-hand side term)
 struct EpiAddRhs {
     double* b;
-    static constexpr bool kTile = false;  // runs with the row-tile kernel
+    static constexpr bool kTile = false;  // not built for the row-tile kernel
     static constexpr int kRed = 0;
     static constexpr bool kSystem = true;
     struct Pre {};
@@ -3981,10 +3981,10 @@ static int solve_constrained(mpet_ctx* c, const double* b, double* x, mpet_stats
 
 int solve_system(mpet_ctx* c, const double* b, double* x, mpet_stats* st, bool homogeneous) {
     // the stored copies that the products of this solve read
+    MPET_CUDA(cudaEventRecord(c->ev_sv0, c->stream));
     need_system_copy<double>(c);
     if (c->prm.precision == MPET_PRECISION_MIXED && !c->sys_patch) need_system_copy<float>(c);
     if (c->prm.precision == MPET_PRECISION_MIXED && c->u_elast) need_copies(c, COPY_NB32);
-    MPET_CUDA(cudaEventRecord(c->ev_sv0, c->stream));
     int s;
     if (c->gmres && (c->ninst > 0 || c->nrigid > 0))
         fail(MPET_ERR_INVALID, "GMRES (non-symmetric S) is built for single instances without rigid modes");
