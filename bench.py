@@ -182,6 +182,25 @@ def time_spmv(solver, torch, lib, reps=20):
     return out
 
 
+def time_step_calls(solver, torch, dt, reps=5):
+    """ms of a step() call (assembly, right-hand side, solve, state handed on), and of its assembly."""
+    solver.problem.time.assign(0.0)
+    solver.up_.vector().zero_()
+    e0, e1, e2 = (torch.cuda.Event(enable_timing=True) for _ in range(3))
+    for k in range(reps + 2):
+        if k == 2:
+            torch.cuda.synchronize()
+            e0.record(solver._stream)
+        solver.step(dt)
+        solver.up_.assign(solver.up)
+    e1.record(solver._stream)
+    for _ in range(reps):
+        solver.ctx.call("mpet_assemble", dt, 1)
+    e2.record(solver._stream)
+    torch.cuda.synchronize()
+    return e0.elapsed_time(e1) / reps, e1.elapsed_time(e2) / reps
+
+
 def time_inner_product(solver, torch, lib, reps=20):
     """The FP32 product of the inner iterations (from the elements, or the stored matrix)."""
     import ctypes
@@ -286,10 +305,28 @@ def spmv_tuning(solver, fp64=False):
             "chosen": variants.get(ch.value, str(ch.value))}
 
 
+def finest_level_roofline(solver, hbm, peak_kind):
+    """Work of the finest displacement level in a V-cycle (smoothing products, residual, transfers), the
+    largest part of an iteration: its algorithmic bytes over its time from a flushed L2."""
+    import ctypes
+    from waterscapes_gb300 import _lib
+    nl = ctypes.c_int32()
+    ms, by = np.zeros(16), np.zeros(16)
+    solver.ctx.call("mpet_profile_vcycle", 0, 7, ctypes.byref(nl), _lib._ptr(ms), _lib._ptr(by))
+    own = ms[0] - (ms[1] if nl.value > 1 else 0.0)
+    kernel = {64: "k_spmv_tile (row tiles)", 16: "k_p2lap_mf (matrix-free)", 8: "k_spmv_nb (node blocks)",
+              32: "k_spmv_sell_h (SELL-32, FP16)"}.get(level_variants(solver)["displacement"][0])
+    return {"kernel": "finest displacement level of the V-cycle, products by " + (kernel or "SELL-32 or CSR"),
+            "bound": "hbm", "achieved": by[0] / own / 1e6, "peak": hbm, "unit": "GB/s",
+            "frac": by[0] / own / 1e6 / hbm, "peak_kind": peak_kind, "ms_per_vcycle": own,
+            "alg_bytes_per_vcycle": by[0]}
+
+
 def level_variants(solver):
     """SpMV variant the set-up autotuner chose for each level's operator, per
     hierarchy (displacement, then each network): 4/5 SELL-32, 6/7 SELL late,
-    0-3 CSR register/staged, 8 node blocks, 16 matrix-free, 32 SELL FP16."""
+    0-3 CSR register/staged, 8 node blocks, 16 matrix-free, 32 SELL FP16,
+    64 row tiles."""
     from waterscapes_gb300 import _lib
     out = {}
     for blk in range(solver.J + 1):
@@ -879,14 +916,11 @@ def main():
     sol._assemble(dt)
     torch.cuda.synchronize()
     t_asm_amg = time.perf_counter() - t0
-    # matrix assembly alone (step() semantics re-assemble every step)
+    # step() calls, which assemble every time, and the assembly alone: after a first step the assembly
+    # writes the stored copies that a step's products read (and, as long as time_spmv has not run, no other)
+    step_ms, asm_ms = time_step_calls(sol, torch, dt)
     e0 = torch.cuda.Event(enable_timing=True)
     e1 = torch.cuda.Event(enable_timing=True)
-    e0.record(sol._stream)
-    sol.ctx.call("mpet_assemble", dt, 1)
-    e1.record(sol._stream)
-    torch.cuda.synchronize()
-    asm_ms = e0.elapsed_time(e1)
     spmv = time_spmv(sol, torch, lib)
     inner_product = time_inner_product(sol, torch, lib) if sol.params["precision"] == "mixed" else None
     precond_ms = time_precond(sol, torch, lib)
@@ -923,9 +957,6 @@ def main():
     e1.record(sol._stream)
     torch.cuda.synchronize()
     e2e_ms = e0.elapsed_time(e1) / ke
-
-    # step() semantics: assemble every step
-    step_ms = asm_ms + ms_mixed / args.steps
 
     res = {"mixed": {"ms_per_step": ms_mixed / args.steps, "iterations": its_mixed}}
     rel_err = None
@@ -1007,11 +1038,13 @@ def main():
         "iteration_breakdown_ms": dict(split, spmv_fp32=(spmv.get("fp32") or spmv["fp64"])["ms"],
                                        inner_product=inner_product, preconditioner=precond_ms),
         "fp64_iteration_breakdown_ms": res.get("fp64", {}).get("iteration_breakdown_ms"),
-        "roofline": {"kernel": ROOFLINE_KERNEL[sp32["layout"]] + (" FP32" if "fp32" in spmv else " FP64")
+        "roofline": finest_level_roofline(sol, hbm, peak_kind),
+        "stored_product": {"kernel": ROOFLINE_KERNEL[sp32["layout"]] + (" FP32" if "fp32" in spmv else " FP64")
                      + (", 64-register kernel" if tuning.get("chosen") == "node-block/64 registers" else ""),
                      "bound": "hbm", "achieved": sp32["gbs"], "peak": hbm, "unit": "GB/s",
                      "frac": sp32["gbs"] / hbm, "peak_kind": peak_kind,
-                     "note": "the product with the stored matrix; see inner_product for the inner iterations'",
+                     "note": "the product with the stored matrix, not part of a step where inner_product is from "
+                             "the elements",
                      "alg_bytes_per_launch": sp32["alg_bytes"],
                      "traffic": (sp32["alg_bytes"] * TRAFFIC_RATIO[sp32["layout"]]
                                  if sp32["layout"] in TRAFFIC_RATIO else None),

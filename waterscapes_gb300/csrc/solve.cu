@@ -2160,9 +2160,12 @@ static void profile_levels(mpet_ctx* c, AmgHier& h, int reps, double* ms, double
         const double nc = (double)h.lev[k + 1].A.n, vecc = nc * NV * sv;
         // a product with A: the CSR entries and row pointers, or (matrix-free) the
         // incidence and per-cell node ids (NN each), the per-cell data, the row
-        // pointers of the incidence and the Dirichlet flags, once each
+        // pointers of the incidence and the Dirichlet flags, once each; by row tiles 16-bit
+        // column ids and the tiles' column lists instead of column ids and row pointers
         const double nn_cell = c->dim == 3 ? 10.0 : 6.0;
         const double mA = L.mf ? (double)c->nc * (2.0 * nn_cell * 4.0 + 8.0 * sv) + n + (n + 1) * 8.0
+                          : L.A.variant == 64 && L.A.rt.nt > 0
+                               ? L.A.nnz * (sv + 2.0) + (double)L.A.rt.nt * L.A.rt.mc * 4.0
                                : L.A.nnz * (sv + 4.0) + (n + 1) * 8.0;
         double b = 2 * vec + dv;                              // first Chebyshev step (no product)
         b += (2 * s - 1) * (mA + 3 * vec + dv);               // the other 2s - 1 smoothing products
