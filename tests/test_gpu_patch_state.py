@@ -119,3 +119,32 @@ def test_the_preconditioner_before_the_assembly():
     s.ctx.call("mpet_setup_preconditioner", dt)
     s.ctx.call("mpet_assemble", dt, 1)
     _check_product(s, 1)
+
+
+def test_vertices_of_no_cell():
+    """Their rows are empty: zero in every product (no patch holds them, so the stored copy serves), and
+    one in the diagonal scaling of the residual."""
+    import scipy.sparse as sp
+    from waterscapes_gb300 import Constant, Mesh, MPETProblem, MPETSolver, UnitCubeMesh, _lib
+    from helpers import cfg_params
+    unit = UnitCubeMesh(3)
+    x0, c0 = unit.coordinates(), unit.cells()
+    # one before all others and two behind
+    mesh = Mesh(np.concatenate([[[2.0, 0.0, 0.0]], x0, [[3.0, 0.0, 0.0], [0.0, 4.0, 1.0]]]), c0 + 1)
+    params, dt = cfg_params(2)
+    s = MPETSolver(MPETProblem(mesh, Constant(0.0), params=params), dict(dt=dt, precision="mixed"))
+    s.ctx.call("mpet_set_element_product", 1)
+    s.ctx.call("mpet_assemble", dt, 1)
+    _check_product(s, 0)
+    rp, ci = s.pattern()
+    A = sp.csr_matrix((s.matrix_values(), ci, rp), shape=(s.N, s.N))
+    d = np.abs(A.diagonal())
+    x = np.random.default_rng(8).standard_normal(s.N)
+    b = np.ones(s.N)
+    xt, bt = (torch.tensor(v, device=s.device) for v in (x, b))
+    r, norms = torch.empty_like(xt), np.zeros(2)
+    s.ctx.call("mpet_residual", _lib._ptr(bt), _lib._ptr(xt), _lib._ptr(r), _lib._ptr(norms))
+    dinv = 1.0 / np.where(d > 0.0, d, 1.0)
+    assert (d == 0.0).sum() == 3 * (3 + 2)
+    ref = [np.linalg.norm(dinv * (b - A @ x)), np.linalg.norm(dinv * b)]
+    assert np.allclose(norms, ref, rtol=1e-12, atol=0.0)

@@ -387,7 +387,7 @@ __global__ void __launch_bounds__(256) k_assemble_matrix(AsmArgs A, MatCoef P) {
                 for (int e = lane; e < L; e += 32) A.v64[rp[q] + e] = e == dpos ? 1.0 : 0.0;
             }
             if (lane == 0) {
-                double dg = fixed ? 1.0 : fabs(at(q, dpos));
+                double dg = fixed ? 1.0 : L > 0 ? fabs(at(q, dpos)) : 0.0;  // (a vertex of no cell: empty rows)
                 A.dinv[rows[q]] = dg > 0.0 ? 1.0 / dg : 1.0;
             }
         }

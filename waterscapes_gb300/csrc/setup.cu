@@ -714,14 +714,16 @@ __global__ void k_patch_node_major(int64_t npn, const u64* __restrict__ key, u64
     if (i < npn) nkey[i] = (key[i] << 32) | (u64)i;
 }
 
-// per node: whether several patches hold it, and its number of partial sums
+// per node: whether several patches hold it, and its number of partial sums; *none: some node is in no
+// patch
 __global__ void k_patch_shared(int64_t nnodes, const u64* __restrict__ nkey, int64_t npn, int32_t* shared,
-                               int32_t* slots) {
+                               int32_t* slots, int32_t* none) {
     const int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (v >= nnodes) return;
     const int n = (int)(lower_bound_u64(nkey, npn, (u64)(v + 1) << 32) - lower_bound_u64(nkey, npn, (u64)v << 32));
     shared[v] = n > 1;
     slots[v] = n > 1 ? n : 0;
+    if (n == 0) *none = 1;
 }
 
 __global__ void k_patch_fill_shared(int64_t npn, const u64* __restrict__ nkey,
@@ -905,19 +907,30 @@ void build_patches(mpet_ctx* c) {
         u64* nk = nullptr;
         sort_unique(c, keys.as<u64>(), s.npn, 32 + bits_for((u64)nn), &nk);
         for (TmpBuf* b : {&shared, &slots}) MPET_CUDA(cudaMemsetAsync(b->p, 0, sizeof(int32_t) * (nn + 1), st));
-        k_patch_shared<<<grid_for(nn, T), T, 0, st>>>(nn, nk, s.npn, shared.as<int32_t>(), slots.as<int32_t>());
+        TmpBuf none(sizeof(int32_t));
+        MPET_CUDA(cudaMemsetAsync(none.p, 0, sizeof(int32_t), st));
+        k_patch_shared<<<grid_for(nn, T), T, 0, st>>>(nn, nk, s.npn, shared.as<int32_t>(), slots.as<int32_t>(),
+                                                      none.as<int32_t>());
         MPET_CHECK_LAUNCH();
         size_t tb = 0;
         MPET_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, shared.as<int32_t>(), sid.as<int32_t>(), (int)(nn + 1), st));
         TmpBuf tmp(tb);
         MPET_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, tb, shared.as<int32_t>(), sid.as<int32_t>(), (int)(nn + 1), st));
         MPET_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, tb, slots.as<int32_t>(), sbase.as<int32_t>(), (int)(nn + 1), st));
-        int32_t tot[4];
+        int32_t tot[5];
+        MPET_CUDA(cudaMemcpyAsync(&tot[4], none.p, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
         MPET_CUDA(cudaMemcpyAsync(&tot[0], sid.as<int32_t>() + nn, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
         MPET_CUDA(cudaMemcpyAsync(&tot[1], sbase.as<int32_t>() + nn, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
         MPET_CUDA(cudaMemcpyAsync(&tot[2], sid.as<int32_t>() + c->nv, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
         MPET_CUDA(cudaMemcpyAsync(&tot[3], sbase.as<int32_t>() + c->nv, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
         MPET_CUDA(cudaStreamSynchronize(st));
+        if (tot[4]) {  // a vertex of no cell: no patch would write its rows of the product
+            c->pool.release(nk);
+            c->pool.release(key);
+            release_patches(c);
+            s.tried = true;
+            return;
+        }
         s.nsh = tot[0];
         s.nslot = tot[1];
         s.nshv = tot[2];
